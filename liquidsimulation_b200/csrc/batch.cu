@@ -3,8 +3,7 @@
 //
 // Scene s owns the slots [base_s, base_s + n_s). An item is a run of at most T particles
 // of one scene and the per-item kernels run one item per block, so a block stages exactly
-// one scene's constants (DevParams) and kernel tables in shared memory, as the single-scene
-// kernels do. Every particle runs the same per-particle function (particle_ops.cuh) with
+// one scene's constants (DevParams) in shared memory. Every particle runs the same per-particle function (particle_ops.cuh) with
 // its scene's constants, so each scene's results are bit-identical to stepping it alone.
 //
 // The persistent loop (kb_pci_loop) advances all scenes in lockstep rounds:
@@ -68,7 +67,7 @@ __global__ void __launch_bounds__(T) kb_keys(BatchArgs a, const float4* __restri
 }
 
 // The lists plus the start-of-step density and pressure (k_neighbors_density in grid.cu),
-// per item with the item's scene constants and tables.
+// per item with the item's scene constants.
 template <int T>
 __global__ void __launch_bounds__(T) kb_neighbors_density(BatchArgs a, const float4* __restrict__ pos,
                                                           const uint32_t* __restrict__ cell_start,
@@ -77,19 +76,15 @@ __global__ void __launch_bounds__(T) kb_neighbors_density(BatchArgs a, const flo
                                                           const float4* __restrict__ vel, float4* __restrict__ vrho)
 {
     __shared__ DevParams P;
-    __shared__ float W[kTableSize], TH2[kTableSize + 1];
     const BatchItem it = a.items[blockIdx.x];
-    const float* tb = scene_tables(a, it.scene);
     stage_params(&P, a.sp, it.scene);
-    stage_table(W, tb, T_W);
-    stage_table(TH2, tb, T_THRESH2);
     __syncthreads();
     const int i = it.begin + (int)threadIdx.x;
     const bool valid = i < it.end;
     int c = 0;
     if (valid) {
         float sum;
-        c = neighbors_one<true>(P, pos, cell_start, nbr, i, W, TH2, &sum);
+        c = neighbors_one<true>(P, pos, cell_start, nbr, i, scene_tables(a, it.scene), &sum);
         count[i] = min(c, P.nbr_cap);
         const float r = P.mass * sum;
         float pr = P.stiffness * (r - P.rho0);
@@ -108,31 +103,26 @@ template <int T, bool kGrad>
 __global__ void __launch_bounds__(T) kb_nonpressure(BatchArgs a, StepBuffers b)
 {
     __shared__ DevParams P;
-    __shared__ float4 NA[kTableSize], NB[kTableSize];
     const BatchItem it = a.items[blockIdx.x];
-    const float* tb = scene_tables(a, it.scene);
     stage_params(&P, a.sp, it.scene);
-    stage_nonpressure_slots(NA, NB, tb);
+    b.tables = scene_tables(a, it.scene);
     __syncthreads();
     const int i = it.begin + (int)threadIdx.x;
     if (i >= it.end) return;
-    nonpressure_one<kGrad>(P, b, NA, NB, i);
+    nonpressure_one<kGrad>(P, b, i);
 }
 
 template <int T>
 __global__ void __launch_bounds__(T) kb_sph_pressure(BatchArgs a, StepBuffers b)
 {
     __shared__ DevParams P;
-    __shared__ float SDW[kTableSize], TH[kTableSize + 1];
     const BatchItem it = a.items[blockIdx.x];
-    const float* tb = scene_tables(a, it.scene);
     stage_params(&P, a.sp, it.scene);
-    stage_table(SDW, tb, T_SPIKY_DW);
-    stage_table(TH, tb, T_THRESH);
+    b.tables = scene_tables(a, it.scene);
     __syncthreads();
     const int i = it.begin + (int)threadIdx.x;
     if (i >= it.end) return;
-    sph_pressure_one(P, b, SDW, TH, i);
+    sph_pressure_one(P, b, i);
 }
 
 template <int T>
@@ -168,16 +158,13 @@ template <int T>
 __global__ void __launch_bounds__(T) kb_density_first(BatchArgs a, StepBuffers b, BatchWarmArgs w)
 {
     __shared__ DevParams P;
-    __shared__ float W[kTableSize], TH2[kTableSize + 1];
     const BatchItem it = a.items[blockIdx.x];
-    const float* tb = scene_tables(a, it.scene);
     stage_params(&P, a.sp, it.scene);
-    stage_table(W, tb, T_W);
-    stage_table(TH2, tb, T_THRESH2);
     __syncthreads();
     const int i = it.begin + (int)threadIdx.x;
     const float p_scale = P.delta * 0.01f * P.rho0;
-    const float e = density_first(P, b, w.feat, b.hist, b.gradrho, p_scale, W, TH2, i, i < it.end);
+    b.tables = scene_tables(a, it.scene);
+    const float e = density_first(P, b, w.feat, b.hist, b.gradrho, p_scale, i, i < it.end);
     uint32_t m = __float_as_uint(e);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -262,7 +249,6 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
     int* preA = dyn + 2 * S;       // phase A item prefix (S + 1)
     int* preB = dyn + 3 * S + 1;   // phase B item prefix (S + 1)
     __shared__ DevParams P;
-    __shared__ float W[kTableSize], SDW[kTableSize], TH[kTableSize + 1], TH2[kTableSize + 1];
     __shared__ int staged;
     __shared__ int warp_sums[32];
     LoopSync* sy = reinterpret_cast<LoopSync*>(l.sync);
@@ -287,12 +273,8 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
     auto stage_scene = [&](int s) {
         if (s == staged) return;
         __syncthreads();
-        const float* tb = scene_tables(a, s);
         stage_params(&P, a.sp, s);
-        stage_table(W, tb, T_W);
-        stage_table(SDW, tb, T_SPIKY_DW);
-        stage_table(TH, tb, T_THRESH);
-        stage_table(TH2, tb, T_THRESH2);
+        b.tables = scene_tables(a, s);
         if (threadIdx.x == 0) staged = s;
         __syncthreads();
     };
@@ -380,7 +362,7 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
             // the scene's last pass is force(k), then the integration and collisions (own
             // data only; the scenes never read each other's particles).
             const bool restart = act == ACT_RESTART, last = act == ACT_FINAL;
-            if (!restart) pci_force_one(P, b, SDW, TH, i, pp(last ? k : k - 1));
+            if (!restart) pci_force_one(P, b, i, pp(last ? k : k - 1));
             if (!last) pci_predict_one(P, b, i, k, pp(k));
             else integrate_one(P, b, i, 1);
         });
@@ -394,7 +376,7 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
             const int k = st_k(w), kp = st_kp(w);
             const int i = P.base + j * T + (int)threadIdx.x;
             float m = 0.f;
-            if (i < P.base + P.n) m = pci_density_one(P, b, W, TH2, i, k, pp(k));
+            if (i < P.base + P.n) m = pci_density_one(P, b, i, k, pp(k));
             // Max of non-negative floats: their bit patterns order like the values.
             uint32_t mb = __float_as_uint(m);
 #pragma unroll

@@ -28,11 +28,11 @@ void HostKernels::build(const lsp_params& p)
     (void)r4;
     step = h / sub;
     const double pi = 3.14159265358979323846;
-    float poly_k = (float)(315.0 / (64.0 * pi * (double)r9));
-    float poly_d1 = (float)(-945.0 / (32.0 * pi * (double)r9));
-    float poly_d2 = (float)(-945.0 / (32.0 * pi * (double)r9));
-    float spiky_d1 = (float)(-45.0 / (pi * (double)r6));
-    float visc_d2 = (float)(45.0 / (pi * (double)r6));
+    poly_k = (float)(315.0 / (64.0 * pi * (double)r9));
+    poly_d1 = (float)(-945.0 / (32.0 * pi * (double)r9));
+    poly_d2 = (float)(-945.0 / (32.0 * pi * (double)r9));
+    spiky_d1 = (float)(-45.0 / (pi * (double)r6));
+    visc_d2 = (float)(45.0 / (pi * (double)r6));
     // Five lookup tables, then the kTableSize + 1 slot thresholds of the device lookup on
     // the distance, then the same thresholds on the squared distance.
     tables.assign(kTableFloats, 0.f);
@@ -86,12 +86,6 @@ void HostKernels::build(const lsp_params& p)
     for (int k = 1; k <= sub; k++) thr2[k] = sq_bound(thr[k]);
     thr2[kTableSize] = std::numeric_limits<float>::infinity();
     cut2 = sq_bound(h);
-    uint32_t w_last;
-    std::memcpy(&w_last, &tables[0 * kTableSize + sub], 4);   // W at slot 1000
-    density_tail0 = w_last == 0u && thr2[sub] <= cut2;
-    uint32_t sdw_last;
-    std::memcpy(&sdw_last, &tables[3 * kTableSize + sub], 4);   // spiky gradient at slot 1000
-    force_tail0 = (sdw_last & 0x7fffffffu) == 0u && thr[sub] <= h;
     float stepSize = 1.6f * p.particle_radius;
     float sum = 0.f;
     for (int i = -3; i <= 3; i++)
@@ -492,8 +486,11 @@ DevParams physics_params(const lsp_params& p, const HostKernels& hk, float dt)
     P.min_it = p.pci_min_iterations;
     P.max_it = p.pci_max_iterations;
     P.exact_tables = hk.exact_tables ? 1 : 0;
-    P.density_tail0 = hk.density_tail0 ? 1 : 0;
-    P.force_tail0 = hk.force_tail0 ? 1 : 0;
+    P.kw = hk.poly_k;
+    P.kdw = hk.poly_d1;
+    P.kd2w = hk.poly_d2;
+    P.ksdw = hk.spiky_d1;
+    P.kvd2w = hk.visc_d2;
     return P;
 }
 

@@ -25,13 +25,9 @@ struct HostKernels {
     // Laplacian) is 0 or within [2^-29, 2^60]: the pass may then divide by the neighbour
     // density with div_by (DevParams::exact_tables).
     bool exact_tables = false;
-    // The W table's last entry (slot 1000) is +0 and every s >= cut2 takes that slot
-    // (thr2[1000] <= cut2): the density lookups may then skip the cutoff's select
-    // (DevParams::density_tail0), since the slot already gives the cutoff's 0.
-    bool density_tail0 = false;
-    // The same for the spiky gradient table and the distance cutoff: its last entry is a zero
-    // and every d >= h takes slot 1000 (thr[1000] <= h) (DevParams::force_tail0).
-    bool force_tail0 = false;
+    // Factors of the five formulas (DevParams::kw ...): the device evaluates the tables' entries
+    // itself (entry_w and the others in lsp_device.cuh).
+    float poly_k = 0, poly_d1 = 0, poly_d2 = 0, spiky_d1 = 0, visc_d2 = 0;
     void build(const lsp_params& p);
     float delta(const lsp_params& p, float dt) const;
     float look(int t, float d) const;

@@ -210,28 +210,23 @@ __global__ void k_rank_gather(DevParams P, const int2* __restrict__ tmp, const u
 }
 
 // Start-of-step neighbour lists (neighbors_one, plain column-major) plus the start-of-step density
-// and pressure of density_one (SPHSolver::calcParticleDensityPressure,
+// and pressure (SPHSolver::calcParticleDensityPressure,
 // SPHSolver.cpp:442-463), summed while the list is built: a pass over the stored list and
 // its position gathers would cost more. (A list that
 // overflows its capacity raises the overflow flag and the step is redone, so the sum over
 // every accepted pair never differs from the stored list's.)
-template <bool kTail0>
 __global__ void k_neighbors_density(DevParams P, const float4* __restrict__ pos,
                                     const uint32_t* __restrict__ cell_start, int32_t* __restrict__ nbr,
                                     int32_t* __restrict__ count, DevStatus* st, const float* __restrict__ tables,
                                     float* __restrict__ rho, float* __restrict__ pres,
                                     const float4* __restrict__ vel, float4* __restrict__ vrho)
 {
-    __shared__ float W[kTableSize], TH2[kTableSize + 1];
-    stage_table(W, tables, T_W);
-    stage_table(TH2, tables, T_THRESH2);
-    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < P.n;
     int c = 0;
     if (valid) {
         float sum;
-        c = neighbors_one<true, kTail0>(P, pos, cell_start, nbr, i, W, TH2, &sum);
+        c = neighbors_one<true>(P, pos, cell_start, nbr, i, tables, &sum);
         count[i] = min(c, P.nbr_cap);
         const float r = P.mass * sum;
         float pr = P.stiffness * (r - P.rho0);
@@ -316,14 +311,8 @@ int launch_neighbors(const GridBuildArgs& a, cudaStream_t s)
 {
     const int T = 256;
     if (a.P.n <= 0) return 0;
-    if (a.P.density_tail0)
-        k_neighbors_density<true><<<blocks_for(a.P.n, T), T, 0, s>>>(a.P, a.pos_out, a.cell_start, a.nbr, a.nbr_count,
-                                                                     a.status, a.tables, a.rho, a.pres, a.vel_out,
-                                                                     a.vrho);
-    else
-        k_neighbors_density<false><<<blocks_for(a.P.n, T), T, 0, s>>>(a.P, a.pos_out, a.cell_start, a.nbr,
-                                                                      a.nbr_count, a.status, a.tables, a.rho, a.pres,
-                                                                      a.vel_out, a.vrho);
+    k_neighbors_density<<<blocks_for(a.P.n, T), T, 0, s>>>(a.P, a.pos_out, a.cell_start, a.nbr, a.nbr_count, a.status,
+                                                           a.tables, a.rho, a.pres, a.vel_out, a.vrho);
     return 1;
 }
 

@@ -93,8 +93,9 @@ struct DevParams {
     int coll_off;
     int scene;
     int exact_tables;   // HostKernels::exact_tables
-    int density_tail0;  // HostKernels::density_tail0
-    int force_tail0;    // HostKernels::force_tail0
+    // Factors of the kernel formulas: poly6 W, gradient and Laplacian, spiky gradient,
+    // viscosity Laplacian (HostKernels::build).
+    float kw, kdw, kd2w, ksdw, kvd2w;
 };
 
 // ----------------------------------------------------------------- vector ops
@@ -212,55 +213,247 @@ __host__ __device__ __forceinline__ int table_slot_sq_from(float s, float d_gues
     const int k = slot_guess(d_guess, inv_step);
     return !(s < thr2[k]) ? k : k - 1;
 }
-__device__ __forceinline__ int table_slot_sq(float s, float inv_step, const float* thr2)
+
+// The kernel weights by arithmetic. Table entry k is a formula in the table distance
+// d_k = k * step (HostKernels::build), and the device evaluates the same operations in the same
+// order on the slot number held as a float, so the value is the table's entry bit for bit (every
+// operation rounds once on both sides; every entry of every table is checked against the
+// host's, tests/test_pair_weights.py). What bounds the neighbour passes is the L1 data pipe (70 to 78 % of
+// its wavefronts in every neighbour pass, against 52 % of the issue slots in the PCISPH loop): a
+// read of a random slot in shared memory took 2.7 wavefronts of it and a pair needed two or more
+// (31 % of the loop's wavefronts, 39 % of the non-pressure pass's), while the formula takes 4 to
+// 10 multiplications and additions and no memory. With the two-pair forms below, at 991,440
+// particles in motion (6 iterations a step): loop 1.130 -> 0.994 ms, non-pressure pass 0.206 ->
+// 0.166 ms a step; 417,792 particles: loop 0.572 -> 0.495, non-pressure 0.091 -> 0.063 ms.
+//
+// The slot: t = d * inv_step - 1/2 rounded to the nearest integer is trunc(d / step) unless d / step lies
+// within the error of the approximate quotient of an integer. For the squared-distance form
+// the relative error is at most 2^-23 (sqrt.approx) + 5 * 2^-24 (inv_step, t, and the
+// roundings of the square root and the quotient that define the slot) = 4.2e-7 < kSlotEps.
+// Closer than that (one pair in about 1,500) the slot comes from the threshold tables in global
+// memory, as does a NaN's. kSlotHalf = (1 - kSlotEps) / 2 shifts the rounding by half the margin
+// so that one comparison covers both edges of the slot: with f = t - k, the quotient is at least
+// k * kSlotEps above k and (k + 1) * kSlotEps below k + 1 exactly when |f| <= kSlotHalf - k * kSlotEps.
+constexpr float kSlotEps = 4.8e-7f;
+constexpr float kSlotHalf = 0.5f - 0.5f * kSlotEps;
+constexpr float kSlotMagic = 12582912.f;   // 1.5 * 2^23: adding it rounds to an integer
+
+// Slot of the distance (or its approximation) `guess` as a float; at or beyond h it may be any
+// number, since every weight is 0 there. kNan: a NaN is unsure (the passes that divide by the
+// distance leave it out: their terms are NaN whatever the weight, and the particle itself, at
+// distance 0, is a NaN of sqrt_rn in every walk of the force pass).
+template <bool kNan>
+__device__ __forceinline__ float slot_from(float guess, float inv_step, bool& unsure)
+{
+    const float t = __fmaf_rn(guess, inv_step, -kSlotHalf);
+    const float k = __fadd_rn(__fadd_rn(t, kSlotMagic), -kSlotMagic);
+    const float f = fabsf(__fadd_rn(t, -k)), m = __fmaf_rn(k, -kSlotEps, kSlotHalf);
+    unsure = kNan ? !(f <= m) : f > m;
+    return k;
+}
+__device__ __forceinline__ float sqrt_guess(float s)
 {
     float d;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(d) : "f"(s));
-    return table_slot_sq_from(s, d, inv_step, thr2);
+    return d;
+}
+// tables: the kernel table block (global memory), read only in the unsure case.
+__device__ __forceinline__ float slot_sq(float s, const DevParams& P, const float* __restrict__ tables)
+{
+    const float d = sqrt_guess(s);
+    bool unsure;
+    float k = slot_from<true>(d, P.inv_step, unsure);
+    if (unsure) k = (float)table_slot_sq_from(s, d, P.inv_step, tables + kThresh2Offset);
+    return k;
+}
+__device__ __forceinline__ float slot_dist(float d, const DevParams& P, const float* __restrict__ tables)
+{
+    bool unsure;
+    float k = slot_from<false>(d, P.inv_step, unsure);
+    if (unsure) k = (float)table_slot(d, P.inv_step, tables + kThreshOffset);
+    return k;
 }
 
-// The table read is unconditional (the slot is always inside the table) and the cutoff a
-// select: measured faster than branching around the read.
-// kTail0 (DevParams::force_tail0, for the spiky table): every d >= h takes slot 1000, whose
-// entry is a zero, so the cutoff's select is left out. (Its sign may be negative; a force sum
-// starts at +0 and a sum of roundings to nearest never reaches -0 from there, so adding either
-// zero leaves it unchanged.)
-template <bool kTail0 = false>
-__device__ __forceinline__ float lookup(const float* tab, const float* thr, float d, const DevParams& P)
+// Table entries at slot k (HostKernels::build's expressions).
+__device__ __forceinline__ float entry_w(float k, const DevParams& P)
 {
-    const float w = tab[table_slot(d, P.inv_step, thr)];
-    return (kTail0 || !(d >= P.h)) ? w : 0.f;
+    const float d = k * P.step, t = P.h2 - d * d;
+    return P.kw * t * t * t;
 }
-// lookup(tab, thr, sqrt(s), P) bit for bit, from the squared distance (d >= h exactly when
-// s >= cut2).
-// kTail0 (DevParams::density_tail0, for the W table): every s >= cut2 takes slot 1000,
-// whose entry is +0, so the cutoff's select is redundant and left out.
-template <bool kTail0 = false>
-__device__ __forceinline__ float lookup_sq(const float* tab, const float* thr2, float s, const DevParams& P)
+__device__ __forceinline__ float entry_sdw(float k, const DevParams& P)
 {
-    const float w = tab[table_slot_sq(s, P.inv_step, thr2)];
-    return (kTail0 || !(s >= P.cut2)) ? w : 0.f;
+    const float s = P.h - k * P.step;
+    return P.ksdw * s * s;
 }
-
-// The non-pressure pass reads three tables at one squared distance s. Its slot records
-// a[k] = {thr2[k], DW[k-1], DW[k], D2W[k-1]} and b[k] = {D2W[k], VD2W[k-1], VD2W[k], -} give
-// all three values with two 16-byte shared-memory reads once the first guess k is known,
-// instead of a threshold read followed by three dependent table reads (measured 6.6 %
-// faster; for one table the split threshold and table reads are faster). The slot is the
-// one table_slot_sq_from picks, so the values are the same entries.
+// SPHKernel::get*Weight of a squared distance (poly6, d >= h exactly when s >= cut2) and of a
+// distance (spiky gradient).
+__device__ __forceinline__ float weight_w(float s, const DevParams& P, const float* __restrict__ tables)
+{
+    const float w = entry_w(slot_sq(s, P, tables), P);
+    return !(s >= P.cut2) ? w : 0.f;
+}
+__device__ __forceinline__ float weight_sdw(float d, const DevParams& P, const float* __restrict__ tables)
+{
+    const float w = entry_sdw(slot_dist(d, P, tables), P);
+    return !(d >= P.h) ? w : 0.f;
+}
+// The non-pressure pass's three weights at one squared distance.
 struct NonpressureWeights {
     float dw, d2w, vd2w;
-    __device__ __forceinline__ NonpressureWeights(const float4* ra, const float4* rb, float s, const DevParams& P)
+    __device__ __forceinline__ NonpressureWeights(float s, const DevParams& P, const float* __restrict__ tables)
     {
-        float g;
-        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(s));
-        const int k = slot_guess(g, P.inv_step);
-        const float4 a = ra[k], b = rb[k];
-        const bool hi = !(s < a.x);
+        const float k = slot_sq(s, P, tables);
+        const float d = k * P.step, t = P.h2 - d * d;
         const bool inside = !(s >= P.cut2);
-        dw = inside ? (hi ? a.z : a.y) : 0.f;
-        d2w = inside ? (hi ? b.x : a.w) : 0.f;
-        vd2w = inside ? (hi ? b.z : b.y) : 0.f;
+        dw = inside ? P.kdw * t * t : 0.f;
+        d2w = inside ? P.kd2w * t * (3.f * P.h2 - 7.f * d * d) : 0.f;
+        vd2w = inside ? P.kvd2w * (P.h - d) : 0.f;
+    }
+};
+
+// Two pairs at a time: sm_100's packed float operations do two IEEE single operations in one
+// instruction (each half rounds as the scalar operation does), which halves the issue slots of
+// the pair arithmetic.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ float lo(F2 a)
+{
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return x;
+}
+__device__ __forceinline__ float hi(F2 a)
+{
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return y;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// a - b for finite or infinite b: a + b * (-1), one rounding.
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return fma2(b, f2(-1.f), a); }
+// -(x^2 + y^2 + z^2), each sum and product rounded once. ptxas contracts an add.rn.f32x2 of a
+// mul.rn.f32x2 into one fma (with -fmad=false too: seen as one-ulp differences from the scalar
+// form), also where the sum is written as an fma with 1; a product that enters an fma as the
+// factor of -1 stays a product, so the sum is formed negated
+// (tests/cpp/pair_weights_check.cu compares it and the operations below with the scalar ones).
+__device__ __forceinline__ F2 neg_sqmag(F2 x, F2 y, F2 z)
+{
+    const F2 m = f2(-1.f);
+    return fma2(z * z, m, fma2(y * y, m, (x * m) * x));
+}
+
+// sqrt_rn, recip_rn and div_by of two pairs on negated arguments: -sqrt(s) from ns = -s,
+// 1 / d from nd = -d, a / d from nd and y = recip_rn(nd) (rounding to nearest is symmetric, so
+// the bits are those of the scalar forms).
+__device__ __forceinline__ F2 neg_sqrt_rn(F2 ns)
+{
+    float a, b;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(-lo(ns)));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(-hi(ns)));
+    const F2 y = f2(a, b);
+    const F2 g = ns * y, h = y * f2(0.5f);
+    return fma2(fma2(g, g, ns), h, g);
+}
+__device__ __forceinline__ F2 recip_rn(F2 nd)
+{
+    float a, b;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(-lo(nd)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(-hi(nd)));
+    const F2 y0 = f2(a, b);
+    return fma2(fma2(nd, y0, f2(1.f)), y0, y0);
+}
+__device__ __forceinline__ F2 div_by(F2 a, F2 nd, F2 y)
+{
+    const F2 q0 = a * y;
+    return fma2(fma2(nd, q0, a), y, q0);
+}
+// slot_from of two pairs, of the negated distances.
+template <bool kNan>
+__device__ __forceinline__ F2 slot_from(F2 nguess, float inv_step, bool& unsure0, bool& unsure1)
+{
+    const F2 t = fma2(nguess, f2(-inv_step), f2(-kSlotHalf));
+    const F2 k = (t + f2(kSlotMagic)) + f2(-kSlotMagic);
+    const F2 f = t - k;
+    const F2 m = fma2(k, f2(-kSlotEps), f2(kSlotHalf));
+    unsure0 = kNan ? !(fabsf(lo(f)) <= lo(m)) : fabsf(lo(f)) > lo(m);
+    unsure1 = kNan ? !(fabsf(hi(f)) <= hi(m)) : fabsf(hi(f)) > hi(m);
+    return k;
+}
+__device__ __forceinline__ F2 slot_sq(F2 ns, const DevParams& P, const float* __restrict__ tables)
+{
+    const float d0 = sqrt_guess(-lo(ns)), d1 = sqrt_guess(-hi(ns));
+    bool u0, u1;
+    F2 k = slot_from<true>(f2(-d0, -d1), P.inv_step, u0, u1);
+    if (u0 || u1) {
+        const float* th = tables + kThresh2Offset;
+        k = f2((float)table_slot_sq_from(-lo(ns), d0, P.inv_step, th),
+               (float)table_slot_sq_from(-hi(ns), d1, P.inv_step, th));
+    }
+    return k;
+}
+__device__ __forceinline__ F2 slot_dist(F2 nd, const DevParams& P, const float* __restrict__ tables)
+{
+    bool u0, u1;
+    F2 k = slot_from<false>(nd, P.inv_step, u0, u1);
+    if (u0 || u1) {
+        const float* th = tables + kThreshOffset;
+        k = f2((float)table_slot(-lo(nd), P.inv_step, th), (float)table_slot(-hi(nd), P.inv_step, th));
+    }
+    return k;
+}
+// weight_w of two negated squared distances, weight_sdw of two negated distances.
+__device__ __forceinline__ F2 weight_w(F2 ns, const DevParams& P, const float* __restrict__ tables)
+{
+    const F2 d = slot_sq(ns, P, tables) * f2(P.step);
+    const F2 t = f2(P.h2) - d * d;
+    const F2 w = f2(P.kw) * t * t * t;
+    return f2(!(-lo(ns) >= P.cut2) ? lo(w) : 0.f, !(-hi(ns) >= P.cut2) ? hi(w) : 0.f);
+}
+__device__ __forceinline__ F2 weight_sdw(F2 nd, const DevParams& P, const float* __restrict__ tables)
+{
+    const F2 s = f2(P.h) - slot_dist(nd, P, tables) * f2(P.step);
+    const F2 w = f2(P.ksdw) * s * s;
+    return f2(!(-lo(nd) >= P.h) ? lo(w) : 0.f, !(-hi(nd) >= P.h) ? hi(w) : 0.f);
+}
+// NonpressureWeights of two negated squared distances.
+struct NonpressureWeights2 {
+    F2 dw, d2w, vd2w;
+    __device__ __forceinline__ NonpressureWeights2(F2 ns, const DevParams& P, const float* __restrict__ tables)
+    {
+        const F2 d = slot_sq(ns, P, tables) * f2(P.step);
+        const F2 t = f2(P.h2) - d * d;
+        const bool in0 = !(-lo(ns) >= P.cut2), in1 = !(-hi(ns) >= P.cut2);
+        const F2 a = f2(P.kdw) * t * t;
+        const F2 b = f2(P.kd2w) * t * (f2(3.f * P.h2) - f2(7.f) * d * d);
+        const F2 c = f2(P.kvd2w) * (f2(P.h) - d);
+        dw = f2(in0 ? lo(a) : 0.f, in1 ? hi(a) : 0.f);
+        d2w = f2(in0 ? lo(b) : 0.f, in1 ? hi(b) : 0.f);
+        vd2w = f2(in0 ? lo(c) : 0.f, in1 ? hi(c) : 0.f);
     }
 };
 
@@ -364,11 +557,11 @@ __device__ __forceinline__ int list_entry(const int32_t* __restrict__ nbr, int64
     return nbr[(((int64_t)(k >> 2) * stride + i) << 2) + (k & 3)];
 }
 
-// for_each_neighbor (B = 2) over particle i's plain column-major list `src` (entry k at
-// src[k * stride + i]) that also stores the list in list_entry's grouped layout at `dst`: every
-// second pair of entries completes a group, which goes out as one 16-byte store (all lanes store
-// in step, so the stores coalesce), and the next pair's indices are in flight while the current
-// pair's records are fetched and its pairs computed, as in for_each_neighbor.
+// Walks particle i's plain column-major list `src` (entry k at src[k * stride + i]) two entries
+// at a time and stores it in list_entry's grouped layout at `dst`: every second pair of entries
+// completes a group, which goes out as one 16-byte store (all lanes store in step, so the stores
+// coalesce), and the next pair's indices are in flight while the current pair's records are
+// fetched and its pairs computed. f(j0, record, j1, record, two) as in for_each_neighbor.
 template <typename Load, typename F>
 __device__ __forceinline__ void for_each_neighbor_regroup(const int32_t* __restrict__ src, int32_t* __restrict__ dst,
                                                           int i, int64_t stride, int cnt, Load load, F f)
@@ -399,8 +592,7 @@ __device__ __forceinline__ void for_each_neighbor_regroup(const int32_t* __restr
             p0 = j0;
             p1 = j1;
         }
-        f(j0, r0);
-        f(j1, r1);
+        f(j0, r0, j1, r1, true);
         j0 = n0;
         j1 = n1;
     }
@@ -409,46 +601,58 @@ __device__ __forceinline__ void for_each_neighbor_regroup(const int32_t* __restr
     if (cnt & 1) {
         const int jj = __ldg(l);
         *reinterpret_cast<int4*>(g) = (full & 1) ? make_int4(p0, p1, jj, 0) : make_int4(jj, 0, 0, 0);
-        f(jj, load(jj));
+        const auto r = load(jj);
+        f(jj, r, jj, r, false);
     } else if (full & 1) {
         *reinterpret_cast<int4*>(g) = make_int4(p0, p1, 0, 0);
     }
 }
 
-// Walks particle i's neighbour list in list order, software pipelined: while a group's
-// records are fetched and its pairs computed (B records at a time, B = 1, 2 or 4), the next
-// group's four indices are already in flight, so the list's DRAM latency overlaps the
-// arithmetic. f(j, record) runs strictly in list order, so every sum accumulates in the
-// reference's order.
+// Walks particle i's neighbour list in list order, two entries per call of f, software
+// pipelined: while a group's records are fetched and its pairs computed (B records at a time,
+// B = 2 or 4), the next group's four indices are already in flight, so the list's DRAM latency
+// overlaps the arithmetic. f(j0, record0, j1, record1, two) runs in list order and must add
+// entry j0's terms before j1's, so every sum accumulates in the reference's order; when `two`
+// is false (an odd last entry) the second entry repeats the first and adds nothing.
 template <int B, typename Load, typename F>
 __device__ __forceinline__ void for_each_neighbor(const int32_t* __restrict__ nbr, int i, int64_t stride, int cnt,
                                                   Load load, F f)
 {
-    static_assert(B == 1 || B == 2 || B == 4, "a walk batch divides the 4-entry group");
+    static_assert(B == 2 || B == 4, "a walk batch divides the 4-entry group");
     const int4* g = reinterpret_cast<const int4*>(nbr) + i;
-    const int full = cnt >> 2;
-    const int rest = cnt & 3;
+    const int groups = (cnt + 3) >> 2;
     int4 cur = make_int4(0, 0, 0, 0);
     if (cnt > 0) cur = __ldg(g);
-    for (int q = 0; q < full; q++) {
+    for (int q = 0; q < groups; q++) {
+        const int left = cnt - 4 * q;   // entries of this group and after
+        if (left < 4) {
+            // The last, partial group: its unused components are not indices.
+            if (left < 2) cur.y = cur.x;
+            cur.z = left > 2 ? cur.z : cur.x;
+            cur.w = cur.z;
+        }
         g += stride;
         int4 nxt = make_int4(0, 0, 0, 0);
-        if (q + 1 < full || rest) nxt = __ldg(g);
-        const int j[4] = {cur.x, cur.y, cur.z, cur.w};
-#pragma unroll
-        for (int s0 = 0; s0 < 4; s0 += B) {
-            decltype(load(0)) r[B];
-#pragma unroll
-            for (int u = 0; u < B; u++) r[u] = load(j[s0 + u]);
-#pragma unroll
-            for (int u = 0; u < B; u++) f(j[s0 + u], r[u]);
+        if (q + 1 < groups) nxt = __ldg(g);
+        if (B == 4) {
+            const auto r0 = load(cur.x);
+            const auto r1 = load(cur.y);
+            const auto r2 = load(cur.z);
+            const auto r3 = load(cur.w);
+            f(cur.x, r0, cur.y, r1, left > 1);
+            if (left > 2) f(cur.z, r2, cur.w, r3, left > 3);
+        } else {
+            const auto r0 = load(cur.x);
+            const auto r1 = load(cur.y);
+            f(cur.x, r0, cur.y, r1, left > 1);
+            if (left > 2) {
+                const auto r2 = load(cur.z);
+                const auto r3 = load(cur.w);
+                f(cur.z, r2, cur.w, r3, left > 3);
+            }
         }
         cur = nxt;
     }
-    // The last, partial group: its first `rest` components.
-    if (rest > 0) f(cur.x, load(cur.x));
-    if (rest > 1) f(cur.y, load(cur.y));
-    if (rest > 2) f(cur.z, load(cur.z));
 }
 
 // Cell coordinate of the reference's CPU grid (SPHSpatialGrid.cpp:80-82).

@@ -9,31 +9,6 @@
 
 namespace lsp {
 
-// T_THRESH: slot thresholds on the distance; T_THRESH2: on the squared distance.
-enum { T_W = 0, T_DW = 1, T_D2W = 2, T_SPIKY_DW = 3, T_VISC_D2W = 4, T_THRESH = 5, T_THRESH2 = 6 };
-
-// Copies table t (the threshold tables have one entry more) into shared memory.
-__device__ __forceinline__ void stage_table(float* sm, const float* g, int t)
-{
-    const int len = t >= T_THRESH ? kTableSize + 1 : kTableSize;
-    const int off = t == T_THRESH2 ? kThresh2Offset : t * kTableSize;
-    for (int i = threadIdx.x; i < len; i += blockDim.x) sm[i] = g[off + i];
-}
-// The non-pressure pass's slot records (NonpressureWeights), built in shared memory from
-// the table block g.
-__device__ __forceinline__ void stage_nonpressure_slots(float4* ra, float4* rb, const float* g)
-{
-    const float* th = g + kThresh2Offset;
-    const float* dw = g + T_DW * kTableSize;
-    const float* d2w = g + T_D2W * kTableSize;
-    const float* vd2w = g + T_VISC_D2W * kTableSize;
-    for (int k = threadIdx.x; k < kTableSize; k += blockDim.x) {
-        const int km = k ? k - 1 : 0;
-        ra[k] = make_float4(th[k], dw[km], dw[k], d2w[km]);
-        rb[k] = make_float4(d2w[k], vd2w[km], vd2w[k], 0.f);
-    }
-}
-
 // Cell key of a position inside the scene's grid box: the CPU grid's cell (int)(x / h)
 // per axis (SPHSpatialGrid.cpp:80-82), clamped into the box, ordered x slowest and z
 // fastest, plus the scene's first cell in a batch.
@@ -64,7 +39,7 @@ __device__ __forceinline__ uint32_t cell_key(const DevParams& P, const float4& p
 template <bool kDensity = false, bool kTail0 = false>
 __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* __restrict__ pos,
                                              const uint32_t* __restrict__ cell_start, int32_t* __restrict__ nbr,
-                                             int i, const float* W = nullptr, const float* TH2 = nullptr,
+                                             int i, const float* __restrict__ tables = nullptr,
                                              float* wsum = nullptr)
 {
     float sum = 0.f;
@@ -100,7 +75,7 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
                     const V3 dq = xi - v3(*pq);
                     const float s = sqmag(dq);
                     if (s <= P.h2) {
-                        if (kDensity) sum += lookup_sq<kTail0>(W, TH2, s, P);
+                        if (kDensity) sum += weight_w(s, P, tables);
                         if (c < cap) {
                             *out = q;
                             out += stride;
@@ -161,39 +136,21 @@ __device__ __forceinline__ void record_neighbor_count(const DevParams& P, int c,
     }
 }
 
-// SPHSolver::calcParticleDensityPressure, CPU branch (SPHSolver.cpp:442-463).
-// The distance serves only the table, so the lookup takes the squared distance (TH2: the
-// thresholds on d^2; the same slot and value as the reference's sqrt-then-divide).
-__device__ __forceinline__ void density_one(const DevParams& P, const StepBuffers& b, const float* W,
-                                            const float* TH2, int i)
-{
-    const V3 xi = v3(b.pos[i]);
-    float sum = 0.f;
-    for_each_neighbor<4>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i),
-                         [&](int j) { return b.pos[j]; },
-                         [&](int, float4 pj) { sum += lookup_sq(W, TH2, sqmag(v3(pj) - xi), P); });
-    float rho = P.mass * sum;
-    float pr = P.stiffness * (rho - P.rho0);
-    if (pr < 0.f) pr *= P.neg;
-    b.rho[i] = rho;
-    b.pres[i] = pr;
-}
-
 // SPHSolver::accumulateNonPressureForces, CPU branch (SPHSolver.cpp:201-248). The
 // reference walks the list up to three times (normal, colour Laplacian when the normal
 // exceeds the threshold, viscosity); each sum is independent, so one walk computes all
 // three with the same per-sum rounding. kGrad adds |grad rho|, a warm-start feature. The
-// distance serves only the tables (the normal sums the unnormalised difference), so the
-// slot comes from the squared distance (slot records NA / NB on d^2).
+// distance serves only the weights (the normal sums the unnormalised difference), so the
+// slot comes from the squared distance.
 //
 // With kExactDiv its seven quotients by the neighbour density per pair come from one
-// reciprocal of rho_j (recip_rn, div_by): the same bits while the step's positions,
-// velocities and densities are in range (DevStatus::np_unsafe clear) and the tables' entries
-// are (DevParams::exact_tables), since every numerator is then 0 or at least 2^-80 in
-// magnitude (nonpressure_one chooses).
+// reciprocal of rho_j (recip_rn, div_by), two pairs at a time: the same bits while the step's
+// positions, velocities and densities are in range (DevStatus::np_unsafe clear) and the tables'
+// entries are (DevParams::exact_tables), since every numerator is then 0 or at least 2^-80 in
+// magnitude (nonpressure_one chooses). The particle itself then adds a zero to the viscosity
+// sum, which starts at +0 and is left unchanged, so it needs no test.
 template <bool kGrad, bool kExactDiv>
-__device__ __forceinline__ void nonpressure_walk(const DevParams& P, const StepBuffers& b, const float4* NA,
-                                                 const float4* NB, int i)
+__device__ __forceinline__ void nonpressure_walk(const DevParams& P, const StepBuffers& b, int i)
 {
     const V3 xi = v3(b.pos[i]);
     const V3 vi = v3(b.vel[i]);
@@ -207,32 +164,49 @@ __device__ __forceinline__ void nonpressure_walk(const DevParams& P, const StepB
     struct Rec {
         float4 x, vr;   // position; velocity and density ({v, rho}, StepBuffers::vrho)
     };
-    for_each_neighbor_regroup(b.nbr_src, b.nbr_out, i, P.nbr_stride, __ldg(b.nbr_count + i),
-                         [&](int j) { return Rec{b.pos[j], b.vrho[j]}; },
-                         [&](int j, const Rec& r) {
-                             const V3 xj = v3(r.x);
-                             V3 dir = xi - xj;
-                             // |x_i - x_j|^2 equals |x_j - x_i|^2 bit for bit
-                             const NonpressureWeights at(NA, NB, sqmag(dir), P);
-                             const float w_dw = at.dw;
-                             if (kExactDiv) {
-                                 const float y = recip_rn(r.vr.w);
-                                 auto q = [&](float a) { return div_by(a, r.vr.w, y); };
-                                 const V3 n = dir * w_dw;
-                                 normal += v3(q(n.x), q(n.y), q(n.z));
-                                 lap += q(at.d2w);
-                                 if (j != i) {
-                                     const V3 dv = v3(r.vr) - vi;
-                                     visc += v3(q(dv.x), q(dv.y), q(dv.z)) * at.vd2w;
-                                 }
-                                 if (kGrad) grad += dir * (w_dw * q(r.vr.w - rhoi));
-                             } else {
-                                 normal += dir * w_dw / r.vr.w;
-                                 lap += at.d2w / r.vr.w;
-                                 if (j != i) visc += ((v3(r.vr) - vi) / r.vr.w) * at.vd2w;
-                                 if (kGrad) grad += dir * (w_dw * ((r.vr.w - rhoi) / r.vr.w));
-                             }
-                         });
+    auto load = [&](int j) { return Rec{b.pos[j], b.vrho[j]}; };
+    auto one = [&](int j, const Rec& r) {
+        V3 dir = xi - v3(r.x);
+        // |x_i - x_j|^2 equals |x_j - x_i|^2 bit for bit
+        const NonpressureWeights at(sqmag(dir), P, b.tables);
+        normal += dir * at.dw / r.vr.w;
+        lap += at.d2w / r.vr.w;
+        if (j != i) visc += ((v3(r.vr) - vi) / r.vr.w) * at.vd2w;
+        if (kGrad) grad += dir * (at.dw * ((r.vr.w - rhoi) / r.vr.w));
+    };
+    auto pair = [&](int j0, const Rec& r0, int j1, const Rec& r1, bool two) {
+        if (!kExactDiv) {
+            one(j0, r0);
+            if (two) one(j1, r1);
+            return;
+        }
+        const F2 dx = f2(xi.x - r0.x.x, xi.x - r1.x.x), dy = f2(xi.y - r0.x.y, xi.y - r1.x.y),
+                 dz = f2(xi.z - r0.x.z, xi.z - r1.x.z);
+        const NonpressureWeights2 at(neg_sqmag(dx, dy, dz), P, b.tables);
+        const F2 nrho = f2(-r0.vr.w, -r1.vr.w);
+        const F2 y = recip_rn(nrho);
+        auto q = [&](F2 a) { return div_by(a, nrho, y); };
+        const F2 nx = q(dx * at.dw), ny = q(dy * at.dw), nz = q(dz * at.dw), l = q(at.d2w);
+        const F2 wx = q(f2(r0.vr.x - vi.x, r1.vr.x - vi.x)) * at.vd2w,
+                 wy = q(f2(r0.vr.y - vi.y, r1.vr.y - vi.y)) * at.vd2w,
+                 wz = q(f2(r0.vr.z - vi.z, r1.vr.z - vi.z)) * at.vd2w;
+        normal += v3(lo(nx), lo(ny), lo(nz));
+        lap += lo(l);
+        visc += v3(lo(wx), lo(wy), lo(wz));
+        F2 g;
+        if (kGrad) {
+            g = at.dw * q(f2(r0.vr.w - rhoi, r1.vr.w - rhoi));
+            const F2 gx = dx * g, gy = dy * g, gz = dz * g;
+            grad += v3(lo(gx), lo(gy), lo(gz));
+            if (two) grad += v3(hi(gx), hi(gy), hi(gz));
+        }
+        if (two) {
+            normal += v3(hi(nx), hi(ny), hi(nz));
+            lap += hi(l);
+            visc += v3(hi(wx), hi(wy), hi(wz));
+        }
+    };
+    for_each_neighbor_regroup(b.nbr_src, b.nbr_out, i, P.nbr_stride, __ldg(b.nbr_count + i), load, pair);
     if (kGrad) b.gradrho[i] = P.mass * mag(grad);
     normal *= P.mass;
     float len = mag(normal);
@@ -242,18 +216,16 @@ __device__ __forceinline__ void nonpressure_walk(const DevParams& P, const StepB
     b.force[i] = f4(F, 0.f);
 }
 template <bool kGrad>
-__device__ __forceinline__ void nonpressure_one(const DevParams& P, const StepBuffers& b, const float4* NA,
-                                                const float4* NB, int i)
+__device__ __forceinline__ void nonpressure_one(const DevParams& P, const StepBuffers& b, int i)
 {
     if (P.exact_tables && *(const volatile uint32_t*)&b.status->np_unsafe == 0u)
-        nonpressure_walk<kGrad, true>(P, b, NA, NB, i);
+        nonpressure_walk<kGrad, true>(P, b, i);
     else
-        nonpressure_walk<kGrad, false>(P, b, NA, NB, i);
+        nonpressure_walk<kGrad, false>(P, b, i);
 }
 
 // SPHSolver::accumulatePressureForces, CPU branch (SPHSolver.cpp:268-290).
-__device__ __forceinline__ void sph_pressure_one(const DevParams& P, const StepBuffers& b, const float* SDW,
-                                                 const float* TH, int i)
+__device__ __forceinline__ void sph_pressure_one(const DevParams& P, const StepBuffers& b, int i)
 {
     const V3 xi = v3(b.pos[i]);
     const float rhoi = b.rho[i];
@@ -263,14 +235,18 @@ __device__ __forceinline__ void sph_pressure_one(const DevParams& P, const StepB
         float4 x;
         float rho, p;
     };
+    auto one = [&](int j, const Rec& r) {
+        if (j == i) return;
+        const V3 xj = v3(r.x);
+        float d = mag(xi - xj);
+        V3 dir = (xi - xj) / d;
+        pf += dir * weight_sdw(d, P, b.tables) * (tf + r.p / (r.rho * r.rho));
+    };
     for_each_neighbor<4>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i),
                          [&](int j) { return Rec{b.pos[j], b.rho[j], b.pres[j]}; },
-                         [&](int j, const Rec& r) {
-                             if (j == i) return;
-                             const V3 xj = v3(r.x);
-                             float d = mag(xi - xj);
-                             V3 dir = (xi - xj) / d;
-                             pf += dir * lookup(SDW, TH, d, P) * (tf + r.p / (r.rho * r.rho));
+                         [&](int j0, const Rec& r0, int j1, const Rec& r1, bool two) {
+                             one(j0, r0);
+                             if (two) one(j1, r1);
                          });
     pf *= -(P.mass * rhoi);
     V3 F = v3(b.force[i]);
@@ -339,18 +315,29 @@ __device__ __forceinline__ void pci_predict_one(const DevParams& P, const StepBu
     }
 }
 
-// PCISPHSolver.cpp:100-126 for one particle; returns |error| (0 for NaN, which the
-// reference's std::max ignores). Table lookups on the squared distance (TH2), as in
-// density_one (kTail0: DevParams::density_tail0 holds).
-template <bool kTail0 = false>
-__device__ __forceinline__ float pci_density_one(const DevParams& P, const StepBuffers& b, const float* W,
-                                                 const float* TH2, int i, int iteration, float4* ppos)
+// Sum of W over particle i's list at the positions x (a W of exactly 0 or more each: adding the
+// +0 of a masked second entry changes no bit).
+__device__ __forceinline__ float density_sum(const DevParams& P, const StepBuffers& b, const float4* x, int i)
 {
-    const V3 xi = v3(ppos[i]);
+    const V3 xi = v3(x[i]);
     float sum = 0.f;
-    for_each_neighbor<4>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i),
-                         [&](int j) { return ppos[j]; },
-                         [&](int, float4 pj) { sum += lookup_sq<kTail0>(W, TH2, sqmag(v3(pj) - xi), P); });
+    for_each_neighbor<4>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i), [&](int j) { return x[j]; },
+                         [&](int, float4 p, int, float4 q, bool two) {
+                             const F2 w = weight_w(neg_sqmag(f2(p.x - xi.x, q.x - xi.x), f2(p.y - xi.y, q.y - xi.y),
+                                                             f2(p.z - xi.z, q.z - xi.z)),
+                                                   P, b.tables);
+                             sum += lo(w);
+                             if (two) sum += hi(w);
+                         });
+    return sum;
+}
+
+// PCISPHSolver.cpp:100-126 for one particle; returns |error| (0 for NaN, which the
+// reference's std::max ignores).
+__device__ __forceinline__ float pci_density_one(const DevParams& P, const StepBuffers& b, int i, int iteration,
+                                                 float4* ppos)
+{
+    const float sum = density_sum(P, b, ppos, i);
     float pd = P.mass * sum;
     float er = pd - P.rho0;
     float pp = P.delta * er;
@@ -376,41 +363,44 @@ __device__ __forceinline__ float pci_density_one(const DevParams& P, const StepB
 // with kExactDiv they come from sqrt_rn and one reciprocal of d (recip_rn, div_by), the same
 // bits for the predicted positions the step's predict passes found safe
 // (DevStatus::div_unsafe clear).
-template <bool kExactDiv, bool kTail0 = false>
-__device__ __forceinline__ void pci_force_walk(const DevParams& P, const StepBuffers& b, const float* SDW,
-                                               const float* TH, int i, const float4* ppos)
+template <bool kExactDiv>
+__device__ __forceinline__ void pci_force_walk(const DevParams& P, const StepBuffers& b, int i, const float4* ppos)
 {
     const float4 pi4 = ppos[i];
     const V3 xi = v3(pi4);
     const float tf = pi4.w;
     V3 pf = v3(0.f, 0.f, 0.f);
-    for_each_neighbor<2>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i),
-                         [&](int j) { return ppos[j]; },
-                         [&](int j, float4 pj4) {
-                             if (j == i) return;
-                             // |x_i - x_j| rounds exactly like the reference's |x_j - x_i|
-                             // (the squares are equal), so one difference serves both.
-                             const V3 dq = xi - v3(pj4);
-                             const float d = kExactDiv ? sqrt_rn(sqmag(dq)) : mag(dq);
-                             V3 dir;
-                             if (kExactDiv) {
-                                 const float y = recip_rn(d);
-                                 dir = v3(div_by(dq.x, d, y), div_by(dq.y, d, y), div_by(dq.z, d, y));
-                             } else {
-                                 dir = dq / d;
-                             }
-                             pf += dir * lookup<kTail0>(SDW, TH, d, P) * (tf + pj4.w);
-                         });
+    auto one = [&](int j, float4 pj4) {
+        if (j == i) return;
+        // |x_i - x_j| rounds exactly like the reference's |x_j - x_i|
+        // (the squares are equal), so one difference serves both.
+        const V3 dq = xi - v3(pj4);
+        const float d = mag(dq);
+        V3 dir = dq / d;
+        pf += dir * weight_sdw(d, P, b.tables) * (tf + pj4.w);
+    };
+    auto pair = [&](int j0, float4 p, int j1, float4 q, bool two) {
+        if (!kExactDiv) {
+            one(j0, p);
+            if (two) one(j1, q);
+            return;
+        }
+        const F2 dx = f2(xi.x - p.x, xi.x - q.x), dy = f2(xi.y - p.y, xi.y - q.y), dz = f2(xi.z - p.z, xi.z - q.z);
+        const F2 nd = neg_sqrt_rn(neg_sqmag(dx, dy, dz)), y = recip_rn(nd);
+        const F2 w = weight_sdw(nd, P, b.tables), s = f2(tf + p.w, tf + q.w);
+        const F2 fx = div_by(dx, nd, y) * w * s, fy = div_by(dy, nd, y) * w * s, fz = div_by(dz, nd, y) * w * s;
+        if (j0 != i) pf += v3(lo(fx), lo(fy), lo(fz));
+        if (two && j1 != i) pf += v3(hi(fx), hi(fy), hi(fz));
+    };
+    for_each_neighbor<2>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i), [&](int j) { return ppos[j]; }, pair);
     pf *= -(P.mass * b.rho[i]);
     if (isnan(pf.x)) pf = v3(0.f, 0.f, 0.f);
     b.pforce[i] = f4(pf, 0.f);
 }
-template <bool kTail0 = false>
-__device__ __forceinline__ void pci_force_one(const DevParams& P, const StepBuffers& b, const float* SDW,
-                                              const float* TH, int i, const float4* ppos)
+__device__ __forceinline__ void pci_force_one(const DevParams& P, const StepBuffers& b, int i, const float4* ppos)
 {
-    if (*(const volatile uint32_t*)&b.status->div_unsafe == 0u) pci_force_walk<true, kTail0>(P, b, SDW, TH, i, ppos);
-    else pci_force_walk<false, kTail0>(P, b, SDW, TH, i, ppos);
+    if (*(const volatile uint32_t*)&b.status->div_unsafe == 0u) pci_force_walk<true>(P, b, i, ppos);
+    else pci_force_walk<false>(P, b, i, ppos);
 }
 
 }  // namespace lsp

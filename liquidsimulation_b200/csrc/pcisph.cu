@@ -30,13 +30,9 @@ __global__ void __launch_bounds__(kThreads) k_pci_predict(DevParams P, StepBuffe
 
 __global__ void __launch_bounds__(kThreads) k_pci_density(DevParams P, StepBuffers b, int iteration)
 {
-    __shared__ float W[kTableSize], TH2[kTableSize + 1];
     __shared__ float wmax[kThreads / 32];
-    stage_table(W, b.tables, T_W);
-    stage_table(TH2, b.tables, T_THRESH2);
-    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float a = i < P.n ? pci_density_one(P, b, W, TH2, i, iteration, b.ppos) : 0.f;
+    float a = i < P.n ? pci_density_one(P, b, i, iteration, b.ppos) : 0.f;
     // Max of non-negative floats: their bit patterns order like the values.
     uint32_t m = __float_as_uint(a);
 #pragma unroll
@@ -52,13 +48,9 @@ __global__ void __launch_bounds__(kThreads) k_pci_density(DevParams P, StepBuffe
 
 __global__ void __launch_bounds__(kThreads) k_pci_force(DevParams P, StepBuffers b)
 {
-    __shared__ float SDW[kTableSize], TH[kTableSize + 1];
-    stage_table(SDW, b.tables, T_SPIKY_DW);
-    stage_table(TH, b.tables, T_THRESH);
-    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
-    pci_force_one(P, b, SDW, TH, i, b.ppos);
+    pci_force_one(P, b, i, b.ppos);
 }
 
 static inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -83,13 +75,9 @@ void launch_pci_force(const DevParams& P, const StepBuffers& b, cudaStream_t s)
 // until the network's guess replaces them (mlp_tc.cu).
 __global__ void __launch_bounds__(kThreads) k_pci_density_first(DevParams P, StepBuffers b, WarmArgs w)
 {
-    __shared__ float W[kTableSize], TH2[kTableSize + 1];
     __shared__ float wmax[kThreads / 32];
-    stage_table(W, b.tables, T_W);
-    stage_table(TH2, b.tables, T_THRESH2);
-    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const float a = density_first(P, b, w.feat, w.hist, w.gradrho, w.p_scale, W, TH2, i, i < P.n);
+    const float a = density_first(P, b, w.feat, w.hist, w.gradrho, w.p_scale, i, i < P.n);
     uint32_t m = __float_as_uint(a);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -132,19 +120,12 @@ void launch_pci_density_first(const DevParams& P, const StepBuffers& b, const Wa
 // One 1024-thread block per SM at 64 registers: measured about 10 % faster than the
 // unconstrained allocation (79 registers, 768 threads per SM; 1280 threads per SM are
 // slower too), and one block of 1024 beats two of 512 by 3.5 % and four of 256 by 4 % (a
-// grid barrier with 148 arrivals, one table copy per SM).
+// grid barrier with 148 arrivals).
 constexpr int kLoopThreads = 1024;
-template <bool kTail0>   // DevParams::density_tail0 && DevParams::force_tail0
 __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepBuffers b, float4* ppos_alt,
                                                              LoopSync* sy, uint32_t* maxerr, int first_done, int warm)
 {
-    __shared__ float W[kTableSize], SDW[kTableSize], TH[kTableSize + 1], TH2[kTableSize + 1];
     __shared__ float wmax[kLoopThreads / 32];
-    stage_table(W, b.tables, T_W);
-    stage_table(SDW, b.tables, T_SPIKY_DW);
-    stage_table(TH, b.tables, T_THRESH);
-    stage_table(TH2, b.tables, T_THRESH2);
-    __syncthreads();
     // x* of iteration parity 0 / 1. A select, not a two-pointer array: an array indexed by
     // the iteration lives in local memory, and reading it per particle cost the loop 3.8 %.
     auto pp = [&](int parity) { return parity ? ppos_alt : b.ppos; };
@@ -171,7 +152,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
     // density(k) over all particles; the block maximum of |error| goes to maxerr[slot].
     auto density_pass = [&](int k, int slot) {
         float m = 0.f;
-        for_particles([&](int i) { m = fmaxf(m, pci_density_one<kTail0>(P, b, W, TH2, i, k, pp(k & 1))); });
+        for_particles([&](int i) { m = fmaxf(m, pci_density_one(P, b, i, k, pp(k & 1))); });
         uint32_t mb = __float_as_uint(m);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, off));
@@ -213,7 +194,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
         const bool unverified = warm && !rejected && k == 0;
         const bool done = (conv && k + 1 >= P.min_it && !unverified) || (k + 1 >= P.max_it);
         for_particles([&](int i) {
-            pci_force_one<kTail0>(P, b, SDW, TH, i, pp(k & 1));
+            pci_force_one(P, b, i, pp(k & 1));
             // The last pass also integrates and collides the particle (SPHParticle::integrate
             // after the loop, PCISPHSolver.cpp:166-169): it reads only the particle's own
             // state and pressure force, which this thread has just written, and no thread of
@@ -237,12 +218,12 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
     }
 }
 
-// Per device, instance (kTail0) and block size (1024 / 512 / 256 / 128 threads): resident
+// Per device and block size (1024 / 512 / 256 / 128 threads): resident
 // blocks of k_pci_loop per SM (0: no cooperative launch).
 constexpr int kMaxDevices = 64;
 constexpr int kLoopShapes = 4;
 // Filled once per device under a lock (solvers on different host threads may launch at once).
-static int g_loop_blocks_per_sm[kMaxDevices][2][kLoopShapes];
+static int g_loop_blocks_per_sm[kMaxDevices][kLoopShapes];
 static bool g_loop_ready[kMaxDevices];
 static std::mutex g_loop_mutex;
 
@@ -267,22 +248,19 @@ bool launch_pci_loop(const DevParams& P, const StepBuffers& b, float4* ppos_alt,
     if (!g_loop_ready[dev]) {
         int coop = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-        for (int t = 0; t < 2; t++)
-            for (int k = 0; k < kLoopShapes; k++) {
-                int per = 0;
-                const void* fn = t ? (const void*)k_pci_loop<true> : (const void*)k_pci_loop<false>;
-                if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kLoopThreads >> k, 0) !=
-                                 cudaSuccess)
-                    per = 0;
-                g_loop_blocks_per_sm[dev][t][k] = per;
-            }
+        for (int k = 0; k < kLoopShapes; k++) {
+            int per = 0;
+            if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pci_loop, kLoopThreads >> k, 0) !=
+                             cudaSuccess)
+                per = 0;
+            g_loop_blocks_per_sm[dev][k] = per;
+        }
         g_loop_ready[dev] = true;
     }
     const int sms = device_sm_count();
     const int shape = loop_shape(P.n, sms);
     const int threads = kLoopThreads >> shape;
-    const int tail0 = (P.density_tail0 && P.force_tail0) ? 1 : 0;
-    const int per_sm = g_loop_blocks_per_sm[dev][tail0][shape];
+    const int per_sm = g_loop_blocks_per_sm[dev][shape];
     lock.unlock();
     if (per_sm <= 0) return false;
     int need = (int)((P.n + threads - 1) / threads);
@@ -291,8 +269,7 @@ bool launch_pci_loop(const DevParams& P, const StepBuffers& b, float4* ppos_alt,
     StepBuffers bc = b;
     LoopSync* sy = (LoopSync*)sync;
     void* args[] = {&Pc, &bc, &ppos_alt, &sy, &maxerr, &first_done, &warm};
-    const void* fn = tail0 ? (const void*)k_pci_loop<true> : (const void*)k_pci_loop<false>;
-    if (cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, 0, s) != cudaSuccess)
+    if (cudaLaunchCooperativeKernel((const void*)k_pci_loop, dim3(grid), dim3(threads), args, 0, s) != cudaSuccess)
         return false;
     if (grid_used) *grid_used = grid;
     return true;
