@@ -79,12 +79,13 @@ __global__ void __launch_bounds__(T) kb_neighbors_density(BatchArgs a, const flo
     const BatchItem it = a.items[blockIdx.x];
     stage_params(&P, a.sp, it.scene);
     __syncthreads();
+    extern __shared__ uint2 masks[];
     const int i = it.begin + (int)threadIdx.x;
     const bool valid = i < it.end;
     int c = 0;
     if (valid) {
         float sum;
-        c = neighbors_one<true>(P, pos, cell_start, nbr, i, scene_tables(a, it.scene), &sum);
+        c = neighbors_one(P, pos, cell_start, nbr, i, scene_tables(a, it.scene), masks + threadIdx.x, &sum);
         count[i] = min(c, P.nbr_cap);
         const float r = P.mass * sum;
         float pr = P.stiffness * (r - P.rho0);
@@ -411,13 +412,26 @@ int launch_batch_keys(const BatchArgs& a, const float4* pos, uint32_t* key, uint
     return 1;
 }
 
+// Above 48 KB of shared memory, its static part included (T = 512 and 1024), a kernel has to be
+// told.
+template <int T>
+static bool scan_smem_ready()
+{
+    return scan_smem(T) + sizeof(DevParams) <= 48 * 1024 ||
+           cudaFuncSetAttribute(kb_neighbors_density<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)scan_smem(T)) == cudaSuccess;
+}
+
 int launch_batch_neighbors_density(const BatchArgs& a, const float4* pos, const uint32_t* cell_start, int32_t* nbr,
                                    int32_t* count, float* rho, float* pres, const float4* vel, float4* vrho,
                                    cudaStream_t s)
 {
     if (!a.items_count) return 0;
-    LSP_BATCH_DISPATCH(a.threads, (kb_neighbors_density<T><<<a.items_count, T, 0, s>>>(a, pos, cell_start, nbr,
-                                                                                      count, rho, pres, vel, vrho)));
+    bool ok = false;
+    LSP_BATCH_DISPATCH(a.threads, (ok = scan_smem_ready<T>()));
+    if (!ok) return 0;
+    LSP_BATCH_DISPATCH(a.threads, (kb_neighbors_density<T><<<a.items_count, T, scan_smem(T), s>>>(
+                                      a, pos, cell_start, nbr, count, rho, pres, vel, vrho)));
     return 1;
 }
 

@@ -18,9 +18,8 @@
 //   k_scatter     particle -> (cell start + slot)
 //   k_rank_gather deterministic rank by caller id inside each cell, then one gather of
 //                 the 64-byte persistent state into the new order
-//   k_neighbors_density  the start-of-step neighbour lists (plain column-major; the
-//                 non-pressure pass regroups them), reference order, with the density and
-//                 pressure summed over the accepted pairs
+//   k_neighbors_density  the start-of-step neighbour lists, reference order, with the density
+//                 and pressure summed over the accepted pairs
 #include "lsp_kernels.h"
 #include "particle_ops.cuh"
 
@@ -209,7 +208,7 @@ __global__ void k_rank_gather(DevParams P, const int2* __restrict__ tmp, const u
     sorted_key[dest] = k;
 }
 
-// Start-of-step neighbour lists (neighbors_one, plain column-major) plus the start-of-step density
+// Start-of-step neighbour lists (neighbors_one) plus the start-of-step density
 // and pressure (SPHSolver::calcParticleDensityPressure,
 // SPHSolver.cpp:442-463), summed while the list is built: a pass over the stored list and
 // its position gathers would cost more. (A list that
@@ -223,10 +222,11 @@ __global__ void k_neighbors_density(DevParams P, const float4* __restrict__ pos,
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < P.n;
+    extern __shared__ uint2 masks[];
     int c = 0;
     if (valid) {
         float sum;
-        c = neighbors_one<true>(P, pos, cell_start, nbr, i, tables, &sum);
+        c = neighbors_one(P, pos, cell_start, nbr, i, tables, masks + threadIdx.x, &sum);
         count[i] = min(c, P.nbr_cap);
         const float r = P.mass * sum;
         float pr = P.stiffness * (r - P.rho0);
@@ -311,7 +311,7 @@ int launch_neighbors(const GridBuildArgs& a, cudaStream_t s)
 {
     const int T = 256;
     if (a.P.n <= 0) return 0;
-    k_neighbors_density<<<blocks_for(a.P.n, T), T, 0, s>>>(a.P, a.pos_out, a.cell_start, a.nbr, a.nbr_count, a.status,
+    k_neighbors_density<<<blocks_for(a.P.n, T), T, scan_smem(T), s>>>(a.P, a.pos_out, a.cell_start, a.nbr, a.nbr_count, a.status,
                                                            a.tables, a.rho, a.pres, a.vel_out, a.vrho);
     return 1;
 }

@@ -549,63 +549,10 @@ __device__ __forceinline__ void collide_all(const Collider* cols, int ncoll, V3&
 // Neighbour-list layout: entry k of particle i is component k & 3 of the int4 at group k >> 2,
 // and each group is column-major over the particles (group g of particle i at
 // ((int4*)nbr)[g * stride + i]). A reader fetches four indices with one coalesced 16-byte
-// load. The neighbour build writes plain column-major lists (one 4-byte store per accepted
-// entry, the cheapest for its accept branch) and the non-pressure pass, which walks every
-// list first, stores them in this layout (for_each_neighbor_regroup).
+// load. The unused components of a list's last group hold the particle's own index.
 __device__ __forceinline__ int list_entry(const int32_t* __restrict__ nbr, int64_t stride, int64_t i, int k)
 {
     return nbr[(((int64_t)(k >> 2) * stride + i) << 2) + (k & 3)];
-}
-
-// Walks particle i's plain column-major list `src` (entry k at src[k * stride + i]) two entries
-// at a time and stores it in list_entry's grouped layout at `dst`: every second pair of entries
-// completes a group, which goes out as one 16-byte store (all lanes store in step, so the stores
-// coalesce), and the next pair's indices are in flight while the current pair's records are
-// fetched and its pairs computed. f(j0, record, j1, record, two) as in for_each_neighbor.
-template <typename Load, typename F>
-__device__ __forceinline__ void for_each_neighbor_regroup(const int32_t* __restrict__ src, int32_t* __restrict__ dst,
-                                                          int i, int64_t stride, int cnt, Load load, F f)
-{
-    const int32_t* l = src + i;
-    int32_t* g = dst + 4 * (int64_t)i;   // the current group of particle i
-    const int full = cnt >> 1;
-    int j0 = 0, j1 = 0;
-    if (full > 0) {
-        j0 = __ldg(l);
-        j1 = __ldg(l + stride);
-        l += 2 * stride;
-    }
-    int p0 = 0, p1 = 0;   // the first pair of the current group
-    for (int b = 0; b < full; b++) {
-        const auto r0 = load(j0);
-        const auto r1 = load(j1);
-        int n0 = 0, n1 = 0;
-        if (b + 1 < full) {
-            n0 = __ldg(l);
-            n1 = __ldg(l + stride);
-            l += 2 * stride;
-        }
-        if (b & 1) {
-            *reinterpret_cast<int4*>(g) = make_int4(p0, p1, j0, j1);
-            g += 4 * stride;
-        } else {
-            p0 = j0;
-            p1 = j1;
-        }
-        f(j0, r0, j1, r1, true);
-        j0 = n0;
-        j1 = n1;
-    }
-    // The last, partial group: a pending pair and / or the odd last entry (its unused
-    // components are never read).
-    if (cnt & 1) {
-        const int jj = __ldg(l);
-        *reinterpret_cast<int4*>(g) = (full & 1) ? make_int4(p0, p1, jj, 0) : make_int4(jj, 0, 0, 0);
-        const auto r = load(jj);
-        f(jj, r, jj, r, false);
-    } else if (full & 1) {
-        *reinterpret_cast<int4*>(g) = make_int4(p0, p1, 0, 0);
-    }
 }
 
 // Walks particle i's neighbour list in list order, two entries per call of f, software
@@ -613,37 +560,27 @@ __device__ __forceinline__ void for_each_neighbor_regroup(const int32_t* __restr
 // B = 2 or 4), the next group's four indices are already in flight, so the list's DRAM latency
 // overlaps the arithmetic. f(j0, record0, j1, record1, two) runs in list order and must add
 // entry j0's terms before j1's, so every sum accumulates in the reference's order; when `two`
-// is false (an odd last entry) the second entry repeats the first and adds nothing.
+// is false (an odd last entry) the second entry is the particle itself and adds nothing.
 template <int B, typename Load, typename F>
 __device__ __forceinline__ void for_each_neighbor(const int32_t* __restrict__ nbr, int i, int64_t stride, int cnt,
                                                   Load load, F f)
 {
     static_assert(B == 2 || B == 4, "a walk batch divides the 4-entry group");
     const int4* g = reinterpret_cast<const int4*>(nbr) + i;
-    const int groups = (cnt + 3) >> 2;
-    int4 cur = make_int4(0, 0, 0, 0);
+    int4 cur = make_int4(i, i, i, i);
     if (cnt > 0) cur = __ldg(g);
-    for (int q = 0; q < groups; q++) {
-        const int left = cnt - 4 * q;   // entries of this group and after
-        if (left < 4) {
-            // The last, partial group: its unused components are not indices.
-            if (left < 2) cur.y = cur.x;
-            cur.z = left > 2 ? cur.z : cur.x;
-            cur.w = cur.z;
-        }
+    for (int left = cnt; left > 0; left -= 4) {   // entries of this group and after
         g += stride;
-        int4 nxt = make_int4(0, 0, 0, 0);
-        if (q + 1 < groups) nxt = __ldg(g);
+        int4 nxt = cur;
+        if (left > 4) nxt = __ldg(g);
+        const auto r0 = load(cur.x);
+        const auto r1 = load(cur.y);
         if (B == 4) {
-            const auto r0 = load(cur.x);
-            const auto r1 = load(cur.y);
             const auto r2 = load(cur.z);
             const auto r3 = load(cur.w);
             f(cur.x, r0, cur.y, r1, left > 1);
             if (left > 2) f(cur.z, r2, cur.w, r3, left > 3);
         } else {
-            const auto r0 = load(cur.x);
-            const auto r1 = load(cur.y);
             f(cur.x, r0, cur.y, r1, left > 1);
             if (left > 2) {
                 const auto r2 = load(cur.z);

@@ -67,15 +67,8 @@ struct StepBuffers {
     float* err;
     float4* hist;             // warm-start pressure history, null when off
     float* gradrho;           // |grad rho|, null when off
-    // neighbours: the lists in list_entry's grouped layout (nbr), read by every walk after
-    // the non-pressure pass. The neighbour build writes them plain column-major (nbr_src,
-    // entry k of particle i at nbr_src[k * stride + i]: one 4-byte store per entry, the
-    // cheapest for its accept branch), and the non-pressure pass, which walks every list
-    // first, regroups them into nbr_out (the same memory as nbr) with 16-byte stores.
-    const int32_t* nbr;
+    const int32_t* nbr;       // neighbour lists in list_entry's layout
     const int32_t* nbr_count;
-    const int32_t* nbr_src;
-    int32_t* nbr_out;
     // {v.x, v.y, v.z, rho} of each particle, written by the neighbour build once rho is known:
     // the non-pressure pass gathers a neighbour's velocity and density with one 16-byte load.
     const float4* vrho;
@@ -84,6 +77,14 @@ struct StepBuffers {
     const Collider* colliders;
     DevStatus* status;
 };
+
+// The neighbour scan reads up to 3 positions past the last one (neighbors_one): position arrays
+// hold that many more.
+constexpr int kPosPad = 4;
+// Masks per thread that the neighbour scan keeps in dynamic shared memory (9 rows, and some to
+// spare), and their bytes for a block.
+constexpr int kScanChunks = 12;
+inline size_t scan_smem(int threads) { return (size_t)threads * kScanChunks * sizeof(uint2); }
 
 // Entries of the histogram and cell-table buffers for `n` live entries: the scan moves them
 // 8 at a time, so both are padded to a multiple of 8 (the padding stays zero); and the scan's

@@ -29,65 +29,132 @@ __device__ __forceinline__ uint32_t cell_key(const DevParams& P, const float4& p
     return P.cell_base + (uint32_t)(((uint32_t)c[0] * (uint32_t)P.ny + (uint32_t)c[1]) * (uint32_t)P.nz + (uint32_t)c[2]);
 }
 
-// Start-of-step neighbour list of particle i: every j with |x_i - x_j|^2 <= h^2,
-// including i, in the reference's order (SPHSpatialGrid::findNeighborParticles,
-// SPHSpatialGrid.cpp:39-76): cell ranges from (x -+ h) / h per axis, x then y rows,
-// each row a contiguous z-run of the sorted array. Stores at most nbr_cap entries and
-// returns the true count. With kDensity it also sums W over the accepted pairs in list
-// order from their squared distances, the sum density_one forms over the stored list
-// (|x_i - x_j|^2 equals |x_j - x_i|^2 bit for bit; W and TH2 as in density_one).
-template <bool kDensity = false, bool kTail0 = false>
+// Start-of-step neighbour list and density sum of particle i: every j with
+// |x_i - x_j|^2 <= h^2, including i, in the reference's order (SPHSpatialGrid::findNeighborParticles,
+// SPHSpatialGrid.cpp:39-76): cell ranges from (x -+ h) / h per axis, x then y rows, each row a
+// contiguous z-run of the sorted array. Stores at most nbr_cap entries in list_entry's layout
+// (the last group filled up with i itself) and returns the true count; *wsum is the sum of W
+// over the accepted pairs in list order, from their squared distances (|x_i - x_j|^2 equals
+// |x_j - x_i|^2 bit for bit).
+//
+// Two phases. The scan tests the rows' candidates, 32 at a time, into bit masks without a
+// branch: s - next_up(h^2) is negative exactly when s <= h^2 (a NaN's sign is clear), and a
+// funnel shift appends that sign to the mask, first candidate highest. The masks wait in a
+// column of shared memory per thread. Then the accepted entries are taken from the masks four
+// at a time, by all lanes in step: their positions are fetched again, W is evaluated for two
+// pairs at a time and the group of four goes out as one 16-byte store that coalesces over the
+// lanes. A scan that handles each accepted candidate at once runs that branch for 10 of 32 lanes
+// on average and scatters its 4-byte stores over as many lines, and its lists had to be regrouped
+// by the next pass. Build 0.254 -> 0.229 ms, non-pressure pass without the regrouping and loop
+// with the filled-up groups 1.16 -> 1.11 ms a step at 991,440 particles; 12,000 particles: build
+// 39 -> 21 us. It is bound by the L1 data pipe (84 % of its wavefronts: a candidate's 16-byte load takes
+// four to eight of them); 40 or 32 registers instead of 50 (6 or 8 blocks of 256 threads per SM) are
+// slower (0.238, 0.289 ms), the larger working set missing more in L1.
 __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* __restrict__ pos,
                                              const uint32_t* __restrict__ cell_start, int32_t* __restrict__ nbr,
-                                             int i, const float* __restrict__ tables = nullptr,
-                                             float* wsum = nullptr)
+                                             int i, const float* __restrict__ tables, uint2* col, float* wsum)
 {
-    float sum = 0.f;
-    const float4 pi = pos[i];
-    const V3 xi = v3(pi);
+    const int pitch = blockDim.x;
+    const V3 xi = v3(pos[i]);
     const float h = P.h;
-    int lo[3] = {(int)((xi.x - h) / h), (int)((xi.y - h) / h), (int)((xi.z - h) / h)};
-    int hi[3] = {(int)((xi.x + h) / h), (int)((xi.y + h) / h), (int)((xi.z + h) / h)};
+    int lo_[3] = {(int)((xi.x - h) / h), (int)((xi.y - h) / h), (int)((xi.z - h) / h)};
+    int hi_[3] = {(int)((xi.x + h) / h), (int)((xi.y + h) / h), (int)((xi.z + h) / h)};
     const int o[3] = {P.ox, P.oy, P.oz};
     const int d[3] = {P.nx, P.ny, P.nz};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         // Both ends clamped into the box: a particle outside it searches the edge cell
         // that holds every clamped particle.
-        lo[a] = min(max(lo[a], o[a]), o[a] + d[a] - 1) - o[a];
-        hi[a] = min(max(hi[a], o[a]), o[a] + d[a] - 1) - o[a];
+        lo_[a] = min(max(lo_[a], o[a]), o[a] + d[a] - 1) - o[a];
+        hi_[a] = min(max(hi_[a], o[a]), o[a] + d[a] - 1) - o[a];
     }
-    const int cap = P.nbr_cap;
+    const float above = __uint_as_float(__float_as_uint(P.h2) + 1u);   // the next float above h^2
+    int4* out = reinterpret_cast<int4*>(nbr) + i;
     const int64_t stride = P.nbr_stride;
-    // Plain column-major (entry c at nbr[c * stride + i]); the non-pressure pass regroups the
-    // lists into list_entry's layout for the walks after it.
-    int32_t* out = nbr + i;
-    int c = 0;
-    if (lo[2] <= hi[2]) {
-        for (int cx = lo[0]; cx <= hi[0]; cx++) {
-            for (int cy = lo[1]; cy <= hi[1]; cy++) {
-                uint32_t row = P.cell_base + ((uint32_t)cx * (uint32_t)P.ny + (uint32_t)cy) * (uint32_t)P.nz;
-                const uint32_t beg = cell_start[row + lo[2]];
-                const uint32_t end = cell_start[row + hi[2] + 1];
-                const float4* pe = pos + end;
-                int32_t q = (int32_t)beg;
-                for (const float4* pq = pos + beg; pq < pe; pq++, q++) {
-                    const V3 dq = xi - v3(*pq);
-                    const float s = sqmag(dq);
-                    if (s <= P.h2) {
-                        if (kDensity) sum += weight_w(s, P, tables);
-                        if (c < cap) {
-                            *out = q;
-                            out += stride;
+    float sum = 0.f;
+    int stored = 0, pending = 0, chunks = 0;   // entries taken from the masks, entries still in them
+    uint32_t m = 0;
+    int last = 0;   // candidate of the mask's bit 0
+    int next = 0;   // next chunk to take
+    auto take = [&]() {
+        if (m == 0u) {
+            const uint2 e = col[next * pitch];
+            next++;
+            last = (int)e.x;
+            m = e.y;
+        }
+        const int b = 31 - __clz((int)m);
+        m ^= 1u << b;
+        return last - b;
+    };
+    // Takes every waiting entry one by one; only when a list needs more masks than the column
+    // holds (rows of more than 32 particles).
+    auto drain = [&]() {
+        for (; pending > 0; pending--) {
+            const int q = take();
+            sum += weight_w(sqmag(xi - v3(pos[q])), P, tables);
+            if (stored < P.nbr_cap) reinterpret_cast<int32_t*>(out + (int64_t)(stored >> 2) * stride)[stored & 3] = q;
+            stored++;
+        }
+        next = chunks = 0;
+    };
+    if (lo_[2] <= hi_[2]) {
+        for (int cx = lo_[0]; cx <= hi_[0]; cx++) {
+            for (int cy = lo_[1]; cy <= hi_[1]; cy++) {
+                const uint32_t row = P.cell_base + ((uint32_t)cx * (uint32_t)P.ny + (uint32_t)cy) * (uint32_t)P.nz;
+                const int end = (int)cell_start[row + hi_[2] + 1];
+                for (int beg = (int)cell_start[row + lo_[2]]; beg < end; beg += 32) {
+                    const int len = min(end - beg, 32);
+                    const float4* p = pos + beg;
+                    uint32_t bits = 0;
+                    for (int k = 0; k < len; k += 4, p += 4) {
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const float s = sqmag(xi - v3(__ldg(p + u)));
+                            bits = __funnelshift_l(__float_as_uint(s - above), bits, 1);
                         }
-                        c++;
+                    }
+                    const int over = -len & 3;   // candidates tested past the row's end
+                    bits &= 0xffffffffu << over;
+                    if (bits) {
+                        if (chunks == kScanChunks) drain();
+                        col[chunks * pitch] = make_uint2((uint32_t)(beg + len + over - 1), bits);
+                        chunks++;
+                        pending += __popc(bits);
                     }
                 }
             }
         }
     }
-    if (kDensity) *wsum = sum;
-    return c;
+    if (stored) {
+        drain();
+        const int rest = -stored & 3;
+        for (int k = stored; k < stored + rest && k < P.nbr_cap; k++)
+            reinterpret_cast<int32_t*>(out + (int64_t)(k >> 2) * stride)[k & 3] = i;
+        *wsum = sum;
+        return stored;
+    }
+    for (int k = 0; k < pending; k += 4) {
+        const int left = pending - k;
+        int4 q = make_int4(i, i, i, i);
+        q.x = take();
+        if (left > 1) q.y = take();
+        if (left > 2) q.z = take();
+        if (left > 3) q.w = take();
+        const float4 a = __ldg(pos + q.x), b = __ldg(pos + q.y), c = __ldg(pos + q.z), e = __ldg(pos + q.w);
+        if (k < P.nbr_cap) *out = q;
+        out += stride;
+        const F2 w0 = weight_w(neg_sqmag(f2(a.x - xi.x, b.x - xi.x), f2(a.y - xi.y, b.y - xi.y), f2(a.z - xi.z, b.z - xi.z)),
+                               P, tables);
+        const F2 w1 = weight_w(neg_sqmag(f2(c.x - xi.x, e.x - xi.x), f2(c.y - xi.y, e.y - xi.y), f2(c.z - xi.z, e.z - xi.z)),
+                               P, tables);
+        sum += lo(w0);
+        if (left > 1) sum += hi(w0);
+        if (left > 2) sum += lo(w1);
+        if (left > 3) sum += hi(w1);
+    }
+    *wsum = sum;
+    return pending;
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt()
@@ -206,7 +273,7 @@ __device__ __forceinline__ void nonpressure_walk(const DevParams& P, const StepB
             visc += v3(hi(wx), hi(wy), hi(wz));
         }
     };
-    for_each_neighbor_regroup(b.nbr_src, b.nbr_out, i, P.nbr_stride, __ldg(b.nbr_count + i), load, pair);
+    for_each_neighbor<2>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i), load, pair);
     if (kGrad) b.gradrho[i] = P.mass * mag(grad);
     normal *= P.mass;
     float len = mag(normal);
