@@ -248,7 +248,8 @@ int lsp_mlp_gradient_static(lsp_solver* s, const float* features, const float* t
 int lsp_timer_mark(lsp_solver* s, int slot);
 int lsp_timer_elapsed(lsp_solver* s, int slot_a, int slot_b, float* ms);
 /* Per-kernel-class device time: with profiling on, every launch is bracketed by events on
- * the solver's stream. read: ms[k] and launches[k] for k < LSP_PROF_COUNT. */
+ * the solver's stream. read: ms[k] and launches[k] for k < LSP_PROF_COUNT. A small scene, whose
+ * step is otherwise one launch, runs as separate kernels (the same bits) while it is profiled. */
 #define LSP_PROF_GRID_SORT     0   /* cell keys and histogram (batches: the whole grid build) */
 #define LSP_PROF_NEIGHBORS     1
 #define LSP_PROF_DENSITY       2

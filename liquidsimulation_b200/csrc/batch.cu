@@ -85,17 +85,10 @@ __global__ void __launch_bounds__(T) kb_neighbors_density(BatchArgs a, const flo
     int c = 0;
     if (valid) {
         float sum;
-        c = neighbors_one(P, pos, cell_start, nbr, i, scene_tables(a, it.scene), masks + threadIdx.x, &sum);
-        count[i] = min(c, P.nbr_cap);
-        const float r = P.mass * sum;
-        float pr = P.stiffness * (r - P.rho0);
-        if (pr < 0.f) pr *= P.neg;
-        rho[i] = r;
-        pres[i] = pr;
-        const float4 v = vel[i];
-        vrho[i] = make_float4(v.x, v.y, v.z, r);
-        // Batch-wide, like the rest of the non-pressure pass's range checks (k_rank_gather).
-        if (!exact_div_density(r)) atomicOr(&a.st[a.scenes].np_unsafe, 1u);
+        c = neighbors_one(P, pos, cell_start, nbr, i, scene_tables(a, it.scene), masks + threadIdx.x, T, &sum);
+        // The range check of the density is batch-wide, like the rest of the non-pressure pass's
+        // (rank_gather_one).
+        store_density(P, i, c, sum, vel, count, rho, pres, vrho, a.st + a.scenes);
     }
     record_neighbor_count(P, c, valid, a.st + it.scene);
 }
@@ -254,6 +247,7 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
     __shared__ int warp_sums[32];
     LoopSync* sy = reinterpret_cast<LoopSync*>(l.sync);
     DevStatus* gst = a.st + S;
+    uint32_t epoch = 0;   // grid barriers passed
     // Predicted positions of iteration k live in buffer k & 1 (selected, not indexed, so the
     // pair stays in registers).
     auto pp = [&](int k) { return (k & 1) ? l.ppos_alt : b.ppos; };
@@ -368,7 +362,7 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
             else integrate_one(P, b, i, 1);
         });
         if (preB[S] == 0) break;
-        if (!grid_barrier(sy, gst)) return;
+        if (!grid_barrier(sy, gst, epoch)) return;
 
         // phase B
         for_items(preB, [&](int s, int j) {
@@ -384,7 +378,7 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
             for (int off = 16; off > 0; off >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, off));
             if ((threadIdx.x & 31) == 0 && mb) atomicMax(l.maxerr + (size_t)s * l.mstride + kp, mb);
         });
-        if (!grid_barrier(sy, gst)) return;
+        if (!grid_barrier(sy, gst, epoch)) return;
     }
 }
 

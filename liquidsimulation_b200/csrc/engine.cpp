@@ -2,9 +2,11 @@
 #include "engine.h"
 #include "mlp.cuh"
 #include "mlp_tc.cuh"
+#include "small_step.h"
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <limits>
 #include <random>
@@ -181,10 +183,8 @@ Engine::Engine(const lsp_params& p, int device)
     CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     CK(cudaMallocHost((void**)&hstatus_, sizeof(DevStatus)));
     std::memset(hstatus_, 0, sizeof(DevStatus));
-    status_.alloc(1);
+    ctl_.alloc(1);
     bounds_.alloc(6);
-    loop_sync_.alloc(4);
-    maxerr_.alloc(kMaxIterationsCap);
     prm_ = p;
     derive();
     mlp_.init(stream_);
@@ -269,7 +269,7 @@ void Engine::ensure_capacity(int64_t n)
     ppos_final_ = ppos_.p;
     rho_.alloc(cap); pres_.alloc(cap); prho_.alloc(cap); err_.alloc(cap); vrho_.alloc(cap);
     key_.alloc(cap); slot_.alloc(cap); sorted_key_.alloc(cap); tmp_.alloc(cap); nbr_count_.alloc(cap);
-    stage_.alloc(cap * 12);
+    stage_.alloc(cap * 13);   // the whole state in caller order (read_state, write_state)
     CK(cudaMemsetAsync(force_.p, 0, cap * sizeof(float4), stream_));
     CK(cudaMemsetAsync(ppos_.p, 0, cap * sizeof(float4), stream_));
     CK(cudaMemsetAsync(ppos_alt_.p, 0, cap * sizeof(float4), stream_));
@@ -420,7 +420,7 @@ void Engine::ensure_grid()
         const int64_t alloc = scan_entries(cells + 1);
         hist_.alloc(alloc);
         cell_start_.alloc(alloc);
-        tile_sums_.alloc(scan_tiles(cells + 1) + 1);
+        tile_sums_.alloc(std::max<int64_t>(scan_tiles(cells + 1) + 1, kSmallStepTiles));
         CK(cudaMemsetAsync(hist_.p, 0, alloc * sizeof(uint32_t), stream_));
         CK(cudaMemsetAsync(cell_start_.p, 0, alloc * sizeof(uint32_t), stream_));
         cells_alloc_ = alloc;
@@ -513,7 +513,7 @@ StepBuffers Engine::buffers()
     b.force = force_.p; b.rho = rho_.p; b.pres = pres_.p;
     b.ppos = ppos_.p; b.phalf = phalf_.p; b.pforce = pforce_.p; b.prho = prho_.p; b.err = err_.p;
     b.nbr = nbr_.p; b.nbr_count = nbr_count_.p; b.vrho = vrho_.p;
-    b.tables = tables_.p; b.colliders = dcols_.p; b.status = status_.p;
+    b.tables = tables_.p; b.colliders = dcols_.p; b.status = status();
     b.hist = phist_[cur_].p;
     b.gradrho = features_on() ? gradrho_.p : nullptr;
     return b;
@@ -637,10 +637,8 @@ bool Engine::pcisph_loop(const DevParams& P, const StepBuffers& b, lsp_step_stat
         features_valid_ = true;
     }
     if (prm_.loop_mode == LSP_LOOP_PERSISTENT) {
-        CK(cudaMemsetAsync(loop_sync_.p, 0, 4 * sizeof(uint32_t), stream_));
-        CK(cudaMemsetAsync(maxerr_.p, 0, (size_t)(P.max_it + 4) * sizeof(uint32_t), stream_));
         if (feats) {
-            w.maxerr0 = maxerr_.p;
+            w.maxerr0 = ctl_.p->maxerr;
             timed(LSP_PROF_PCI_PREDICT, [&] { launch_pci_predict(P, b, 0, stream_); return 1; });
             timed(LSP_PROF_WARM_START, [&] {
                 launch_pci_density_first(P, b, w, stream_);
@@ -651,7 +649,7 @@ bool Engine::pcisph_loop(const DevParams& P, const StepBuffers& b, lsp_step_stat
         bool ok = false;
         int grid = 0;
         timed(LSP_PROF_PCI_LOOP, [&] {
-            ok = launch_pci_loop(P, b, ppos_alt_.p, loop_sync_.p, maxerr_.p, feats ? 1 : 0, warm ? 1 : 0, stream_,
+            ok = launch_pci_loop(P, b, ppos_alt_.p, ctl_.p->sync, ctl_.p->maxerr, feats ? 1 : 0, warm ? 1 : 0, stream_,
                                  &grid);
             return ok ? 1 : 0;
         });
@@ -662,7 +660,7 @@ bool Engine::pcisph_loop(const DevParams& P, const StepBuffers& b, lsp_step_stat
     // Per-phase loop; the convergence test reads the iteration's maximum back every time.
     auto read_err = [&]() {
         float e;
-        CK(cudaMemcpyAsync(&hstatus_->max_err_bits, &status_.p->max_err_bits, sizeof(uint32_t),
+        CK(cudaMemcpyAsync(&hstatus_->max_err_bits, &status()->max_err_bits, sizeof(uint32_t),
                            cudaMemcpyDeviceToHost, stream_));
         CK(cudaStreamSynchronize(stream_));
         std::memcpy(&e, &hstatus_->max_err_bits, 4);
@@ -672,7 +670,7 @@ bool Engine::pcisph_loop(const DevParams& P, const StepBuffers& b, lsp_step_stat
     bool conv = false, rejected = false;
     timed(LSP_PROF_PCI_PREDICT, [&] { launch_pci_predict(P, b, 0, stream_); return 1; });
     if (feats) {
-        w.maxerr0 = &status_.p->max_err_bits;
+        w.maxerr0 = &status()->max_err_bits;
         timed(LSP_PROF_WARM_START, [&] {
             launch_pci_density_first(P, b, w, stream_);
             if (warm) launch_warm_guess_tc(mlp_.umma(), P, b, feat_.p, stream_);
@@ -740,6 +738,44 @@ int grown_neighbor_capacity(int needed, int current)
     return (int)std::max<int64_t>(needed, std::min<int64_t>(c, 4096));
 }
 
+// Waits for the step; true when a neighbour list overflowed and the step is to be redone (the
+// grid build left the pre-step buffers untouched) with longer lists.
+bool Engine::retry_step(int attempt)
+{
+    CK(cudaStreamSynchronize(stream_));
+    if (!(hstatus_->error_flags & kErrNeighborOverflow) || attempt >= 3) return false;
+    cur_ = 1 - cur_;
+    ensure_neighbors(grown_neighbor_capacity((int)hstatus_->max_neighbors, nbr_cap_));
+    return true;
+}
+
+// Small scenes take the whole step in one launch (small_step_lanes has the rule); the per-class
+// profile, the per-phase loop and the warm start's features need the separate kernels.
+bool Engine::run_small(const GridBuildArgs& g, const StepBuffers& b)
+{
+    const bool pci = prm_.solver == LSP_SOLVER_PCISPH;
+    if (profile_ || features_on()) return false;
+    if (pci && (prm_.loop_mode != LSP_LOOP_PERSISTENT || g.P.max_it <= 0)) return false;
+    const int lanes = small_step_lanes(n_, cells_);
+    if (!lanes) return false;
+    SmallStepArgs a{};
+    a.g = g;
+    a.b = b;
+    a.ppos_alt = ppos_alt_.p;
+    a.sync = ctl_.p->sync;
+    a.maxerr = ctl_.p->maxerr;
+    a.host = hstatus_;
+    a.pcisph = pci ? 1 : 0;
+    std::memset(hstatus_, 0, sizeof(DevStatus));
+    if (!launch_small_step(a, lanes, stream_)) {
+        cudaGetLastError();   // the device refused the cooperative launch
+        return false;
+    }
+    launches_++;
+    ppos_final_ = ppos_.p;
+    return true;
+}
+
 void Engine::run_step(float dt, lsp_step_stats* st)
 {
     if (st) std::memset(st, 0, sizeof(*st));
@@ -765,7 +801,9 @@ void Engine::run_step(float dt, lsp_step_stats* st)
     for (int attempt = 0;; attempt++) {
         device_loop = false;
         DevParams P = device_params(dt);
-        CK(cudaMemsetAsync(status_.p, 0, sizeof(DevStatus), stream_));
+        // The barrier words, the status and the maxima that this step's iterations can write.
+        CK(cudaMemsetAsync(ctl_.p, 0, offsetof(Control, maxerr) + (size_t)(std::max(P.max_it, 0) + 4) * sizeof(uint32_t),
+                           stream_));
         GridBuildArgs g{};
         g.P = P;
         g.pos_in = pos_[cur_].p; g.vel_in = vel_[cur_].p; g.half_in = half_[cur_].p; g.old_in = old_[cur_].p;
@@ -774,16 +812,22 @@ void Engine::run_step(float dt, lsp_step_stats* st)
         g.key = key_.p; g.slot = slot_.p; g.hist = hist_.p; g.tile_sums = tile_sums_.p; g.cell_start = cell_start_.p;
         g.tmp = tmp_.p; g.slot_of_id = slot_of_id_.p; g.sorted_key = sorted_key_.p;
         g.hist_in = phist_[cur_].p; g.hist_out = phist_[1 - cur_].p;
-        g.nbr = nbr_.p; g.nbr_count = nbr_count_.p; g.status = status_.p;
+        g.nbr = nbr_.p; g.nbr_count = nbr_count_.p; g.status = status();
         // The neighbour build also sums the start-of-step density (k_neighbors_density).
         g.tables = tables_.p; g.rho = rho_.p; g.pres = pres_.p; g.vrho = vrho_.p;
+        cur_ = 1 - cur_;
+        StepBuffers b = buffers();
+        if (run_small(g, b)) {
+            device_loop = prm_.solver == LSP_SOLVER_PCISPH;
+            local.converged = 1;
+            if (retry_step(attempt)) continue;
+            break;
+        }
         timed(LSP_PROF_GRID_SORT, [&] { return launch_grid_keys(g, stream_); });
         timed(LSP_PROF_GRID_SCAN, [&] { return launch_grid_scan(g, stream_); });
         timed(LSP_PROF_GRID_SCATTER, [&] { return launch_grid_scatter(g, stream_); });
         timed(LSP_PROF_GRID_GATHER, [&] { return launch_grid_gather(g, stream_); });
         timed(LSP_PROF_NEIGHBORS, [&] { return launch_neighbors(g, stream_); });
-        cur_ = 1 - cur_;
-        StepBuffers b = buffers();
         timed(LSP_PROF_NONPRESSURE, [&] { launch_nonpressure(P, b, stream_); return 1; });
         if (prm_.solver == LSP_SOLVER_SPH) {
             timed(LSP_PROF_SPH_PRESSURE, [&] { launch_sph_pressure(P, b, stream_); return 1; });
@@ -797,14 +841,8 @@ void Engine::run_step(float dt, lsp_step_stats* st)
                 timed(LSP_PROF_INTEGRATE, [&] { launch_integrate_collide(P, b, true, stream_); return 1; });
         }
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(hstatus_, status_.p, sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
-        CK(cudaStreamSynchronize(stream_));
-        if ((hstatus_->error_flags & kErrNeighborOverflow) && attempt < 3) {
-            cur_ = 1 - cur_;   // the gather left the pre-step state untouched: redo the step
-            ensure_neighbors(grown_neighbor_capacity((int)hstatus_->max_neighbors, nbr_cap_));
-            continue;
-        }
-        break;
+        CK(cudaMemcpyAsync(hstatus_, status(), sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
+        if (!retry_step(attempt)) break;
     }
     stepped_ = true;
     if (device_loop) {

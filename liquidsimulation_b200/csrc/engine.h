@@ -139,6 +139,9 @@ private:
     void ensure_neighbors(int cap);
     void upload_colliders();
     void run_step(float dt, lsp_step_stats* st);
+    // Waits for a step; true when it is to be redone. The one-launch step of a small scene; false when this step runs as separate kernels.
+    bool retry_step(int attempt);
+    bool run_small(const GridBuildArgs& g, const StepBuffers& b);
     // Returns true when the persistent device loop ran (its stats arrive with the status).
     bool pcisph_loop(const DevParams& P, const StepBuffers& b, lsp_step_stats* st);
     void stage(size_t floats);
@@ -153,7 +156,6 @@ private:
     DevArray<float4> pos_[2], vel_[2], half_[2], old_[2];
     DevArray<float4> force_, ppos_, ppos_alt_, phalf_, pforce_;
     const float4* ppos_final_ = nullptr;   // buffer holding the last iteration's x*
-    DevArray<uint32_t> loop_sync_, maxerr_;
     DevArray<float> rho_, pres_, prho_, err_;
     DevArray<float4> vrho_;   // {v, rho} for the non-pressure pass (StepBuffers::vrho)
     DevArray<uint32_t> key_, slot_, sorted_key_;
@@ -174,7 +176,15 @@ private:
     std::vector<Collider> cols_;
     bool cols_dirty_ = true, tables_dirty_ = true;
 
-    DevArray<DevStatus> status_;
+    // What a step starts from zero, cleared by one memset: the loop's barrier words, the status
+    // and the loop's maximum error per iteration.
+    struct Control {
+        uint32_t sync[4];
+        DevStatus status;
+        uint32_t maxerr[kMaxIterationsCap + 4];
+    };
+    DevArray<Control> ctl_;
+    DevStatus* status() const { return &ctl_.p->status; }
     DevStatus* hstatus_ = nullptr;   // pinned
     DevArray<float> stage_;
 

@@ -22,13 +22,12 @@
 //                 and pressure summed over the accepted pairs
 #include "lsp_kernels.h"
 #include "particle_ops.cuh"
+#include "scan_ops.cuh"
 
 namespace lsp {
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-constexpr int kMaxCellOccupancy = 4096;
 
 __global__ void k_keys_hist(DevParams P, const float4* __restrict__ pos, uint32_t* __restrict__ key,
                             uint32_t* __restrict__ slot, uint32_t* __restrict__ hist, DevStatus* st)
@@ -44,47 +43,6 @@ __global__ void k_keys_hist(DevParams P, const float4* __restrict__ pos, uint32_
         slot[i] = sl;
     }
     record_key_flags(valid, escaped, bad, st);
-}
-
-// Block-wide exclusive scan of kScanItems consecutive items per thread, warp shuffles
-// inside each warp, then the warp totals.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* warp_sums, uint32_t* total)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-        uint32_t w = lane < nw ? warp_sums[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < nw) warp_sums[lane] = w;
-    }
-    __syncthreads();
-    uint32_t warp_prefix = warp ? warp_sums[warp - 1] : 0u;
-    if (total) *total = warp_sums[(blockDim.x >> 5) - 1];
-    __syncthreads();
-    return warp_prefix + x - v;
-}
-
-// The histogram and the cell table are padded with zeros to a multiple of 8 entries
-// (scan_entries): each thread moves its 8 consecutive entries as two 16-byte vectors. n8 is
-// the padded count.
-__device__ __forceinline__ void load8(const uint32_t* p, uint32_t (&v)[kScanItems])
-{
-    const uint4 a = *reinterpret_cast<const uint4*>(p);
-    const uint4 b = *reinterpret_cast<const uint4*>(p + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const uint32_t* __restrict__ in, int64_t n8,
@@ -145,18 +103,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(uint32_t* __restric
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) s += v[j];
     uint32_t ex = block_exclusive_scan(s, ws, nullptr) + prefix;
-    if (base < n8) {
-        uint32_t o[kScanItems];
-#pragma unroll
-        for (int j = 0; j < kScanItems; j++) {
-            o[j] = ex;
-            ex += v[j];
-        }
-        *reinterpret_cast<uint4*>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
-        *reinterpret_cast<uint4*>(out + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
-        *reinterpret_cast<uint4*>(hist + base) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(hist + base + 4) = make_uint4(0u, 0u, 0u, 0u);
-    }
+    if (base < n8) store8_scan(out + base, hist + base, v, ex);
 }
 
 __global__ void k_scatter(DevParams P, const float4* __restrict__ pos, const uint32_t* __restrict__ key,
@@ -169,43 +116,11 @@ __global__ void k_scatter(DevParams P, const float4* __restrict__ pos, const uin
     tmp[cell_start[k] + slot[i]] = make_int2(i, id_of(pos[i]));
 }
 
-// Final slot = cell start + number of particles of the same cell with a smaller caller id.
-// Then moves the particle's persistent state (x|id, v|first, v_half|p1, v_half_old|p2).
-__global__ void k_rank_gather(DevParams P, const int2* __restrict__ tmp, const uint32_t* __restrict__ key,
-                              const uint32_t* __restrict__ cell_start,
-                              const float4* __restrict__ ipos, const float4* __restrict__ ivel,
-                              const float4* __restrict__ ihalf, const float4* __restrict__ iold,
-                              float4* __restrict__ opos, float4* __restrict__ ovel,
-                              float4* __restrict__ ohalf, float4* __restrict__ oold,
-                              int32_t* __restrict__ slot_of_id, uint32_t* __restrict__ sorted_key, DevStatus* st,
-                              const float4* __restrict__ ihist, float4* __restrict__ ohist)
+// rank_gather_one (particle_ops.cuh) for every sorted slot.
+__global__ void k_rank_gather(GridBuildArgs g)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P.n) return;
-    int2 e = tmp[p];
-    uint32_t k = key[e.x];
-    uint32_t beg = cell_start[k], end = cell_start[k + 1];
-    uint32_t rank = 0;
-    if (end - beg <= (uint32_t)kMaxCellOccupancy) {
-        for (uint32_t q = beg; q < end; q++) rank += tmp[q].y < e.y ? 1u : 0u;
-    } else {
-        rank = (uint32_t)p - beg;   // order inside an overfull cell is not the reference's
-        atomicOr(&st->error_flags, kErrScan);
-    }
-    uint32_t dest = beg + rank;
-    const float4 x = ipos[e.x], v = ivel[e.x];
-    opos[dest] = x;
-    ovel[dest] = v;
-    // The non-pressure pass divides pair terms by densities with div_by while every position
-    // and velocity of the step is in exact_div_safe's range.
-    if (!(exact_div_safe(x.x) && exact_div_safe(x.y) && exact_div_safe(x.z) && exact_div_safe(v.x) &&
-          exact_div_safe(v.y) && exact_div_safe(v.z)))
-        atomicOr(&st->np_unsafe, 1u);
-    ohalf[dest] = ihalf[e.x];
-    oold[dest] = iold[e.x];
-    if (ohist) ohist[dest] = ihist[e.x];
-    slot_of_id[e.y] = (int32_t)dest;
-    sorted_key[dest] = k;
+    if (p < g.P.n) rank_gather_one(g, p);
 }
 
 // Start-of-step neighbour lists (neighbors_one) plus the start-of-step density
@@ -220,22 +135,14 @@ __global__ void k_neighbors_density(DevParams P, const float4* __restrict__ pos,
                                     float* __restrict__ rho, float* __restrict__ pres,
                                     const float4* __restrict__ vel, float4* __restrict__ vrho)
 {
+    extern __shared__ uint2 masks[];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < P.n;
-    extern __shared__ uint2 masks[];
     int c = 0;
     if (valid) {
         float sum;
-        c = neighbors_one(P, pos, cell_start, nbr, i, tables, masks + threadIdx.x, &sum);
-        count[i] = min(c, P.nbr_cap);
-        const float r = P.mass * sum;
-        float pr = P.stiffness * (r - P.rho0);
-        if (pr < 0.f) pr *= P.neg;
-        rho[i] = r;
-        pres[i] = pr;
-        const float4 v = vel[i];
-        vrho[i] = make_float4(v.x, v.y, v.z, r);
-        if (!exact_div_density(r)) atomicOr(&st->np_unsafe, 1u);
+        c = neighbors_one(P, pos, cell_start, nbr, i, tables, masks + threadIdx.x, blockDim.x, &sum);
+        store_density(P, i, c, sum, vel, count, rho, pres, vrho, st);
     }
     record_neighbor_count(P, c, valid, st);
 }
@@ -272,10 +179,7 @@ int launch_grid_scatter(const GridBuildArgs& a, cudaStream_t s)
 int launch_grid_gather(const GridBuildArgs& a, cudaStream_t s)
 {
     if (a.P.n <= 0) return 0;
-    k_rank_gather<<<blocks_for(a.P.n, 256), 256, 0, s>>>(a.P, a.tmp, a.key, a.cell_start, a.pos_in, a.vel_in,
-                                                         a.half_in, a.old_in, a.pos_out, a.vel_out, a.half_out,
-                                                         a.old_out, a.slot_of_id, a.sorted_key, a.status,
-                                                         a.hist_in, a.hist_out);
+    k_rank_gather<<<blocks_for(a.P.n, 256), 256, 0, s>>>(a);
     return 1;
 }
 
@@ -286,10 +190,7 @@ int launch_grid_order(const GridBuildArgs& a, cudaStream_t s)
     int launches = launch_grid_scan(a, s);
     if (P.n > 0) {
         k_scatter<<<blocks_for(P.n, T), T, 0, s>>>(P, a.pos_in, a.key, a.slot, a.cell_start, a.tmp);
-        k_rank_gather<<<blocks_for(P.n, T), T, 0, s>>>(P, a.tmp, a.key, a.cell_start, a.pos_in, a.vel_in,
-                                                       a.half_in, a.old_in, a.pos_out, a.vel_out, a.half_out,
-                                                       a.old_out, a.slot_of_id, a.sorted_key, a.status, a.hist_in,
-                                                       a.hist_out);
+        k_rank_gather<<<blocks_for(P.n, T), T, 0, s>>>(a);
         launches += 2;
     }
     return launches;
@@ -311,8 +212,9 @@ int launch_neighbors(const GridBuildArgs& a, cudaStream_t s)
 {
     const int T = 256;
     if (a.P.n <= 0) return 0;
-    k_neighbors_density<<<blocks_for(a.P.n, T), T, scan_smem(T), s>>>(a.P, a.pos_out, a.cell_start, a.nbr, a.nbr_count, a.status,
-                                                           a.tables, a.rho, a.pres, a.vel_out, a.vrho);
+    k_neighbors_density<<<blocks_for(a.P.n, T), T, scan_smem(T), s>>>(a.P, a.pos_out, a.cell_start, a.nbr,
+                                                                      a.nbr_count, a.status, a.tables, a.rho, a.pres,
+                                                                      a.vel_out, a.vrho);
     return 1;
 }
 

@@ -18,36 +18,51 @@ struct LoopSync {
 };
 
 static __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *(const volatile uint32_t*)p; }
+static __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p)
+{
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+static __device__ __forceinline__ void add_release(uint32_t* p)
+{
+    asm volatile("red.add.release.gpu.global.u32 [%0], 1;" : : "l"(p) : "memory");
+}
+
+// Thread 0's bounded wait for the arrival counter to reach target; false when it, or another
+// block, gave up. The first polls come without a pause: a small scene's phases are about as long
+// as one.
+static __device__ __forceinline__ bool barrier_wait(LoopSync* sy, DevStatus* st, uint32_t target,
+                                                    unsigned long long spin_limit)
+{
+    unsigned long long spins = 0;
+    while ((int)(ld_acquire(&sy->count) - target) < 0) {
+        if (++spins < 64) continue;
+        if (ld_volatile(&sy->abort)) return false;
+        if (spins > spin_limit) {
+            atomicExch(&sy->abort, 1u);
+            atomicOr(&st->error_flags, kErrTimeout);
+            return false;
+        }
+        __nanosleep(64);
+    }
+    return ld_volatile(&sy->abort) == 0u;
+}
 
 // Returns false when the loop must stop (a barrier gave up somewhere). The arrival counter
-// only grows during a launch (the host clears it before each one): the block that arrives
-// as the a-th waits until the counter reaches the next multiple of the number of parties
-// (the grid size), so one atomic per block and barrier is all the traffic (measured 1.2 %
-// faster loop than a counter reset by the last arrival plus a generation word).
-static __device__ bool grid_barrier(LoopSync* sy, DevStatus* st, uint32_t parties = 0,
-                                    unsigned long long spin_limit = kBarrierSpinLimit)
+// only grows during a launch (the host clears it before each one): the e-th barrier of a launch
+// is over when the counter reaches e times the grid size, so one reduction per block and barrier
+// is all the traffic; epoch counts the barriers this block has passed. The arrival releases and
+// the last poll acquires at device scope; block barriers on both sides carry that to the other
+// threads.
+static __device__ bool grid_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch)
 {
-    if (parties == 0) parties = gridDim.x;
     __shared__ int ok;
+    const uint32_t target = ++epoch * gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
-        ok = 1;
-        __threadfence();
-        const uint32_t arrived = atomicAdd(&sy->count, 1u);
-        const uint32_t target = (arrived / parties + 1u) * parties;
-        unsigned long long spins = 0;
-        while ((int)(ld_volatile(&sy->count) - target) < 0) {
-            if (ld_volatile(&sy->abort)) { ok = 0; break; }
-            if (++spins > spin_limit) {
-                atomicExch(&sy->abort, 1u);
-                atomicOr(&st->error_flags, kErrTimeout);
-                ok = 0;
-                break;
-            }
-            __nanosleep(64);
-        }
-        if (ld_volatile(&sy->abort)) ok = 0;
-        __threadfence();
+        add_release(&sy->count);
+        ok = barrier_wait(sy, st, target, kBarrierSpinLimit) ? 1 : 0;
     }
     __syncthreads();
     return ok != 0;

@@ -328,12 +328,14 @@ __device__ __forceinline__ float lo(F2 a)
 {
     float x, y;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    (void)y;
     return x;
 }
 __device__ __forceinline__ float hi(F2 a)
 {
     float x, y;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    (void)x;
     return y;
 }
 __device__ __forceinline__ F2 operator+(F2 a, F2 b)

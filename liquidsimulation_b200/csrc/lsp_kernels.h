@@ -78,9 +78,9 @@ struct StepBuffers {
     DevStatus* status;
 };
 
-// The neighbour scan reads up to 3 positions past the last one (neighbors_one): position arrays
-// hold that many more.
-constexpr int kPosPad = 4;
+// The neighbour scans read up to 7 positions past the last one (scan_row): position arrays hold
+// that many more.
+constexpr int kPosPad = 8;
 // Masks per thread that the neighbour scan keeps in dynamic shared memory (9 rows, and some to
 // spare), and their bytes for a block.
 constexpr int kScanChunks = 12;
@@ -89,7 +89,7 @@ inline size_t scan_smem(int threads) { return (size_t)threads * kScanChunks * si
 // Entries of the histogram and cell-table buffers for `n` live entries: the scan moves them
 // 8 at a time, so both are padded to a multiple of 8 (the padding stays zero); and the scan's
 // tiles of 2048 entries.
-inline int64_t scan_entries(int64_t n) { return (n + 7) / 8 * 8; }
+__host__ __device__ inline int64_t scan_entries(int64_t n) { return (n + 7) / 8 * 8; }
 inline int64_t scan_tiles(int64_t n) { return (scan_entries(n) + 2047) / 2048; }
 
 // All return the number of kernels launched.

@@ -29,6 +29,43 @@ __device__ __forceinline__ uint32_t cell_key(const DevParams& P, const float4& p
     return P.cell_base + (uint32_t)(((uint32_t)c[0] * (uint32_t)P.ny + (uint32_t)c[1]) * (uint32_t)P.nz + (uint32_t)c[2]);
 }
 
+// Cells the neighbour search of a particle at x visits, relative to the grid box
+// (SPHSpatialGrid.cpp:44-50).
+__device__ __forceinline__ void search_box(const DevParams& P, V3 x, int (&lo_)[3], int (&hi_)[3])
+{
+    const float h = P.h;
+    const int a0[3] = {(int)((x.x - h) / h), (int)((x.y - h) / h), (int)((x.z - h) / h)};
+    const int a1[3] = {(int)((x.x + h) / h), (int)((x.y + h) / h), (int)((x.z + h) / h)};
+    const int o[3] = {P.ox, P.oy, P.oz};
+    const int d[3] = {P.nx, P.ny, P.nz};
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        // Both ends clamped into the box: a particle outside it searches the edge cell
+        // that holds every clamped particle.
+        lo_[a] = min(max(a0[a], o[a]), o[a] + d[a] - 1) - o[a];
+        hi_[a] = min(max(a1[a], o[a]), o[a] + d[a] - 1) - o[a];
+    }
+}
+
+// Tests candidates [beg, beg + len), len <= 32, of a particle at xi: bit b of the result is
+// candidate last - b (`above`: the float after h^2). Reads U at a time, up to U - 1 past the end.
+template <int U>
+__device__ __forceinline__ uint32_t scan_row(const float4* pos, V3 xi, float above, int beg, int len, int& last)
+{
+    const float4* p = pos + beg;
+    uint32_t bits = 0;
+    for (int k = 0; k < len; k += U, p += U) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const float s = sqmag(xi - v3(p[u]));
+            bits = __funnelshift_l(__float_as_uint(s - above), bits, 1);
+        }
+    }
+    const int over = -len & (U - 1);   // candidates tested past the end
+    last = beg + len + over - 1;
+    return bits & (0xffffffffu << over);
+}
+
 // Start-of-step neighbour list and density sum of particle i: every j with
 // |x_i - x_j|^2 <= h^2, including i, in the reference's order (SPHSpatialGrid::findNeighborParticles,
 // SPHSpatialGrid.cpp:39-76): cell ranges from (x -+ h) / h per axis, x then y rows, each row a
@@ -40,7 +77,7 @@ __device__ __forceinline__ uint32_t cell_key(const DevParams& P, const float4& p
 // Two phases. The scan tests the rows' candidates, 32 at a time, into bit masks without a
 // branch: s - next_up(h^2) is negative exactly when s <= h^2 (a NaN's sign is clear), and a
 // funnel shift appends that sign to the mask, first candidate highest. The masks wait in a
-// column of shared memory per thread. Then the accepted entries are taken from the masks four
+// column of shared memory per thread (col, entries `pitch` apart). Then the accepted entries are taken from the masks four
 // at a time, by all lanes in step: their positions are fetched again, W is evaluated for two
 // pairs at a time and the group of four goes out as one 16-byte store that coalesces over the
 // lanes. A scan that handles each accepted candidate at once runs that branch for 10 of 32 lanes
@@ -52,22 +89,12 @@ __device__ __forceinline__ uint32_t cell_key(const DevParams& P, const float4& p
 // slower (0.238, 0.289 ms), the larger working set missing more in L1.
 __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* __restrict__ pos,
                                              const uint32_t* __restrict__ cell_start, int32_t* __restrict__ nbr,
-                                             int i, const float* __restrict__ tables, uint2* col, float* wsum)
+                                             int i, const float* __restrict__ tables, uint2* col, int pitch,
+                                             float* wsum)
 {
-    const int pitch = blockDim.x;
     const V3 xi = v3(pos[i]);
-    const float h = P.h;
-    int lo_[3] = {(int)((xi.x - h) / h), (int)((xi.y - h) / h), (int)((xi.z - h) / h)};
-    int hi_[3] = {(int)((xi.x + h) / h), (int)((xi.y + h) / h), (int)((xi.z + h) / h)};
-    const int o[3] = {P.ox, P.oy, P.oz};
-    const int d[3] = {P.nx, P.ny, P.nz};
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        // Both ends clamped into the box: a particle outside it searches the edge cell
-        // that holds every clamped particle.
-        lo_[a] = min(max(lo_[a], o[a]), o[a] + d[a] - 1) - o[a];
-        hi_[a] = min(max(hi_[a], o[a]), o[a] + d[a] - 1) - o[a];
-    }
+    int lo_[3], hi_[3];
+    search_box(P, xi, lo_, hi_);
     const float above = __uint_as_float(__float_as_uint(P.h2) + 1u);   // the next float above h^2
     int4* out = reinterpret_cast<int4*>(nbr) + i;
     const int64_t stride = P.nbr_stride;
@@ -104,21 +131,11 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
                 const uint32_t row = P.cell_base + ((uint32_t)cx * (uint32_t)P.ny + (uint32_t)cy) * (uint32_t)P.nz;
                 const int end = (int)cell_start[row + hi_[2] + 1];
                 for (int beg = (int)cell_start[row + lo_[2]]; beg < end; beg += 32) {
-                    const int len = min(end - beg, 32);
-                    const float4* p = pos + beg;
-                    uint32_t bits = 0;
-                    for (int k = 0; k < len; k += 4, p += 4) {
-#pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            const float s = sqmag(xi - v3(__ldg(p + u)));
-                            bits = __funnelshift_l(__float_as_uint(s - above), bits, 1);
-                        }
-                    }
-                    const int over = -len & 3;   // candidates tested past the row's end
-                    bits &= 0xffffffffu << over;
+                    int last_q;
+                    const uint32_t bits = scan_row<4>(pos, xi, above, beg, min(end - beg, 32), last_q);
                     if (bits) {
                         if (chunks == kScanChunks) drain();
-                        col[chunks * pitch] = make_uint2((uint32_t)(beg + len + over - 1), bits);
+                        col[chunks * pitch] = make_uint2((uint32_t)last_q, bits);
                         chunks++;
                         pending += __popc(bits);
                     }
@@ -141,7 +158,7 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
         if (left > 1) q.y = take();
         if (left > 2) q.z = take();
         if (left > 3) q.w = take();
-        const float4 a = __ldg(pos + q.x), b = __ldg(pos + q.y), c = __ldg(pos + q.z), e = __ldg(pos + q.w);
+        const float4 a = pos[q.x], b = pos[q.y], c = pos[q.z], e = pos[q.w];
         if (k < P.nbr_cap) *out = q;
         out += stride;
         const F2 w0 = weight_w(neg_sqmag(f2(a.x - xi.x, b.x - xi.x), f2(a.y - xi.y, b.y - xi.y), f2(a.z - xi.z, b.z - xi.z)),
@@ -203,6 +220,61 @@ __device__ __forceinline__ void record_neighbor_count(const DevParams& P, int c,
     }
 }
 
+// Density, pressure and {v, rho} record of particle i from its neighbour count and sum of W
+// (SPHSolver::calcParticleDensityPressure, CPU branch, SPHSolver.cpp:442-463).
+__device__ __forceinline__ void store_density(const DevParams& P, int i, int c, float sum, const float4* vel,
+                                              int32_t* count, float* rho, float* pres, float4* vrho, DevStatus* st)
+{
+    count[i] = min(c, P.nbr_cap);
+    const float r = P.mass * sum;
+    float pr = P.stiffness * (r - P.rho0);
+    if (pr < 0.f) pr *= P.neg;
+    rho[i] = r;
+    pres[i] = pr;
+    const float4 v = vel[i];
+    vrho[i] = make_float4(v.x, v.y, v.z, r);
+    if (!exact_div_density(r)) atomicOr(&st->np_unsafe, 1u);
+}
+
+// Stores a particle's persistent state (x|id, v|first, v_half|p1, v_half_old|p2) at its sorted slot.
+__device__ __forceinline__ void store_sorted(const GridBuildArgs& g, uint32_t dest, int id, uint32_t key, float4 x, float4 v,
+                                             float4 half, float4 old)
+{
+    g.pos_out[dest] = x;
+    g.vel_out[dest] = v;
+    // The non-pressure pass divides pair terms by densities with div_by while every position
+    // and velocity of the step is in exact_div_safe's range.
+    if (!(exact_div_safe(x.x) && exact_div_safe(x.y) && exact_div_safe(x.z) && exact_div_safe(v.x) &&
+          exact_div_safe(v.y) && exact_div_safe(v.z)))
+        atomicOr(&g.status->np_unsafe, 1u);
+    g.half_out[dest] = half;
+    g.old_out[dest] = old;
+    g.slot_of_id[id] = (int32_t)dest;
+    g.sorted_key[dest] = key;
+}
+
+// Final slot of the particle scattered to p = cell start + number of particles of the same cell
+// with a smaller caller id. Then moves the particle's persistent state.
+constexpr int kMaxCellOccupancy = 4096;
+__device__ __forceinline__ void rank_gather_one(const GridBuildArgs& g, int p)
+{
+    auto ld = [](const auto* q) { return __ldg(q); };
+    const int2 e = ld(g.tmp + p);
+    const uint32_t k = ld(g.key + e.x);
+    const uint32_t beg = ld(g.cell_start + k), end = ld(g.cell_start + k + 1);
+    uint32_t rank = 0;
+    if (end - beg <= (uint32_t)kMaxCellOccupancy) {
+        for (uint32_t q = beg; q < end; q++) rank += ld(g.tmp + q).y < e.y ? 1u : 0u;
+    } else {
+        rank = (uint32_t)p - beg;   // order inside an overfull cell is not the reference's
+        atomicOr(&g.status->error_flags, kErrScan);
+    }
+    const uint32_t dest = beg + rank;
+    store_sorted(g, dest, e.y, k, __ldg(g.pos_in + e.x), __ldg(g.vel_in + e.x), __ldg(g.half_in + e.x),
+                 __ldg(g.old_in + e.x));
+    if (g.hist_out) g.hist_out[dest] = __ldg(g.hist_in + e.x);
+}
+
 // SPHSolver::accumulateNonPressureForces, CPU branch (SPHSolver.cpp:201-248). The
 // reference walks the list up to three times (normal, colour Laplacian when the normal
 // exceeds the threshold, viscosity); each sum is independent, so one walk computes all
@@ -216,71 +288,109 @@ __device__ __forceinline__ void record_neighbor_count(const DevParams& P, int c,
 // entries are (DevParams::exact_tables), since every numerator is then 0 or at least 2^-80 in
 // magnitude (nonpressure_one chooses). The particle itself then adds a zero to the viscosity
 // sum, which starts at +0 and is left unchanged, so it needs no test.
+__device__ __forceinline__ V3 nonpressure_force(const DevParams& P, float rhoi, V3 normal, float lap, V3 visc)
+{
+    V3 F = v3(0.f, 0.f, 0.f);
+    F += v3(P.gx, P.gy, P.gz) * rhoi;
+    normal *= P.mass;
+    float len = mag(normal);
+    if (len > P.sigma_thr) F += (normal / len) * (-P.sigma * lap * P.mass);
+    visc *= P.viscosity * P.mass;
+    F += visc;
+    return F;
+}
+struct NonpressureRec {
+    float4 x, vr;   // position; velocity and density ({v, rho}, StepBuffers::vrho)
+};
+// The terms of one pair with IEEE division, and of two pairs with div_by (the halves of the F2).
+// grad: the warm-start feature's (rho_j - rho_i) / rho_j grad W_ij.
+struct NonpressureTerms {
+    V3 normal, visc, grad;
+    float lap;
+};
+template <bool kGrad>
+__device__ __forceinline__ NonpressureTerms nonpressure_term(const DevParams& P, const float* __restrict__ tables, V3 xi,
+                                                             V3 vi, float rhoi, const NonpressureRec& r)
+{
+    NonpressureTerms t;
+    const V3 dir = xi - v3(r.x);
+    // |x_i - x_j|^2 equals |x_j - x_i|^2 bit for bit
+    const NonpressureWeights at(sqmag(dir), P, tables);
+    t.normal = dir * at.dw / r.vr.w;
+    t.lap = at.d2w / r.vr.w;
+    t.visc = ((v3(r.vr) - vi) / r.vr.w) * at.vd2w;
+    if (kGrad) t.grad = dir * (at.dw * ((r.vr.w - rhoi) / r.vr.w));
+    return t;
+}
+struct NonpressureTerms2 {
+    F2 nx, ny, nz, lap, vx, vy, vz, gx, gy, gz;
+};
+template <bool kGrad>
+__device__ __forceinline__ NonpressureTerms2 nonpressure_pair(const DevParams& P, const float* __restrict__ tables, V3 xi,
+                                                              V3 vi, float rhoi, const NonpressureRec& r0,
+                                                              const NonpressureRec& r1)
+{
+    NonpressureTerms2 t;
+    const F2 dx = f2(xi.x - r0.x.x, xi.x - r1.x.x), dy = f2(xi.y - r0.x.y, xi.y - r1.x.y),
+             dz = f2(xi.z - r0.x.z, xi.z - r1.x.z);
+    const NonpressureWeights2 at(neg_sqmag(dx, dy, dz), P, tables);
+    const F2 nrho = f2(-r0.vr.w, -r1.vr.w);
+    const F2 y = recip_rn(nrho);
+    auto q = [&](F2 a) { return div_by(a, nrho, y); };
+    t.nx = q(dx * at.dw);
+    t.ny = q(dy * at.dw);
+    t.nz = q(dz * at.dw);
+    t.lap = q(at.d2w);
+    t.vx = q(f2(r0.vr.x - vi.x, r1.vr.x - vi.x)) * at.vd2w;
+    t.vy = q(f2(r0.vr.y - vi.y, r1.vr.y - vi.y)) * at.vd2w;
+    t.vz = q(f2(r0.vr.z - vi.z, r1.vr.z - vi.z)) * at.vd2w;
+    if (kGrad) {
+        const F2 g = at.dw * q(f2(r0.vr.w - rhoi, r1.vr.w - rhoi));
+        t.gx = dx * g;
+        t.gy = dy * g;
+        t.gz = dz * g;
+    }
+    return t;
+}
 template <bool kGrad, bool kExactDiv>
 __device__ __forceinline__ void nonpressure_walk(const DevParams& P, const StepBuffers& b, int i)
 {
     const V3 xi = v3(b.pos[i]);
     const V3 vi = v3(b.vel[i]);
     const float rhoi = b.rho[i];
-    V3 F = v3(0.f, 0.f, 0.f);
-    F += v3(P.gx, P.gy, P.gz) * rhoi;
     V3 normal = v3(0.f, 0.f, 0.f);
     V3 visc = v3(0.f, 0.f, 0.f);
+    V3 grad = v3(0.f, 0.f, 0.f);
     float lap = 0.f;
-    V3 grad = v3(0.f, 0.f, 0.f);   // sum (rho_j - rho_i) / rho_j grad W_ij: a warm-start feature only
-    struct Rec {
-        float4 x, vr;   // position; velocity and density ({v, rho}, StepBuffers::vrho)
+    auto one = [&](int j, const NonpressureRec& r) {
+        const NonpressureTerms t = nonpressure_term<kGrad>(P, b.tables, xi, vi, rhoi, r);
+        normal += t.normal;
+        lap += t.lap;
+        if (j != i) visc += t.visc;
+        if (kGrad) grad += t.grad;
     };
-    auto load = [&](int j) { return Rec{b.pos[j], b.vrho[j]}; };
-    auto one = [&](int j, const Rec& r) {
-        V3 dir = xi - v3(r.x);
-        // |x_i - x_j|^2 equals |x_j - x_i|^2 bit for bit
-        const NonpressureWeights at(sqmag(dir), P, b.tables);
-        normal += dir * at.dw / r.vr.w;
-        lap += at.d2w / r.vr.w;
-        if (j != i) visc += ((v3(r.vr) - vi) / r.vr.w) * at.vd2w;
-        if (kGrad) grad += dir * (at.dw * ((r.vr.w - rhoi) / r.vr.w));
-    };
-    auto pair = [&](int j0, const Rec& r0, int j1, const Rec& r1, bool two) {
+    auto pair = [&](int j0, const NonpressureRec& r0, int j1, const NonpressureRec& r1, bool two) {
         if (!kExactDiv) {
             one(j0, r0);
             if (two) one(j1, r1);
             return;
         }
-        const F2 dx = f2(xi.x - r0.x.x, xi.x - r1.x.x), dy = f2(xi.y - r0.x.y, xi.y - r1.x.y),
-                 dz = f2(xi.z - r0.x.z, xi.z - r1.x.z);
-        const NonpressureWeights2 at(neg_sqmag(dx, dy, dz), P, b.tables);
-        const F2 nrho = f2(-r0.vr.w, -r1.vr.w);
-        const F2 y = recip_rn(nrho);
-        auto q = [&](F2 a) { return div_by(a, nrho, y); };
-        const F2 nx = q(dx * at.dw), ny = q(dy * at.dw), nz = q(dz * at.dw), l = q(at.d2w);
-        const F2 wx = q(f2(r0.vr.x - vi.x, r1.vr.x - vi.x)) * at.vd2w,
-                 wy = q(f2(r0.vr.y - vi.y, r1.vr.y - vi.y)) * at.vd2w,
-                 wz = q(f2(r0.vr.z - vi.z, r1.vr.z - vi.z)) * at.vd2w;
-        normal += v3(lo(nx), lo(ny), lo(nz));
-        lap += lo(l);
-        visc += v3(lo(wx), lo(wy), lo(wz));
-        F2 g;
-        if (kGrad) {
-            g = at.dw * q(f2(r0.vr.w - rhoi, r1.vr.w - rhoi));
-            const F2 gx = dx * g, gy = dy * g, gz = dz * g;
-            grad += v3(lo(gx), lo(gy), lo(gz));
-            if (two) grad += v3(hi(gx), hi(gy), hi(gz));
-        }
+        const NonpressureTerms2 t = nonpressure_pair<kGrad>(P, b.tables, xi, vi, rhoi, r0, r1);
+        normal += v3(lo(t.nx), lo(t.ny), lo(t.nz));
+        lap += lo(t.lap);
+        visc += v3(lo(t.vx), lo(t.vy), lo(t.vz));
+        if (kGrad) grad += v3(lo(t.gx), lo(t.gy), lo(t.gz));
         if (two) {
-            normal += v3(hi(nx), hi(ny), hi(nz));
-            lap += hi(l);
-            visc += v3(hi(wx), hi(wy), hi(wz));
+            normal += v3(hi(t.nx), hi(t.ny), hi(t.nz));
+            lap += hi(t.lap);
+            visc += v3(hi(t.vx), hi(t.vy), hi(t.vz));
+            if (kGrad) grad += v3(hi(t.gx), hi(t.gy), hi(t.gz));
         }
     };
-    for_each_neighbor<2>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i), load, pair);
+    for_each_neighbor<2>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i),
+                         [&](int j) { return NonpressureRec{b.pos[j], b.vrho[j]}; }, pair);
     if (kGrad) b.gradrho[i] = P.mass * mag(grad);
-    normal *= P.mass;
-    float len = mag(normal);
-    if (len > P.sigma_thr) F += (normal / len) * (-P.sigma * lap * P.mass);
-    visc *= P.viscosity * P.mass;
-    F += visc;
-    b.force[i] = f4(F, 0.f);
+    b.force[i] = f4(nonpressure_force(P, rhoi, normal, lap, visc), 0.f);
 }
 template <bool kGrad>
 __device__ __forceinline__ void nonpressure_one(const DevParams& P, const StepBuffers& b, int i)
@@ -292,26 +402,30 @@ __device__ __forceinline__ void nonpressure_one(const DevParams& P, const StepBu
 }
 
 // SPHSolver::accumulatePressureForces, CPU branch (SPHSolver.cpp:268-290).
+struct SphRec {
+    float4 x;
+    float rho, p;
+};
+__device__ __forceinline__ V3 sph_pressure_term(const DevParams& P, const float* __restrict__ tables, V3 xi, float tf,
+                                                const SphRec& r)
+{
+    const V3 dq = xi - v3(r.x);
+    const float d = mag(dq);
+    const V3 dir = dq / d;
+    return dir * weight_sdw(d, P, tables) * (tf + r.p / (r.rho * r.rho));
+}
 __device__ __forceinline__ void sph_pressure_one(const DevParams& P, const StepBuffers& b, int i)
 {
     const V3 xi = v3(b.pos[i]);
     const float rhoi = b.rho[i];
     const float tf = b.pres[i] / (rhoi * rhoi);
     V3 pf = v3(0.f, 0.f, 0.f);
-    struct Rec {
-        float4 x;
-        float rho, p;
-    };
-    auto one = [&](int j, const Rec& r) {
-        if (j == i) return;
-        const V3 xj = v3(r.x);
-        float d = mag(xi - xj);
-        V3 dir = (xi - xj) / d;
-        pf += dir * weight_sdw(d, P, b.tables) * (tf + r.p / (r.rho * r.rho));
+    auto one = [&](int j, const SphRec& r) {
+        if (j != i) pf += sph_pressure_term(P, b.tables, xi, tf, r);
     };
     for_each_neighbor<4>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i),
-                         [&](int j) { return Rec{b.pos[j], b.rho[j], b.pres[j]}; },
-                         [&](int j0, const Rec& r0, int j1, const Rec& r1, bool two) {
+                         [&](int j) { return SphRec{b.pos[j], b.rho[j], b.pres[j]}; },
+                         [&](int j0, const SphRec& r0, int j1, const SphRec& r1, bool two) {
                              one(j0, r0);
                              if (two) one(j1, r1);
                          });
@@ -322,27 +436,32 @@ __device__ __forceinline__ void sph_pressure_one(const DevParams& P, const StepB
 }
 
 // SPHParticle::integrate (SPHParticle.cpp:30-44) then SPHSolver::handleCollisions
-// (SPHSolver.cpp:337-355) for one particle. With add_pforce the PCISPH pressure force is
-// added first (PCISPHSolver.cpp:166-169).
+// (SPHSolver.cpp:337-355) for one particle with total force F: x and half are moved on, v and old
+// set; first is the first-step flag.
+__device__ __forceinline__ void integrate_motion(const DevParams& P, const Collider* cols, V3 F, float rho, V3& x, V3& v,
+                                                 float& first, V3& half, V3& old)
+{
+    V3 acc = F / rho;
+    if (first != 0.f) {
+        half = v - acc * P.dt / 2.f;
+        first = 0.f;
+    }
+    old = half;
+    half = v3(half.x + acc.x * P.dt, half.y + acc.y * P.dt, half.z + acc.z * P.dt);
+    x = v3(x.x + half.x * P.dt, x.y + half.y * P.dt, x.z + half.z * P.dt);
+    collide_all(cols, P.ncoll, x, half, P);
+    v = (old + half) / 2.f;
+}
+// integrate_motion on the stored state. With add_pforce the PCISPH pressure force is added first
+// (PCISPHSolver.cpp:166-169).
 __device__ __forceinline__ void integrate_one(const DevParams& P, const StepBuffers& b, int i, int add_pforce)
 {
     float4 p4 = b.pos[i], v4 = b.vel[i], h4 = b.half[i], o4 = b.old[i];
     V3 F = v3(b.force[i]);
     if (add_pforce) F += v3(b.pforce[i]);
-    const float rho = b.rho[i];
-    V3 acc = F / rho;
-    V3 half = v3(h4);
+    V3 x = v3(p4), v = v3(v4), half = v3(h4), old;
     float first = v4.w;
-    if (first != 0.f) {
-        half = v3(v4) - acc * P.dt / 2.f;
-        first = 0.f;
-    }
-    V3 old = half;
-    half = v3(half.x + acc.x * P.dt, half.y + acc.y * P.dt, half.z + acc.z * P.dt);
-    V3 x = v3(p4);
-    x = v3(x.x + half.x * P.dt, x.y + half.y * P.dt, x.z + half.z * P.dt);
-    collide_all(b.colliders + P.coll_off, P.ncoll, x, half, P);
-    V3 v = (old + half) / 2.f;
+    integrate_motion(P, b.colliders + P.coll_off, F, b.rho[i], x, v, first, half, old);
     b.pos[i] = f4(x, p4.w);
     b.vel[i] = f4(v, first);
     b.half[i] = f4(half, h4.w);
@@ -354,34 +473,45 @@ __device__ __forceinline__ void integrate_one(const DevParams& P, const StepBuff
     }
 }
 
-// PCISPHSolver.cpp:67-97 for one particle. Iteration 0 starts from p = 0, F_p = 0
-// (:58-62). aproximateVelocity (:96, SPHParticle.cpp:46-49) sets v = (v_half_old + v_half)/2;
-// within a step it is idempotent, so it is applied in iteration 0 only, after the
-// prediction has read v.
+// PCISPHSolver.cpp:67-95 for one particle: predicted half velocity and position under F + Fp. The
+// force pass divides by pair distances with div_by while every prediction of the step stays in its
+// exact range; one position outside switches it to IEEE division (DevStatus::div_unsafe).
+__device__ __forceinline__ void predict_motion(const DevParams& P, const Collider* cols, DevStatus* st, V3 F, V3 Fp,
+                                               float rho, V3 x, V3 v, float first, V3 half, V3& px, V3& ph)
+{
+    V3 acc = (F + Fp) / rho;
+    if (first != 0.f) half = v - acc * P.dt / 2.f;
+    ph = half + acc * P.dt;
+    px = x + ph * P.dt;
+    collide_all(cols, P.ncoll, px, ph, P);
+    if (!(exact_div_safe(px.x) && exact_div_safe(px.y) && exact_div_safe(px.z))) atomicOr(&st->div_unsafe, 1u);
+}
+// predict_motion on the stored state. Iteration 0 starts from p = 0, F_p = 0 (:58-62).
+// aproximateVelocity (:96, SPHParticle.cpp:46-49) sets v = (v_half_old + v_half)/2; within a step
+// it is idempotent, so it is applied in iteration 0 only, after the prediction has read v.
 __device__ __forceinline__ void pci_predict_one(const DevParams& P, const StepBuffers& b, int i, int iteration,
                                                 float4* ppos)
 {
     float4 v4 = b.vel[i];
-    V3 F = v3(b.force[i]);
-    V3 Fp = iteration == 0 ? v3(0.f, 0.f, 0.f) : v3(b.pforce[i]);
-    const float rho = b.rho[i];
-    V3 hv = v3(b.half[i]);
-    V3 acc = (F + Fp) / rho;
-    if (v4.w != 0.f) hv = v3(v4) - acc * P.dt / 2.f;
-    V3 ph = hv + acc * P.dt;
-    V3 px = v3(b.pos[i]) + ph * P.dt;
-    collide_all(b.colliders + P.coll_off, P.ncoll, px, ph, P);
-    // The force pass divides by pair distances with div_by while every prediction of the
-    // step stays in its exact range; one position outside switches it to IEEE division.
-    if (!(exact_div_safe(px.x) && exact_div_safe(px.y) && exact_div_safe(px.z))) atomicOr(&b.status->div_unsafe, 1u);
+    const V3 half = v3(b.half[i]);
+    const V3 Fp = iteration == 0 ? v3(0.f, 0.f, 0.f) : v3(b.pforce[i]);
+    V3 px, ph;
+    predict_motion(P, b.colliders + P.coll_off, b.status, v3(b.force[i]), Fp, b.rho[i], v3(b.pos[i]), v3(v4), v4.w, half,
+                   px, ph);
     ppos[i] = f4(px, 0.f);
     b.phalf[i] = f4(ph, 0.f);
     if (iteration == 0 && !P.keep_initial_velocity) {
-        V3 v = (v3(b.old[i]) + v3(b.half[i])) / 2.f;
+        V3 v = (v3(b.old[i]) + half) / 2.f;
         b.vel[i] = f4(v, v4.w);
     }
 }
 
+// W of the pairs of a particle at xi with particles at p and q.
+__device__ __forceinline__ F2 density_pair(const DevParams& P, const float* __restrict__ tables, V3 xi, float4 p, float4 q)
+{
+    return weight_w(neg_sqmag(f2(p.x - xi.x, q.x - xi.x), f2(p.y - xi.y, q.y - xi.y), f2(p.z - xi.z, q.z - xi.z)), P,
+                    tables);
+}
 // Sum of W over particle i's list at the positions x (a W of exactly 0 or more each: adding the
 // +0 of a masked second entry changes no bit).
 __device__ __forceinline__ float density_sum(const DevParams& P, const StepBuffers& b, const float4* x, int i)
@@ -390,29 +520,38 @@ __device__ __forceinline__ float density_sum(const DevParams& P, const StepBuffe
     float sum = 0.f;
     for_each_neighbor<4>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i), [&](int j) { return x[j]; },
                          [&](int, float4 p, int, float4 q, bool two) {
-                             const F2 w = weight_w(neg_sqmag(f2(p.x - xi.x, q.x - xi.x), f2(p.y - xi.y, q.y - xi.y),
-                                                             f2(p.z - xi.z, q.z - xi.z)),
-                                                   P, b.tables);
+                             const F2 w = density_pair(P, b.tables, xi, p, q);
                              sum += lo(w);
                              if (two) sum += hi(w);
                          });
     return sum;
 }
 
-// PCISPHSolver.cpp:100-126 for one particle; returns |error| (0 for NaN, which the
-// reference's std::max ignores).
-__device__ __forceinline__ float pci_density_one(const DevParams& P, const StepBuffers& b, int i, int iteration,
-                                                 float4* ppos)
+// PCISPHSolver.cpp:100-126 for one particle from its sum of W: predicted density, error and the
+// pressure p moved on.
+__device__ __forceinline__ void pressure_update(const DevParams& P, float sum, float& pd, float& er, float& p)
 {
-    const float sum = density_sum(P, b, ppos, i);
-    float pd = P.mass * sum;
-    float er = pd - P.rho0;
+    pd = P.mass * sum;
+    er = pd - P.rho0;
     float pp = P.delta * er;
     if (pp < 0.f) {
         er *= P.neg;
         pp *= P.neg;
     }
-    float p = (iteration == 0 ? 0.f : b.pres[i]) + pp;
+    p += pp;
+}
+// |error| for the maximum: 0 for NaN, which the reference's std::max ignores.
+__device__ __forceinline__ float error_magnitude(float er)
+{
+    const float a = fabsf(er);
+    return a == a ? a : 0.f;
+}
+// pressure_update on the stored state; returns the error's magnitude.
+__device__ __forceinline__ float pci_density_finish(const DevParams& P, const StepBuffers& b, int i, int iteration,
+                                                    float4* ppos, float sum)
+{
+    float pd, er, p = iteration == 0 ? 0.f : b.pres[i];
+    pressure_update(P, sum, pd, er, p);
     b.prho[i] = pd;
     b.err[i] = er;
     b.pres[i] = p;
@@ -420,8 +559,12 @@ __device__ __forceinline__ float pci_density_one(const DevParams& P, const StepB
     // pass fetches a neighbour's position and factor in one 16-byte load. Other threads
     // read only x*.xyz of this element during this pass.
     reinterpret_cast<float*>(ppos + i)[3] = p / (pd * pd);
-    float a = fabsf(er);
-    return a == a ? a : 0.f;
+    return error_magnitude(er);
+}
+__device__ __forceinline__ float pci_density_one(const DevParams& P, const StepBuffers& b, int i, int iteration,
+                                                 float4* ppos)
+{
+    return pci_density_finish(P, b, i, iteration, ppos, density_sum(P, b, ppos, i));
 }
 
 // PCISPHSolver.cpp:129-150 for one particle. s = p / rho*^2 is the per-particle factor the
@@ -430,6 +573,36 @@ __device__ __forceinline__ float pci_density_one(const DevParams& P, const StepB
 // with kExactDiv they come from sqrt_rn and one reciprocal of d (recip_rn, div_by), the same
 // bits for the predicted positions the step's predict passes found safe
 // (DevStatus::div_unsafe clear).
+// F_p from the sum over the pairs; a NaN sum counts as no force (PCISPHSolver.cpp:144-149).
+__device__ __forceinline__ V3 pci_pressure_force(const DevParams& P, float rho, V3 pf)
+{
+    pf *= -(P.mass * rho);
+    if (isnan(pf.x)) pf = v3(0.f, 0.f, 0.f);
+    return pf;
+}
+// The terms of one pair with IEEE operations, and of two pairs with the exact forms. A particle's
+// own entry gives NaN (0 / 0) and is left out by the caller.
+__device__ __forceinline__ V3 pci_force_term(const DevParams& P, const float* __restrict__ tables, V3 xi, float tf,
+                                             float4 p)
+{
+    // |x_i - x_j| rounds exactly like the reference's |x_j - x_i| (the squares are equal), so one
+    // difference serves both.
+    const V3 dq = xi - v3(p);
+    const float d = mag(dq);
+    const V3 dir = dq / d;
+    return dir * weight_sdw(d, P, tables) * (tf + p.w);
+}
+struct V3x2 {
+    F2 x, y, z;
+};
+__device__ __forceinline__ V3x2 pci_force_pair(const DevParams& P, const float* __restrict__ tables, V3 xi, float tf,
+                                               float4 p, float4 q)
+{
+    const F2 dx = f2(xi.x - p.x, xi.x - q.x), dy = f2(xi.y - p.y, xi.y - q.y), dz = f2(xi.z - p.z, xi.z - q.z);
+    const F2 nd = neg_sqrt_rn(neg_sqmag(dx, dy, dz)), y = recip_rn(nd);
+    const F2 w = weight_sdw(nd, P, tables), s = f2(tf + p.w, tf + q.w);
+    return V3x2{div_by(dx, nd, y) * w * s, div_by(dy, nd, y) * w * s, div_by(dz, nd, y) * w * s};
+}
 template <bool kExactDiv>
 __device__ __forceinline__ void pci_force_walk(const DevParams& P, const StepBuffers& b, int i, const float4* ppos)
 {
@@ -437,32 +610,18 @@ __device__ __forceinline__ void pci_force_walk(const DevParams& P, const StepBuf
     const V3 xi = v3(pi4);
     const float tf = pi4.w;
     V3 pf = v3(0.f, 0.f, 0.f);
-    auto one = [&](int j, float4 pj4) {
-        if (j == i) return;
-        // |x_i - x_j| rounds exactly like the reference's |x_j - x_i|
-        // (the squares are equal), so one difference serves both.
-        const V3 dq = xi - v3(pj4);
-        const float d = mag(dq);
-        V3 dir = dq / d;
-        pf += dir * weight_sdw(d, P, b.tables) * (tf + pj4.w);
-    };
     auto pair = [&](int j0, float4 p, int j1, float4 q, bool two) {
         if (!kExactDiv) {
-            one(j0, p);
-            if (two) one(j1, q);
+            if (j0 != i) pf += pci_force_term(P, b.tables, xi, tf, p);
+            if (two && j1 != i) pf += pci_force_term(P, b.tables, xi, tf, q);
             return;
         }
-        const F2 dx = f2(xi.x - p.x, xi.x - q.x), dy = f2(xi.y - p.y, xi.y - q.y), dz = f2(xi.z - p.z, xi.z - q.z);
-        const F2 nd = neg_sqrt_rn(neg_sqmag(dx, dy, dz)), y = recip_rn(nd);
-        const F2 w = weight_sdw(nd, P, b.tables), s = f2(tf + p.w, tf + q.w);
-        const F2 fx = div_by(dx, nd, y) * w * s, fy = div_by(dy, nd, y) * w * s, fz = div_by(dz, nd, y) * w * s;
-        if (j0 != i) pf += v3(lo(fx), lo(fy), lo(fz));
-        if (two && j1 != i) pf += v3(hi(fx), hi(fy), hi(fz));
+        const V3x2 f = pci_force_pair(P, b.tables, xi, tf, p, q);
+        if (j0 != i) pf += v3(lo(f.x), lo(f.y), lo(f.z));
+        if (two && j1 != i) pf += v3(hi(f.x), hi(f.y), hi(f.z));
     };
     for_each_neighbor<2>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i), [&](int j) { return ppos[j]; }, pair);
-    pf *= -(P.mass * b.rho[i]);
-    if (isnan(pf.x)) pf = v3(0.f, 0.f, 0.f);
-    b.pforce[i] = f4(pf, 0.f);
+    b.pforce[i] = f4(pci_pressure_force(P, b.rho[i], pf), 0.f);
 }
 __device__ __forceinline__ void pci_force_one(const DevParams& P, const StepBuffers& b, int i, const float4* ppos)
 {

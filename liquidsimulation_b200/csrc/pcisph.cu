@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
                                                              LoopSync* sy, uint32_t* maxerr, int first_done, int warm)
 {
     __shared__ float wmax[kLoopThreads / 32];
+    uint32_t epoch = 0;   // grid barriers passed
     // x* of iteration parity 0 / 1. A select, not a two-pointer array: an array indexed by
     // the iteration lives in local memory, and reading it per particle cost the loop 3.8 %.
     auto pp = [&](int parity) { return parity ? ppos_alt : b.ppos; };
@@ -170,9 +171,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
     bool conv = false, rejected = false;
     if (!first_done) {
         for_particles([&](int i) { pci_predict_one(P, b, i, 0, pp(0)); });
-        if (!grid_barrier(sy, b.status)) return;
+        if (!grid_barrier(sy, b.status, epoch)) return;
         density_pass(0, 0);
-        if (!grid_barrier(sy, b.status)) return;
+        if (!grid_barrier(sy, b.status, epoch)) return;
     }
     for (;;) {
         const float me = __uint_as_float(ld_volatile(&maxerr[kp]));
@@ -182,9 +183,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
             k = 0;
             kp++;
             for_particles([&](int i) { pci_predict_one(P, b, i, 0, pp(0)); });
-            if (!grid_barrier(sy, b.status)) return;
+            if (!grid_barrier(sy, b.status, epoch)) return;
             density_pass(0, kp);
-            if (!grid_barrier(sy, b.status)) return;
+            if (!grid_barrier(sy, b.status, epoch)) return;
             continue;
         }
         // PCISPHSolver.cpp:152-162: ratio = max|e| / rho0 in float, exit when below eta.
@@ -203,11 +204,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
             else integrate_one(P, b, i, 1);
         });
         if (done) break;
-        if (!grid_barrier(sy, b.status)) return;
+        if (!grid_barrier(sy, b.status, epoch)) return;
         k++;
         kp++;
         density_pass(k, kp);
-        if (!grid_barrier(sy, b.status)) return;
+        if (!grid_barrier(sy, b.status, epoch)) return;
     }
     if (tid == 0) {
         b.status->iterations = kp + 1;
@@ -277,13 +278,15 @@ bool launch_pci_loop(const DevParams& P, const StepBuffers& b, float4* ppos_alt,
 
 // ------------------------------------------------------------------ barrier probe
 //
-// One grid barrier with `parties` arrivals per round and a short spin limit, for the test
-// of the bounded wait: with fewer blocks than parties nothing completes the round, the
-// waiting blocks give up, raise kErrTimeout and leave, and the device stays usable.
+// One round of the loops' bounded wait with `parties` arrivals and a short spin limit, for the test
+// of that wait: the block that arrives as the a-th waits for the next multiple of the parties, so
+// with fewer blocks than that nothing completes the round, the waiting blocks give up, raise
+// kErrTimeout and leave, and the device stays usable.
 __global__ void k_barrier_probe(LoopSync* sy, DevStatus* st, uint32_t parties, unsigned long long limit, int* done)
 {
-    const bool ok = grid_barrier(sy, st, parties, limit);
-    if (threadIdx.x == 0 && ok) atomicAdd(done, 1);
+    if (threadIdx.x != 0) return;
+    const uint32_t arrived = atomicAdd(&sy->count, 1u);
+    if (barrier_wait(sy, st, (arrived / parties + 1u) * parties, limit)) atomicAdd(done, 1);
 }
 
 void barrier_probe(int blocks, int parties, int* completed, uint32_t* error_flags)

@@ -1,0 +1,317 @@
+// The whole step of a small scene in one cooperative launch: grid build, neighbour lists,
+// non-pressure forces, the pressure (SPH force or the PCISPH loop) and the integration, separated
+// by grid barriers, with a group of L lanes per particle where a neighbour list is walked
+// (group_ops.cuh). Each result carries the bits of the separate kernels (grid.cu, sph.cu,
+// pcisph.cu), which larger scenes use.
+//
+// What bounds a small scene is latency: at 1,200 particles the separate kernels took 134 us of
+// device time for a four-iteration step, in which the chip did about 2 us of work; a third of it
+// went into launches and memsets, the rest into serial walks. Here a group keeps its particle's
+// list and state in registers for the whole step, so a pass is one dependent fetch (the neighbours'
+// positions) and a barrier. A PCISPH step with 4 iterations, wall clock, separate kernels -> this:
+// 1,200 particles 89 -> 42 us, 4,700 145 -> 73, 9,400 156 -> 93, 18,900 177 -> 118, 30,000 203 ->
+// 180, 37,800 219 -> 188 us. About 1.2 us of it is each grid barrier (7 + 2 per iteration).
+//
+//   keys | scan sums | scan apply | scatter | rank + gather | lists + density |
+//   non-pressure + predict(0), then the loop of k_pci_loop       (PCISPH)
+//   non-pressure + pressure | integrate                          (SPH)
+//
+// Everything one phase writes and a later one reads goes through plain or L2 loads; the grid
+// barrier orders them.
+#include "group_ops.cuh"
+#include "host_util.h"
+#include "loop_sync.cuh"
+#include "scan_ops.cuh"
+#include "small_step.h"
+
+#include <mutex>
+
+namespace lsp {
+
+// 512 threads per SM leave each 128 registers: the groups keep their particle's list and state there.
+constexpr int kMaxThreads = 512;
+// Shared memory of a group in the build: one row of terms and the list.
+template <int L>
+constexpr int build_words()
+{
+    return group_pitch(L) + kGroupList;
+}
+
+template <int L>
+__global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
+{
+    extern __shared__ float4 dyn[];   // the groups' terms; in the build also their lists
+    __shared__ uint32_t ws[32];
+    __shared__ Collider cols[kMaxColliders];
+    __shared__ uint32_t block_max;
+    const GridBuildArgs& g = a.g;
+    const StepBuffers& b = a.b;
+    const DevParams& P = g.P;
+    DevStatus* st = b.status;
+    LoopSync* sy = reinterpret_cast<LoopSync*>(a.sync);
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = P.n;
+    uint32_t epoch = 0;
+    // A barrier that gave up tells the host at once: the status copy at the end is not reached.
+    auto barrier = [&]() {
+        const bool ok = grid_barrier(sy, st, epoch);
+        if (!ok && threadIdx.x == 0) a.host->error_flags = kErrTimeout;
+        return ok;
+    };
+    for (int w = threadIdx.x; w < P.ncoll * (int)(sizeof(Collider) / 4); w += blockDim.x)
+        reinterpret_cast<uint32_t*>(cols)[w] = reinterpret_cast<const uint32_t*>(b.colliders + P.coll_off)[w];
+
+    // ---- cell keys and histogram (k_keys_hist); thread t holds particle t until the gather
+    const bool mine = tid < n;
+    uint32_t key = 0xffffffffu;
+    float4 x4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool escaped = false, bad = false;
+    if (mine) {
+        x4 = __ldg(g.pos_in + tid);
+        key = cell_key(P, x4, escaped, bad);
+    }
+    const uint32_t slot = hist_slot(key, mine, g.hist);
+    record_key_flags(mine, escaped, bad, st);
+    if (!barrier()) return;
+
+    // ---- scan: each block owns a contiguous run of cells
+    const int64_t n8 = scan_entries((int64_t)P.cells + 1);
+    const int64_t per = (n8 / kScanItems + gridDim.x - 1) / gridDim.x * kScanItems;
+    const int64_t c0 = min((int64_t)blockIdx.x * per, n8), c1 = min(c0 + per, n8);
+    {
+        uint32_t s = 0;
+        for (int64_t e = c0 + (int64_t)threadIdx.x * kScanItems; e < c1; e += (int64_t)blockDim.x * kScanItems) {
+            uint32_t v[kScanItems];
+            load8(g.hist + e, v);
+#pragma unroll
+            for (int j = 0; j < kScanItems; j++) s += v[j];
+        }
+        uint32_t total;
+        block_exclusive_scan(s, ws, &total);
+        if (threadIdx.x == 0) g.tile_sums[blockIdx.x] = total;
+    }
+    if (!barrier()) return;
+    {
+        uint32_t s = 0, carry;
+        for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) s += __ldcg(g.tile_sums + k);
+        block_exclusive_scan(s, ws, &carry);
+        for (int64_t e0 = c0; e0 < c1; e0 += (int64_t)blockDim.x * kScanItems) {
+            const int64_t e = e0 + (int64_t)threadIdx.x * kScanItems;
+            uint32_t v[kScanItems] = {0, 0, 0, 0, 0, 0, 0, 0};
+            if (e < c1) load8(g.hist + e, v);
+            uint32_t sum = 0, total;
+#pragma unroll
+            for (int j = 0; j < kScanItems; j++) sum += v[j];
+            const uint32_t ex = block_exclusive_scan(sum, ws, &total) + carry;
+            if (e < c1) store8_scan(g.cell_start + e, g.hist + e, v, ex);
+            carry += total;
+        }
+    }
+    if (!barrier()) return;
+
+    // ---- scatter (k_scatter), then rank by caller id inside the cell and move the state
+    // (rank_gather_one, from the particle's side)
+    uint32_t beg = 0, end = 0;
+    if (mine) {
+        beg = __ldcg(g.cell_start + key);
+        end = __ldcg(g.cell_start + key + 1);
+        g.tmp[beg + slot] = make_int2(tid, id_of(x4));
+    }
+    if (!barrier()) return;
+    if (mine) {
+        const float4 v4 = __ldg(g.vel_in + tid), h4 = __ldg(g.half_in + tid), o4 = __ldg(g.old_in + tid);
+        const int id = id_of(x4);
+        uint32_t rank = 0;
+        if (end - beg <= (uint32_t)kMaxCellOccupancy) {
+            for (uint32_t q = beg; q < end; q++) rank += __ldcg(g.tmp + q).y < id ? 1u : 0u;
+        } else {
+            rank = slot;   // order inside an overfull cell is not the reference's
+            atomicOr(&st->error_flags, kErrScan);
+        }
+        const uint32_t dest = beg + rank;
+        store_sorted(g, dest, id, key, x4, v4, h4, o4);
+        if (g.hist_out) g.hist_out[dest] = __ldg(g.hist_in + tid);
+    }
+    if (!barrier()) return;
+
+    // ---- neighbour lists, density, pressure (k_neighbors_density); from here a group holds
+    // sorted particle i
+    const int i = min(tid / L, n - 1);
+    const bool valid = tid / L < n;
+    {
+        Group<L> own(reinterpret_cast<float*>(dyn));
+        own.row = reinterpret_cast<float*>(dyn) + (threadIdx.x / L) * build_words<L>();
+        int* list = reinterpret_cast<int*>(own.row + group_pitch(L));
+        float sum;
+        const int c = group_neighbors(own, P, b.pos, b.tables, g.cell_start, g.nbr, i, valid, list, &sum);
+        const bool first = valid && own.lane == 0;
+        if (first) store_density(P, i, c, sum, b.vel, g.nbr_count, g.rho, g.pres, g.vrho, st);
+        record_neighbor_count(P, c, first, st);
+    }
+    if (threadIdx.x == 0) block_max = 0u;
+    if (!barrier()) return;
+
+    const Group<L> grp(reinterpret_cast<float*>(dyn));
+    const HeldList<L> list(grp, P, b, i, valid);
+    const float4 p4 = b.pos[i], v4 = b.vel[i], h4 = b.half[i], o4 = b.old[i];
+    const float rho = b.rho[i];
+    const V3 x0 = v3(p4), half0 = v3(h4);
+    V3 v = v3(v4);
+    const bool lead = valid && grp.lane == 0;   // the lane that stores the particle's results
+    V3 F = group_nonpressure(grp, P, b, i, x0, v, rho, list);
+    auto integrate = [&](V3 total, float p) {
+        V3 x = x0, half = half0, old;
+        float first = v4.w;
+        integrate_motion(P, cols, total, rho, x, v, first, half, old);
+        if (!lead) return;
+        b.pos[i] = f4(x, p4.w);
+        b.vel[i] = f4(v, first);
+        b.half[i] = f4(half, h4.w);
+        b.old[i] = f4(old, o4.w);
+        if (b.hist) {
+            // Warm-start pressure history: (p_n, p_{n-1}, p_{n-2}) for the next step's features.
+            const float4 hs = b.hist[i];
+            b.hist[i] = make_float4(p, hs.x, hs.y, 0.f);
+        }
+    };
+
+    if (!a.pcisph) {
+        const float pres = b.pres[i];
+        F += group_sph_pressure(grp, P, b, i, x0, rho, pres, list);
+        if (!barrier()) return;   // the positions are read by other groups until here
+        integrate(F, pres);
+        if (tid == 0) *a.host = *st;
+        return;
+    }
+
+    // ---- PCISPH: the loop of k_pci_loop from zero pressure. All lanes follow the particle's
+    // predicted state.
+    auto pp = [&](int parity) { return parity ? a.ppos_alt : b.ppos; };
+    V3 px, ph;
+    predict_motion(P, cols, st, F, v3(0.f, 0.f, 0.f), rho, x0, v, v4.w, half0, px, ph);
+    if (lead) pp(0)[i] = f4(px, 0.f);
+    if (!P.keep_initial_velocity) v = (v3(o4) + half0) / 2.f;
+    float p = 0.f;
+    if (!barrier()) return;
+    for (int k = 0;; k++) {
+        const float sum = group_density_sum(grp, P, b.tables, pp(k & 1), px, list.cnt, list.most, list);
+        float pd, er;
+        pressure_update(P, sum, pd, er, p);
+        const float tf = p / (pd * pd);
+        if (lead) reinterpret_cast<float*>(pp(k & 1) + i)[3] = tf;
+        // Maximum of non-negative floats: their bit patterns order like the values.
+        const uint32_t mb = __reduce_max_sync(kFullWarp, lead ? __float_as_uint(error_magnitude(er)) : 0u);
+        if ((threadIdx.x & 31) == 0 && mb) atomicMax(&block_max, mb);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (block_max) atomicMax(&a.maxerr[k], block_max);
+            block_max = 0u;
+        }
+        if (!barrier()) return;
+        const uint32_t me = ld_volatile(&a.maxerr[k]);
+        // PCISPHSolver.cpp:152-162: ratio = max|e| / rho0 in float, exit when below eta.
+        const bool conv = fabsf(__uint_as_float(me) / P.rho0) < P.eta;
+        const bool done = (conv && k + 1 >= P.min_it) || k + 1 >= P.max_it;
+        const V3 Fp = group_pci_force(grp, P, b, i, pp(k & 1), px, tf, rho, list);
+        if (done) {
+            if (lead) {
+                b.prho[i] = pd;
+                b.err[i] = er;
+                b.pres[i] = p;
+                b.phalf[i] = f4(ph, 0.f);
+                b.pforce[i] = f4(Fp, 0.f);
+            }
+            F += Fp;
+            integrate(F, p);
+            if (tid == 0) {
+                st->iterations = k + 1;
+                st->converged = conv ? 1 : 0;
+                st->max_err_bits = me;
+                st->warm_used = 0;
+                st->last_k = k;
+                *a.host = *st;
+            }
+            return;
+        }
+        predict_motion(P, cols, st, F, Fp, rho, x0, v, v4.w, half0, px, ph);
+        if (lead) pp((k + 1) & 1)[i] = f4(px, 0.f);
+        if (!barrier()) return;
+    }
+}
+
+// ------------------------------------------------------------------ launch
+
+constexpr int kMaxDevices = 64;
+constexpr int kLaneChoices = 4;   // 16, 8, 4 and 2 lanes
+static const void* const g_kernel[kLaneChoices] = {(const void*)k_small_step<16>, (const void*)k_small_step<8>,
+                                                   (const void*)k_small_step<4>, (const void*)k_small_step<2>};
+template <int L>
+static size_t lanes_smem(int threads)
+{
+    const size_t walk = group_smem(threads, L), build = (size_t)(threads / L) * build_words<L>() * sizeof(float);
+    return walk > build ? walk : build;
+}
+static size_t step_smem(int choice, int threads)
+{
+    return choice == 0   ? lanes_smem<16>(threads)
+           : choice == 1 ? lanes_smem<8>(threads)
+           : choice == 2 ? lanes_smem<4>(threads)
+                         : lanes_smem<2>(threads);
+}
+// Whether a block of each choice fits an SM (asked once per device, under a lock: solvers on
+// different host threads may launch at once).
+static bool g_fits[kMaxDevices][kLaneChoices], g_ready[kMaxDevices];
+static std::mutex g_mutex;
+
+// As many lanes per particle as the threads allow: fewer lanes take longer walks (12,000 particles:
+// 93 us a step with 4 lanes). Beyond two lanes per particle the separate kernels, with one thread
+// per particle and full occupancy, are as fast (45,000 particles: 252 us either way).
+int small_step_lanes(int64_t n, int64_t cells)
+{
+    if (n <= 0 || cells > kSmallStepCells) return 0;
+    const int64_t threads = (int64_t)device_sm_count() * kMaxThreads;
+    for (int lanes = 16; lanes >= 2; lanes /= 2)
+        if (n * lanes <= threads) return lanes;
+    return 0;
+}
+
+bool launch_small_step(const SmallStepArgs& a, int lanes, cudaStream_t s)
+{
+    const int c = lanes == 16 ? 0 : lanes == 8 ? 1 : lanes == 4 ? 2 : 3;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+    bool fits;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        if (!g_ready[dev]) {
+            int coop = 0;
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+            for (int k = 0; k < kLaneChoices; k++) {
+                int per = 0;
+                const size_t smem = step_smem(k, kMaxThreads);
+                g_fits[dev][k] =
+                    coop &&
+                    cudaFuncSetAttribute(g_kernel[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
+                        cudaSuccess &&
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, g_kernel[k], kMaxThreads, smem) == cudaSuccess &&
+                    per > 0;
+            }
+            g_ready[dev] = true;
+        }
+        fits = g_fits[dev][c];
+    }
+    if (!fits) return false;
+    // One group per particle in one block per SM, as evenly as whole warps allow.
+    const int sms = device_sm_count();
+    const int64_t threads = (int64_t)a.g.P.n * lanes;
+    const int64_t per_sm = (threads + sms - 1) / sms;
+    const int block = (int)((per_sm + 63) / 64 * 64 < 128 ? 128 : (per_sm + 63) / 64 * 64);
+    if (block > kMaxThreads) return false;
+    const int grid = (int)((threads + block - 1) / block);
+    SmallStepArgs ac = a;
+    void* args[] = {&ac};
+    return cudaLaunchCooperativeKernel(g_kernel[c], dim3(grid), dim3(block), args, step_smem(c, block), s) ==
+           cudaSuccess;
+}
+
+}  // namespace lsp

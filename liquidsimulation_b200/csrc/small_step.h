@@ -1,0 +1,30 @@
+// Launch interface of the one-launch step of small scenes (small_step.cu).
+#pragma once
+
+#include "lsp_kernels.h"
+
+namespace lsp {
+
+struct SmallStepArgs {
+    GridBuildArgs g;
+    StepBuffers b;       // the buffers the grid build gathers into
+    float4* ppos_alt;
+    void* sync;          // 16 zeroed bytes
+    uint32_t* maxerr;    // max_it zeroed words
+    DevStatus* host;     // pinned: the step's status, written at its end
+    int pcisph;
+};
+
+// Largest grid box of the one-launch step, whose blocks scan a contiguous share of the cells each:
+// 1,200 particles take 42 us a step in 15,600 cells and 49 us in 1,000,000 (separate kernels 89).
+constexpr int64_t kSmallStepCells = 1 << 20;
+// Entries of tile_sums the one-launch step needs (one per block).
+constexpr int kSmallStepTiles = 1024;
+
+// Lanes per particle of the one-launch step for n particles in a grid of `cells`, 0 when the
+// separate kernels are used.
+int small_step_lanes(int64_t n, int64_t cells);
+// False when the device refuses the launch (the caller then runs the separate kernels).
+bool launch_small_step(const SmallStepArgs& a, int lanes, cudaStream_t s);
+
+}  // namespace lsp
