@@ -40,6 +40,7 @@ struct GridBuildArgs {
 };
 
 struct MlpPacked;
+struct MlpUmma;
 
 // Learned warm start inputs (device order). Features of particle i: feat[8*i .. 8*i+7].
 struct WarmArgs {
@@ -127,14 +128,15 @@ void launch_pci_density_first(const DevParams& P, const StepBuffers& b, const Wa
 // MLP (mlp.cu).
 void launch_mlp_pack(const float* master, MlpPacked* packed, cudaStream_t s);
 int mlp_grad_rows(int nb);
-void launch_mlp_grad(const MlpPacked* packed, const float* feat, const float* target, const int32_t* idx, int nb,
+// With draw > 0, the batch's nb rows are drawn from the first `draw` rows by a hash of the seed.
+void launch_mlp_grad(const MlpPacked* packed, const float* feat, const float* target, int draw, uint64_t seed, int nb,
                      float over_weight, float* partial, float* loss_partial, cudaStream_t s);
 // k_mlp_grad on exactly `blocks` blocks of 256 threads: writes blocks * 8 partial rows.
 void launch_mlp_grad_blocks(const MlpPacked* packed, const float* feat, const float* target, int nb, int blocks,
                             float* partial, float* loss_partial, cudaStream_t s);
 void launch_mlp_adam(const float* partial, const float* loss_partial, int rows, float* master, float* m1, float* m2,
-                     float* grad_out, float* loss_out, float lr, int step, int apply, cudaStream_t s);
-void launch_random_indices(int32_t* idx, int nb, int n, uint64_t seed, cudaStream_t s);
+                     float* grad_out, float* loss_out, MlpPacked* packed, MlpUmma* umma, float lr, int step, int apply,
+                     cudaStream_t s);
 
 // Gathers a per-particle field from device order into caller order.
 // comps: 1 (float) or 3 (xyz of a float4); src is float* or float4* accordingly.

@@ -31,8 +31,8 @@ void MlpModel::init(cudaStream_t s)
 
 void MlpModel::repack()
 {
-    launch_mlp_pack(master_.p, reinterpret_cast<MlpPacked*>(packed_.p), s_);
-    launch_mlp_pack_umma(master_.p, reinterpret_cast<MlpUmma*>(umma_.p), s_);
+    launch_mlp_pack(master_.p, packed_image(), s_);
+    launch_mlp_pack_umma(master_.p, umma_image(), s_);
     CK(cudaGetLastError());
 }
 
@@ -83,13 +83,12 @@ float MlpModel::train(const float* feat, const float* tgt, int64_t n, int iterat
     const int rows = mlp_grad_rows(batch);
     if (partial_.n < (size_t)rows * kMlpParams) partial_.alloc((size_t)rows * kMlpParams);
     if (loss_part_.n < (size_t)rows) loss_part_.alloc(rows);
-    if (idx_.n < (size_t)batch) idx_.alloc(batch);
     for (int it = 0; it < iterations; it++) {
-        launch_random_indices(idx_.p, batch, (int)n, seed * 1000003ull + (uint64_t)it, s_);
-        launch_mlp_grad(packed(), feat, tgt, idx_.p, batch, over_weight_, partial_.p, loss_part_.p, s_);
+        launch_mlp_grad(packed(), feat, tgt, (int)n, seed * 1000003ull + (uint64_t)it, batch, over_weight_, partial_.p,
+                        loss_part_.p, s_);
         step_++;
-        launch_mlp_adam(partial_.p, loss_part_.p, rows, master_.p, m1_.p, m2_.p, nullptr, loss_.p, lr, step_, 1, s_);
-        repack();
+        launch_mlp_adam(partial_.p, loss_part_.p, rows, master_.p, m1_.p, m2_.p, nullptr, loss_.p, packed_image(),
+                        umma_image(), lr, step_, 1, s_);
     }
     CK(cudaGetLastError());
     float loss = 0.f;
@@ -128,8 +127,9 @@ float MlpModel::gradient(const float* feat, const float* target, int64_t n, floa
     const int rows = mlp_grad_rows((int)n);
     if (partial_.n < (size_t)rows * kMlpParams) partial_.alloc((size_t)rows * kMlpParams);
     if (loss_part_.n < (size_t)rows) loss_part_.alloc(rows);
-    launch_mlp_grad(packed(), df, dt, nullptr, (int)n, 1.f, partial_.p, loss_part_.p, s_);
-    launch_mlp_adam(partial_.p, loss_part_.p, rows, master_.p, m1_.p, m2_.p, grad_.p, loss_.p, 0.f, 1, 0, s_);
+    launch_mlp_grad(packed(), df, dt, 0, 0, (int)n, 1.f, partial_.p, loss_part_.p, s_);
+    launch_mlp_adam(partial_.p, loss_part_.p, rows, master_.p, m1_.p, m2_.p, grad_.p, loss_.p, packed_image(),
+                    umma_image(), 0.f, 1, 0, s_);
     CK(cudaGetLastError());
     float loss = 0.f;
     CK(cudaMemcpyAsync(grad, grad_.p, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, s_));

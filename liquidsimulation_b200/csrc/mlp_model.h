@@ -38,9 +38,10 @@ public:
 
 private:
     void repack();
+    MlpPacked* packed_image() { return reinterpret_cast<MlpPacked*>(packed_.p); }
+    MlpUmma* umma_image() { return reinterpret_cast<MlpUmma*>(umma_.p); }
     cudaStream_t s_ = nullptr;
     DevArray<float> master_, m1_, m2_, partial_, loss_part_, grad_, loss_, io_;
-    DevArray<int32_t> idx_;
     DevArray<uint32_t> packed_, umma_, err_;
     int step_ = 0;
     float over_weight_ = 1.f;

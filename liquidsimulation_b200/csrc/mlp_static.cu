@@ -64,21 +64,20 @@ float* scratch_on(int device)
 
 namespace {
 
-// Sums the partial rows in a fixed order: grad[p] = sum_r partial[r][p], loss = sum_r loss[r] / n.
+// Sums the partial rows in a fixed order: grad[p] = sum_r partial[r][p], loss = sum_r loss[r] / n
+// (kSumCols parameters per block, the last block the losses).
 __global__ void k_static_reduce(const float* __restrict__ scratch, int rows, float inv_n, float* __restrict__ grad,
                                 float* __restrict__ loss)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    const float* loss_part = scratch + (int64_t)rows * kMlpParams;
-    if (p == 0) {
-        float l = 0.f;
-        for (int r = 0; r < rows; r++) l += loss_part[r];
-        *loss = l * inv_n;
+    __shared__ SumBuffer buf;
+    if (blockIdx.x == gridDim.x - 1) {
+        const float l = ordered_sum(scratch + (int64_t)rows * kMlpParams, rows, buf);
+        if (threadIdx.x == 0) *loss = l * inv_n;
+        return;
     }
-    if (p >= kMlpParams) return;
-    float g = 0.f;
-    for (int r = 0; r < rows; r++) g += scratch[(int64_t)r * kMlpParams + p];
-    grad[p] = g;
+    const float g = ordered_column_sum(scratch, rows, kMlpParams, blockIdx.x * kSumCols, buf);
+    const int p = blockIdx.x * kSumCols + (int)threadIdx.x;
+    if (threadIdx.x < kSumCols && p < kMlpParams) grad[p] = g;
 }
 
 // Device memory of `device` itself, or managed memory (reachable from every device). Memory
@@ -120,7 +119,7 @@ extern "C" int lsp_mlp_gradient_static(lsp_solver* s, const float* features, con
         lsp::launch_mlp_grad_blocks(reinterpret_cast<const lsp::MlpPacked*>(e.mlp_packed_device()), features,
                                     targets, (int)n, lsp::kStaticBlocks, scratch,
                                     scratch + (int64_t)lsp::kStaticRows * lsp::kMlpParams, st);
-        lsp::k_static_reduce<<<(lsp::kMlpParams + 255) / 256, 256, 0, st>>>(scratch, lsp::kStaticRows,
+        lsp::k_static_reduce<<<lsp::sum_blocks(lsp::kMlpParams), lsp::kSumThreads, 0, st>>>(scratch, lsp::kStaticRows,
                                                                           1.f / (float)n, grad, loss);
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) throw lsp::Error(LSP_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(err));
