@@ -243,9 +243,9 @@ __device__ __forceinline__ void store_sorted(const GridBuildArgs& g, uint32_t de
     g.pos_out[dest] = x;
     g.vel_out[dest] = v;
     // The non-pressure pass divides pair terms by densities with div_by while every position
-    // and velocity of the step is in exact_div_safe's range.
-    if (!(exact_div_safe(x.x) && exact_div_safe(x.y) && exact_div_safe(x.z) && exact_div_safe(v.x) &&
-          exact_div_safe(v.y) && exact_div_safe(v.z)))
+    // and velocity of the step is in range.
+    if (!(exact_div_safe(x.x) && exact_div_safe(x.y) && exact_div_safe(x.z) && exact_div_velocity(v.x) &&
+          exact_div_velocity(v.y) && exact_div_velocity(v.z)))
         atomicOr(&g.status->np_unsafe, 1u);
     g.half_out[dest] = half;
     g.old_out[dest] = old;
