@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
     LoopSync* sy = reinterpret_cast<LoopSync*>(l.sync);
     DevStatus* gst = a.st + S;
     uint32_t epoch = 0;   // grid barriers passed
+    const bool any_first = ld_volatile(&gst->any_first) != 0u;
     // Predicted positions of iteration k live in buffer k & 1 (selected, not indexed, so the
     // pair stays in registers).
     auto pp = [&](int k) { return (k & 1) ? l.ppos_alt : b.ppos; };
@@ -351,15 +352,13 @@ __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuff
             const int act = st_act(w), k = st_k(w);
             const int i = P.base + j * T + (int)threadIdx.x;
             if (i >= P.base + P.n) return;
-            // One call site each for the force walk and the prediction (separate call sites
-            // per action spilled 148 bytes; this form 84, batched step 2 % faster). A restart
-            // (k = 0) only predicts iteration 0; a step adds force(k - 1) before predict(k);
-            // the scene's last pass is force(k), then the integration and collisions (own
-            // data only; the scenes never read each other's particles).
-            const bool restart = act == ACT_RESTART, last = act == ACT_FINAL;
-            if (!restart) pci_force_one(P, b, i, pp(last ? k : k - 1));
-            if (!last) pci_predict_one(P, b, i, k, pp(k));
-            else integrate_one(P, b, i, 1);
+            // A restart (k = 0) only predicts iteration 0; a step is force(k - 1) and predict(k); the
+            // scene's last pass is force(k), then the integration and collisions (own data only; the
+            // scenes never read each other's particles).
+            if (act == ACT_RESTART)
+                pci_predict_one(P, b, i, 0, pp(0));
+            else
+                pci_force_and_move(P, b, i, pp(act == ACT_FINAL ? k : k - 1), pp(k), act == ACT_FINAL, any_first);
         });
         if (preB[S] == 0) break;
         if (!grid_barrier(sy, gst, epoch)) return;

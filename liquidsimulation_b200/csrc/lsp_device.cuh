@@ -54,7 +54,8 @@ struct DevStatus {
     uint32_t div_unsafe;        // a predicted position left exact_div_safe's range this step
     uint32_t np_unsafe;         // a start-of-step position, velocity or density left the range
                                 // where the non-pressure pass divides with div_by
-    uint32_t pad[2];
+    uint32_t any_first;         // a particle is on its first step
+    uint32_t pad;
 };
 
 struct DevParams {
@@ -408,11 +409,12 @@ template <bool kNan>
 __device__ __forceinline__ F2 slot_from(F2 nguess, float inv_step, bool& unsure0, bool& unsure1)
 {
     const F2 t = fma2(nguess, f2(-inv_step), f2(-kSlotHalf));
-    const F2 k = (t + f2(kSlotMagic)) + f2(-kSlotMagic);
+    // The constants are shared where they can be (a packed constant takes two registers).
+    const F2 k = (t + f2(kSlotMagic)) - f2(kSlotMagic);
     const F2 f = t - k;
-    const F2 m = fma2(k, f2(-kSlotEps), f2(kSlotHalf));
-    unsure0 = kNan ? !(fabsf(lo(f)) <= lo(m)) : fabsf(lo(f)) > lo(m);
-    unsure1 = kNan ? !(fabsf(hi(f)) <= hi(m)) : fabsf(hi(f)) > hi(m);
+    const F2 m = fma2(k, f2(kSlotEps), f2(-kSlotHalf));   // the margin, negated
+    unsure0 = kNan ? !(fabsf(lo(f)) <= -lo(m)) : fabsf(lo(f)) > -lo(m);
+    unsure1 = kNan ? !(fabsf(hi(f)) <= -hi(m)) : fabsf(hi(f)) > -hi(m);
     return k;
 }
 __device__ __forceinline__ F2 slot_sq(F2 ns, const DevParams& P, const float* __restrict__ tables)

@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
 
     int k = 0, kp = 0;
     bool conv = false, rejected = false;
+    const bool first = ld_volatile(&b.status->any_first) != 0u;
     if (!first_done) {
         for_particles([&](int i) { pci_predict_one(P, b, i, 0, pp(0)); });
         if (!grid_barrier(sy, b.status, epoch)) return;
@@ -194,15 +195,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pci_loop(DevParams P, StepB
         // A learned guess is only checked at iteration 1, so a warm step cannot stop at 0.
         const bool unverified = warm && !rejected && k == 0;
         const bool done = (conv && k + 1 >= P.min_it && !unverified) || (k + 1 >= P.max_it);
-        for_particles([&](int i) {
-            pci_force_one(P, b, i, pp(k & 1));
-            // The last pass also integrates and collides the particle (SPHParticle::integrate
-            // after the loop, PCISPHSolver.cpp:166-169): it reads only the particle's own
-            // state and pressure force, which this thread has just written, and no thread of
-            // this pass reads what it writes (the force pass reads predicted positions).
-            if (!done) pci_predict_one(P, b, i, k + 1, pp((k + 1) & 1));
-            else integrate_one(P, b, i, 1);
-        });
+        // The last pass also integrates and collides the particle (SPHParticle::integrate
+        // after the loop, PCISPHSolver.cpp:166-169): it reads only the particle's own
+        // state and pressure force, which this thread has just computed, and no thread of
+        // this pass reads what it writes (the force pass reads predicted positions).
+        for_particles([&](int i) { pci_force_and_move(P, b, i, pp(k & 1), pp((k + 1) & 1), done, first); });
         if (done) break;
         if (!grid_barrier(sy, b.status, epoch)) return;
         k++;
