@@ -250,8 +250,7 @@ int lsp_synchronize(lsp_solver* s)
 int lsp_read_particles(lsp_solver* s, float* xyz, float* vel, int64_t n)
 {
     return lsp::guard([&] {
-        if (xyz) E(s).read_field(LSP_FIELD_POSITION, xyz, n);
-        if (vel) E(s).read_field(LSP_FIELD_VELOCITY, vel, n);
+        E(s).read_particles(xyz, vel, n);
     });
 }
 int lsp_read_field(lsp_solver* s, int field, float* out, int64_t n)

@@ -692,15 +692,21 @@ void BatchEngine::read_field(int scene, int field, float* out, int64_t n)
     case LSP_FIELD_NEIGHBOR_COUNT: break;
     default: throw Error(LSP_ERR_INVALID, "unknown field");
     }
-    stage((size_t)n * comps);
     const int32_t* soi = slot_of_id_.p + s.base;
+    const size_t bytes = (size_t)n * comps * sizeof(float);
+    HostTransfer h(hstage_, false);
+    h.add(out, bytes);
+    const bool direct = bytes <= kDirectTransferBytes && h.ready();
+    if (!direct) stage((size_t)n * comps);
+    float* to = direct ? (float*)h.view(0) : stage_.p;
     if (field == LSP_FIELD_NEIGHBOR_COUNT)
-        launch_gather_count(nbr_count_.p, soi, stage_.p, n, stream_);
+        launch_gather_count(nbr_count_.p, soi, to, n, stream_);
     else
-        launch_gather_field(src, comps, mode, soi, stage_.p, n, stream_);
+        launch_gather_field(src, comps, mode, soi, to, n, stream_);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, stage_.p, (size_t)n * comps * sizeof(float), cudaMemcpyDeviceToHost, stream_));
+    if (!direct) CK(cudaMemcpyAsync(out, stage_.p, bytes, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
+    if (direct) h.finish();
 }
 
 void BatchEngine::read_neighbors(int scene, int64_t* offsets, int32_t* index, int64_t n, int64_t capacity)
@@ -763,6 +769,19 @@ void BatchEngine::read_state(float* x, float* v, float* half, float* old, int32_
     if (n != n_ || !x || !v || !half || !old || !first) throw Error(LSP_ERR_INVALID, "read_state: bad arguments");
     if (!built_) throw Error(LSP_ERR_STATE, "no step has run");
     activate();
+    if ((size_t)n * 52 <= kDirectTransferBytes) {
+        HostTransfer h(hstage_, false);
+        for (float* p : {x, v, half, old}) h.add(p, (size_t)n * 3 * sizeof(float));
+        h.add(first, (size_t)n * sizeof(int32_t));
+        if (h.ready()) {
+            launch_gather_state(pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, slot_of_id_.p, (float*)h.view(0),
+                                (float*)h.view(1), (float*)h.view(2), (float*)h.view(3), (int32_t*)h.view(4), n, stream_);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream_));
+            h.finish();
+            return;
+        }
+    }
     stage((size_t)n * 13);
     float* s = stage_.p;
     launch_gather_state(pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, slot_of_id_.p, s, s + 3 * n,
@@ -783,6 +802,19 @@ void BatchEngine::write_state(const float* x, const float* v, const float* half,
     if (n != n_ || !x || !v || !half || !old || !first) throw Error(LSP_ERR_INVALID, "write_state: bad arguments");
     if (!built_) throw Error(LSP_ERR_STATE, "no step has run");
     activate();
+    if ((size_t)n * 52 <= kDirectTransferBytes) {
+        HostTransfer h(hstage_, true);
+        for (const float* p : {x, v, half, old}) h.add(p, (size_t)n * 3 * sizeof(float));
+        h.add(first, (size_t)n * sizeof(int32_t));
+        if (h.ready()) {
+            launch_scatter_state((const float*)h.view(0), (const float*)h.view(1), (const float*)h.view(2),
+                                 (const float*)h.view(3), (const int32_t*)h.view(4), slot_of_id_.p, pos_[cur_].p,
+                                 vel_[cur_].p, half_[cur_].p, old_[cur_].p, n, stream_);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream_));
+            return;
+        }
+    }
     stage((size_t)n * 13);
     float* s = stage_.p;
     size_t b3 = (size_t)n * 3 * sizeof(float);

@@ -120,6 +120,7 @@ private:
     DevArray<int2> tmp_;
     DevArray<int32_t> slot_of_id_, nbr_, nbr_count_;
     DevArray<float> tables_, stage_;
+    HostStage hstage_;
     DevArray<Collider> dcols_;
     DevArray<DevParams> dparams_;
     DevArray<BatchItem> items_;

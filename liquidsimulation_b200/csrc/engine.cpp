@@ -919,13 +919,41 @@ void Engine::read_field(int field, float* out, int64_t n)
     case LSP_FIELD_NEIGHBOR_COUNT: break;
     default: throw Error(LSP_ERR_INVALID, "unknown field");
     }
-    stage((size_t)n * comps);
+    const size_t bytes = (size_t)n * comps * sizeof(float);
+    HostTransfer h(hstage_, false);
+    h.add(out, bytes);
+    const bool direct = bytes <= kDirectTransferBytes && h.ready();
+    if (!direct) stage((size_t)n * comps);
+    float* to = direct ? (float*)h.view(0) : stage_.p;
     if (field == LSP_FIELD_NEIGHBOR_COUNT)
-        launch_gather_count(nbr_count_.p, slot_of_id_.p, stage_.p, n, stream_);
+        launch_gather_count(nbr_count_.p, slot_of_id_.p, to, n, stream_);
     else
-        launch_gather_field(src, comps, mode, slot_of_id_.p, stage_.p, n, stream_);
-    CK(cudaMemcpyAsync(out, stage_.p, (size_t)n * comps * sizeof(float), cudaMemcpyDeviceToHost, stream_));
+        launch_gather_field(src, comps, mode, slot_of_id_.p, to, n, stream_);
+    CK(cudaGetLastError());
+    if (!direct) CK(cudaMemcpyAsync(out, stage_.p, bytes, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
+    if (direct) h.finish();
+}
+
+// Positions and velocities (lsp_read_particles): one launch and one wait for both.
+void Engine::read_particles(float* x, float* v, int64_t n)
+{
+    if (x && v && n == n_ && n > 0 && (size_t)n * 24 <= kDirectTransferBytes) {
+        activate();
+        HostTransfer h(hstage_, false);
+        h.add(x, (size_t)n * 3 * sizeof(float));
+        h.add(v, (size_t)n * 3 * sizeof(float));
+        if (h.ready()) {
+            launch_gather_particles(pos_[cur_].p, vel_[cur_].p, slot_of_id_.p, (float*)h.view(0), (float*)h.view(1), n,
+                                    stream_);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream_));
+            h.finish();
+            return;
+        }
+    }
+    if (x) read_field(LSP_FIELD_POSITION, x, n);
+    if (v) read_field(LSP_FIELD_VELOCITY, v, n);
 }
 
 void Engine::read_state(float* x, float* v, float* half, float* old, int32_t* first, int64_t n)
@@ -933,6 +961,19 @@ void Engine::read_state(float* x, float* v, float* half, float* old, int32_t* fi
     if (n != n_ || !x || !v || !half || !old || !first) throw Error(LSP_ERR_INVALID, "read_state: bad arguments");
     if (n == 0) return;
     activate();
+    if ((size_t)n * 52 <= kDirectTransferBytes) {
+        HostTransfer h(hstage_, false);
+        for (float* p : {x, v, half, old}) h.add(p, (size_t)n * 3 * sizeof(float));
+        h.add(first, (size_t)n * sizeof(int32_t));
+        if (h.ready()) {
+            launch_gather_state(pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, slot_of_id_.p, (float*)h.view(0),
+                                (float*)h.view(1), (float*)h.view(2), (float*)h.view(3), (int32_t*)h.view(4), n, stream_);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream_));
+            h.finish();
+            return;
+        }
+    }
     stage((size_t)n * 13);
     float* s = stage_.p;
     launch_gather_state(pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, slot_of_id_.p, s, s + 3 * n,
@@ -952,6 +993,20 @@ void Engine::write_state(const float* x, const float* v, const float* half, cons
     if (n != n_ || !x || !v || !half || !old || !first) throw Error(LSP_ERR_INVALID, "write_state: bad arguments");
     if (n == 0) return;
     activate();
+    if ((size_t)n * 52 <= kDirectTransferBytes) {
+        HostTransfer h(hstage_, true);
+        for (const float* p : {x, v, half, old}) h.add(p, (size_t)n * 3 * sizeof(float));
+        h.add(first, (size_t)n * sizeof(int32_t));
+        if (h.ready()) {
+            launch_scatter_state((const float*)h.view(0), (const float*)h.view(1), (const float*)h.view(2),
+                                 (const float*)h.view(3), (const int32_t*)h.view(4), slot_of_id_.p, pos_[cur_].p,
+                                 vel_[cur_].p, half_[cur_].p, old_[cur_].p, n, stream_);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream_));
+            if (domain_from_particles_) grid_valid_ = false;
+            return;
+        }
+    }
     stage((size_t)n * 13);
     float* s = stage_.p;
     size_t b3 = (size_t)n * 3 * sizeof(float);

@@ -11,6 +11,7 @@
 
 #include "../../include/lsp.h"
 #include "host_util.h"
+#include "host_view.h"
 #include "lsp_kernels.h"
 #include "mlp_model.h"
 
@@ -97,6 +98,7 @@ public:
     void synchronize();
 
     void read_field(int field, float* out, int64_t n);
+    void read_particles(float* x, float* v, int64_t n);
     void read_state(float* x, float* v, float* half, float* old, int32_t* first, int64_t n);
     void write_state(const float* x, const float* v, const float* half, const float* old, const int32_t* first,
                      int64_t n);
@@ -187,6 +189,7 @@ private:
     DevStatus* status() const { return &ctl_.p->status; }
     DevStatus* hstatus_ = nullptr;   // pinned
     DevArray<float> stage_;
+    HostStage hstage_;
 
     // Launch bracketing for the per-class profile.
     template <typename F>

@@ -12,15 +12,92 @@ namespace lsp {
 constexpr int kThreads = 256;
 static inline unsigned blocks_for(int64_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
-__global__ void k_gather_vec(const float4* __restrict__ src, const int32_t* __restrict__ slot_of_id,
-                             float* __restrict__ out, int64_t n)
+// Rows of three floats between caller order (packed, possibly host memory) and device slots: a
+// block moves 256 consecutive rows of up to four arrays and the first-step flags. The packed side
+// goes through shared memory, so that it is read and written contiguously, 16 bytes at a time where
+// every array's alignment allows (a row at a time it would be three strided accesses, each a
+// request of its own over PCIe).
+struct RowArrays {
+    const float4* slots[4];
+    float* rows[4];
+    int count;
+    const float4* flag_slots;   // w != 0 is the flag, null when there are no flags
+    int32_t* flags;
+};
+
+// Moves `floats` floats between shared and packed memory (kStore: to packed).
+template <bool kVector, bool kStore>
+__device__ __forceinline__ void move_rows(float* packed, float* sm, int floats)
 {
-    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    int done = 0;
+    if (kVector) {
+        done = floats & ~3;
+        for (int k = 4 * threadIdx.x; k < done; k += 4 * blockDim.x) {
+            if (kStore) *reinterpret_cast<float4*>(packed + k) = *reinterpret_cast<const float4*>(sm + k);
+            else *reinterpret_cast<float4*>(sm + k) = *reinterpret_cast<const float4*>(packed + k);
+        }
+    }
+    for (int k = done + threadIdx.x; k < floats; k += blockDim.x) {
+        if (kStore) packed[k] = sm[k];
+        else sm[k] = packed[k];
+    }
+}
+
+template <bool kVector>
+__global__ void __launch_bounds__(kThreads) k_gather_rows3(RowArrays a, const int32_t* __restrict__ slot_of_id, int64_t n)
+{
+    __shared__ alignas(16) float sm[4][3 * kThreads];
+    const int64_t base = (int64_t)blockIdx.x * kThreads, id = base + threadIdx.x;
+    if (id < n) {
+        const int32_t s = slot_of_id[id];
+        for (int c = 0; c < a.count; c++) {
+            const float4 v = a.slots[c][s];
+            sm[c][3 * threadIdx.x] = v.x;
+            sm[c][3 * threadIdx.x + 1] = v.y;
+            sm[c][3 * threadIdx.x + 2] = v.z;
+        }
+        if (a.flag_slots) a.flags[id] = a.flag_slots[s].w != 0.f ? 1 : 0;
+    }
+    __syncthreads();
+    const int floats = 3 * (int)min((int64_t)kThreads, n - base);
+    for (int c = 0; c < a.count; c++) move_rows<kVector, true>(a.rows[c] + 3 * base, sm[c], floats);
+}
+
+// The other way for the whole state: positions (w: caller id), velocities (w: flag), half and old
+// half velocities (w kept).
+template <bool kVector>
+__global__ void __launch_bounds__(kThreads) k_scatter_state(RowArrays a, float4* pos, float4* vel, float4* hv, float4* ov,
+                                                            const int32_t* __restrict__ slot_of_id, int64_t n)
+{
+    __shared__ alignas(16) float sm[4][3 * kThreads];
+    const int64_t base = (int64_t)blockIdx.x * kThreads, id = base + threadIdx.x;
+    const int floats = 3 * (int)min((int64_t)kThreads, n - base);
+#pragma unroll
+    for (int c = 0; c < 4; c++) move_rows<kVector, false>(a.rows[c] + 3 * base, sm[c], floats);
+    const int32_t flag = id < n ? a.flags[id] : 0;
+    const int32_t s = id < n ? slot_of_id[id] : 0;
+    __syncthreads();
     if (id >= n) return;
-    float4 v = src[slot_of_id[id]];
-    out[3 * id] = v.x;
-    out[3 * id + 1] = v.y;
-    out[3 * id + 2] = v.z;
+    auto row = [&](int c, float w) {
+        return make_float4(sm[c][3 * threadIdx.x], sm[c][3 * threadIdx.x + 1], sm[c][3 * threadIdx.x + 2], w);
+    };
+    pos[s] = row(0, __int_as_float((int)id));
+    vel[s] = row(1, flag ? 1.f : 0.f);
+    hv[s] = row(2, hv[s].w);
+    ov[s] = row(3, ov[s].w);
+}
+
+static bool aligned_rows(const RowArrays& a)
+{
+    for (int c = 0; c < a.count; c++)
+        if ((uintptr_t)a.rows[c] % sizeof(float4)) return false;
+    return true;
+}
+static void gather_rows3(const RowArrays& a, const int32_t* slot_of_id, int64_t n, cudaStream_t s)
+{
+    if (!n) return;
+    if (aligned_rows(a)) k_gather_rows3<true><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
+    else k_gather_rows3<false><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
 }
 
 __global__ void k_gather_w(const float4* __restrict__ src, const int32_t* __restrict__ slot_of_id,
@@ -59,9 +136,13 @@ void launch_gather_field(const void* src, int comps, int mode, const int32_t* sl
                          cudaStream_t s)
 {
     if (!n) return;
-    if (comps == 3)
-        k_gather_vec<<<blocks_for(n), kThreads, 0, s>>>((const float4*)src, slot_of_id, out, n);
-    else if (mode == 1)
+    if (comps == 3) {
+        RowArrays a{};
+        a.slots[0] = (const float4*)src;
+        a.rows[0] = out;
+        a.count = 1;
+        gather_rows3(a, slot_of_id, n, s);
+    } else if (mode == 1)
         k_gather_w<<<blocks_for(n), kThreads, 0, s>>>((const float4*)src, slot_of_id, out, n);
     else if (mode == 2)
         k_gather_sqlen<<<blocks_for(n), kThreads, 0, s>>>((const float4*)src, slot_of_id, out, n);
@@ -74,27 +155,30 @@ void launch_gather_count(const int32_t* count, const int32_t* slot_of_id, float*
     if (n) k_gather_count<<<blocks_for(n), kThreads, 0, s>>>(count, slot_of_id, out, n);
 }
 
-__global__ void k_scatter_state(const float* __restrict__ x, const float* __restrict__ v,
-                                const float* __restrict__ h, const float* __restrict__ o,
-                                const int32_t* __restrict__ first, const int32_t* __restrict__ slot_of_id,
-                                float4* pos, float4* vel, float4* hv, float4* ov, int64_t n)
+void launch_gather_particles(const float4* pos, const float4* vel, const int32_t* slot_of_id, float* x, float* v,
+                             int64_t n, cudaStream_t s)
 {
-    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    int32_t s = slot_of_id[id];
-    pos[s] = make_float4(x[3 * id], x[3 * id + 1], x[3 * id + 2], __int_as_float((int)id));
-    vel[s] = make_float4(v[3 * id], v[3 * id + 1], v[3 * id + 2], first[id] ? 1.f : 0.f);
-    float4 a = hv[s], b = ov[s];
-    hv[s] = make_float4(h[3 * id], h[3 * id + 1], h[3 * id + 2], a.w);
-    ov[s] = make_float4(o[3 * id], o[3 * id + 1], o[3 * id + 2], b.w);
+    RowArrays a{};
+    a.slots[0] = pos;
+    a.slots[1] = vel;
+    a.rows[0] = x;
+    a.rows[1] = v;
+    a.count = 2;
+    gather_rows3(a, slot_of_id, n, s);
 }
 
 void launch_scatter_state(const float* x, const float* v, const float* half, const float* old, const int32_t* first,
                           const int32_t* slot_of_id, float4* pos, float4* vel, float4* hvel, float4* oldv,
                           int64_t n, cudaStream_t s)
 {
-    if (n) k_scatter_state<<<blocks_for(n), kThreads, 0, s>>>(x, v, half, old, first, slot_of_id, pos, vel, hvel,
-                                                               oldv, n);
+    if (!n) return;
+    RowArrays a{};
+    const float* rows[4] = {x, v, half, old};
+    for (int c = 0; c < 4; c++) a.rows[c] = const_cast<float*>(rows[c]);
+    a.count = 4;
+    a.flags = const_cast<int32_t*>(first);
+    if (aligned_rows(a)) k_scatter_state<true><<<blocks_for(n), kThreads, 0, s>>>(a, pos, vel, hvel, oldv, slot_of_id, n);
+    else k_scatter_state<false><<<blocks_for(n), kThreads, 0, s>>>(a, pos, vel, hvel, oldv, slot_of_id, n);
 }
 
 __global__ void k_scatter_vec(const float* __restrict__ in, const int32_t* __restrict__ slot_of_id,
@@ -110,28 +194,21 @@ void launch_scatter_vec(const float* in, const int32_t* slot_of_id, float4* dst,
     if (n) k_scatter_vec<<<blocks_for(n), kThreads, 0, s>>>(in, slot_of_id, dst, n);
 }
 
-__global__ void k_gather_state(const float4* __restrict__ pos, const float4* __restrict__ vel,
-                               const float4* __restrict__ hv, const float4* __restrict__ ov,
-                               const int32_t* __restrict__ slot_of_id, float* x, float* v, float* h, float* o,
-                               int32_t* first, int64_t n)
-{
-    const int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    int32_t s = slot_of_id[id];
-    float4 a = pos[s], b = vel[s], c = hv[s], d = ov[s];
-    x[3 * id] = a.x; x[3 * id + 1] = a.y; x[3 * id + 2] = a.z;
-    v[3 * id] = b.x; v[3 * id + 1] = b.y; v[3 * id + 2] = b.z;
-    h[3 * id] = c.x; h[3 * id + 1] = c.y; h[3 * id + 2] = c.z;
-    o[3 * id] = d.x; o[3 * id + 1] = d.y; o[3 * id + 2] = d.z;
-    first[id] = b.w != 0.f ? 1 : 0;
-}
-
 void launch_gather_state(const float4* pos, const float4* vel, const float4* hvel, const float4* oldv,
                          const int32_t* slot_of_id, float* x, float* v, float* half, float* old, int32_t* first,
                          int64_t n, cudaStream_t s)
 {
-    if (n) k_gather_state<<<blocks_for(n), kThreads, 0, s>>>(pos, vel, hvel, oldv, slot_of_id, x, v, half, old,
-                                                              first, n);
+    RowArrays a{};
+    const float4* slots[4] = {pos, vel, hvel, oldv};
+    float* rows[4] = {x, v, half, old};
+    for (int c = 0; c < 4; c++) {
+        a.slots[c] = slots[c];
+        a.rows[c] = rows[c];
+    }
+    a.count = 4;
+    a.flag_slots = vel;
+    a.flags = first;
+    gather_rows3(a, slot_of_id, n, s);
 }
 
 __global__ void k_neighbor_export(const int32_t* __restrict__ nbr, const int32_t* __restrict__ count, int64_t stride,
