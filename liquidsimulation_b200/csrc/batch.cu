@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(T) kb_neighbors_density(BatchArgs a, const flo
                                                           const uint32_t* __restrict__ cell_start,
                                                           int32_t* __restrict__ nbr, int32_t* __restrict__ count,
                                                           float* __restrict__ rho, float* __restrict__ pres,
-                                                          const float4* __restrict__ vel, float4* __restrict__ vrho)
+                                                          const float4* __restrict__ vel, float4* __restrict__ vrho,
+                                                          float4* __restrict__ xpf)
 {
     __shared__ DevParams P;
     const BatchItem it = a.items[blockIdx.x];
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(T) kb_neighbors_density(BatchArgs a, const flo
         c = neighbors_one(P, pos, cell_start, nbr, i, scene_tables(a, it.scene), masks + threadIdx.x, T, &sum);
         // The range check of the density is batch-wide, like the rest of the non-pressure pass's
         // (rank_gather_one).
-        store_density(P, i, c, sum, vel, count, rho, pres, vrho, a.st + a.scenes);
+        store_density(P, i, c, sum, pos, vel, count, rho, pres, vrho, xpf, a.st + a.scenes);
     }
     record_neighbor_count(P, c, valid, a.st + it.scene);
 }
@@ -417,14 +418,14 @@ static bool scan_smem_ready()
 
 int launch_batch_neighbors_density(const BatchArgs& a, const float4* pos, const uint32_t* cell_start, int32_t* nbr,
                                    int32_t* count, float* rho, float* pres, const float4* vel, float4* vrho,
-                                   cudaStream_t s)
+                                   float4* xpf, cudaStream_t s)
 {
     if (!a.items_count) return 0;
     bool ok = false;
     LSP_BATCH_DISPATCH(a.threads, (ok = scan_smem_ready<T>()));
     if (!ok) return 0;
     LSP_BATCH_DISPATCH(a.threads, (kb_neighbors_density<T><<<a.items_count, T, scan_smem(T), s>>>(
-                                      a, pos, cell_start, nbr, count, rho, pres, vel, vrho)));
+                                      a, pos, cell_start, nbr, count, rho, pres, vel, vrho, xpf)));
     return 1;
 }
 

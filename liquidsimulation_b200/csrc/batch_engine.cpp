@@ -350,6 +350,7 @@ StepBuffers BatchEngine::buffers(int c)
     b.force = force_.p; b.rho = rho_.p; b.pres = pres_.p;
     b.ppos = ppos_.p; b.phalf = phalf_.p; b.pforce = pforce_.p; b.prho = prho_.p; b.err = err_.p;
     b.nbr = nbr_.p; b.nbr_count = nbr_count_.p; b.vrho = vrho_.p;
+    b.xpf = ppos_alt_.p;   // SPH has no predicted positions
     b.tables = tables_.p; b.colliders = dcols_.p; b.status = status_.p + sc_.size();
     b.hist = history_on() ? phist_[c].p : nullptr;
     b.gradrho = features_on() ? gradrho_.p : nullptr;
@@ -381,7 +382,7 @@ int BatchEngine::enqueue_step(int c, int grid)
     launches += launch_grid_order(g, stream_);
     StepBuffers b = buffers(1 - c);
     launches += launch_batch_neighbors_density(a, pos_[1 - c].p, cell_start_.p, nbr_.p, nbr_count_.p, rho_.p,
-                                               pres_.p, vel_[1 - c].p, vrho_.p, stream_);
+                                               pres_.p, vel_[1 - c].p, vrho_.p, pcisph_ ? nullptr : ppos_alt_.p, stream_);
     launches += launch_batch_nonpressure(a, b, stream_);
     if (pcisph_) {
         CK(cudaMemsetAsync(loop_sync_.p, 0, 4 * sizeof(uint32_t), stream_));

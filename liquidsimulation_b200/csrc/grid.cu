@@ -133,7 +133,8 @@ __global__ void k_neighbors_density(DevParams P, const float4* __restrict__ pos,
                                     const uint32_t* __restrict__ cell_start, int32_t* __restrict__ nbr,
                                     int32_t* __restrict__ count, DevStatus* st, const float* __restrict__ tables,
                                     float* __restrict__ rho, float* __restrict__ pres,
-                                    const float4* __restrict__ vel, float4* __restrict__ vrho)
+                                    const float4* __restrict__ vel, float4* __restrict__ vrho,
+                                    float4* __restrict__ xpf)
 {
     extern __shared__ uint2 masks[];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -142,7 +143,7 @@ __global__ void k_neighbors_density(DevParams P, const float4* __restrict__ pos,
     if (valid) {
         float sum;
         c = neighbors_one(P, pos, cell_start, nbr, i, tables, masks + threadIdx.x, blockDim.x, &sum);
-        store_density(P, i, c, sum, vel, count, rho, pres, vrho, st);
+        store_density(P, i, c, sum, pos, vel, count, rho, pres, vrho, xpf, st);
     }
     record_neighbor_count(P, c, valid, st);
 }
@@ -214,7 +215,7 @@ int launch_neighbors(const GridBuildArgs& a, cudaStream_t s)
     if (a.P.n <= 0) return 0;
     k_neighbors_density<<<blocks_for(a.P.n, T), T, scan_smem(T), s>>>(a.P, a.pos_out, a.cell_start, a.nbr,
                                                                       a.nbr_count, a.status, a.tables, a.rho, a.pres,
-                                                                      a.vel_out, a.vrho);
+                                                                      a.vel_out, a.vrho, a.xpf);
     return 1;
 }
 

@@ -261,35 +261,11 @@ __device__ __forceinline__ V3 group_nonpressure(const Group<L>& g, const DevPara
                : group_nonpressure_walk<L, false>(g, P, b, i, xi, vi, rhoi, list);
 }
 
-// The SPH pressure force of particle i (sph_pressure_one), in every lane.
-template <int L>
-__device__ __forceinline__ V3 group_sph_pressure(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i, V3 xi,
-                                                 float rhoi, float pres, const HeldList<L>& list)
-{
-    const float tf = pres / (rhoi * rhoi);
-    float sum[(3 + L - 1) / L];
-    group_walk<L, 3>(
-        g, list.cnt, list.most, list, [&](int j) { return SphRec{b.pos[j], b.rho[j], b.pres[j]}; },
-        [&](int j0, const SphRec& r0, int j1, const SphRec& r1, float (&t)[3][2]) {
-            auto one = [&](int j, const SphRec& r, int e) {
-                const V3 f = sph_pressure_term(P, b.tables, xi, tf, r);
-                t[0][e] = j != i ? f.x : 0.f, t[1][e] = j != i ? f.y : 0.f, t[2][e] = j != i ? f.z : 0.f;
-            };
-            one(j0, r0, 0);
-            one(j1, r1, 1);
-        },
-        sum);
-    V3 pf = v3(group_sum<L>(sum, 0), group_sum<L>(sum, 1), group_sum<L>(sum, 2));
-    pf *= -(P.mass * rhoi);
-    return pf;
-}
-
-// The PCISPH pressure force of particle i at predicted position xi with factor tf (pci_force_one),
-// in every lane.
+// The pressure force's sum over the pairs of particle i at predicted position xi with factor tf
+// (pci_force_walk), in every lane.
 template <int L, bool kExactDiv>
 __device__ __forceinline__ V3 group_pci_force_walk(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i,
-                                                   const float4* ppos, V3 xi, float tf, float rhoi,
-                                                   const HeldList<L>& list)
+                                                   const float4* ppos, V3 xi, float tf, const HeldList<L>& list)
 {
     float sum[(3 + L - 1) / L];
     group_walk<L, 3>(
@@ -308,15 +284,28 @@ __device__ __forceinline__ V3 group_pci_force_walk(const Group<L>& g, const DevP
             t[0][1] = j1 != i ? f1.x : 0.f, t[1][1] = j1 != i ? f1.y : 0.f, t[2][1] = j1 != i ? f1.z : 0.f;
         },
         sum);
-    return pci_pressure_force(P, rhoi, v3(group_sum<L>(sum, 0), group_sum<L>(sum, 1), group_sum<L>(sum, 2)));
+    return v3(group_sum<L>(sum, 0), group_sum<L>(sum, 1), group_sum<L>(sum, 2));
 }
 template <int L>
 __device__ __forceinline__ V3 group_pci_force(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i,
                                               const float4* ppos, V3 xi, float tf, float rhoi, const HeldList<L>& list)
 {
-    return *(const volatile uint32_t*)&b.status->div_unsafe == 0u
-               ? group_pci_force_walk<L, true>(g, P, b, i, ppos, xi, tf, rhoi, list)
-               : group_pci_force_walk<L, false>(g, P, b, i, ppos, xi, tf, rhoi, list);
+    return pci_pressure_force(P, rhoi,
+                              *(const volatile uint32_t*)&b.status->div_unsafe == 0u
+                                  ? group_pci_force_walk<L, true>(g, P, b, i, ppos, xi, tf, list)
+                                  : group_pci_force_walk<L, false>(g, P, b, i, ppos, xi, tf, list));
+}
+// The SPH pressure force of particle i (sph_pressure_one), in every lane.
+template <int L>
+__device__ __forceinline__ V3 group_sph_pressure(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i, V3 xi,
+                                                 float rhoi, const HeldList<L>& list)
+{
+    const float tf = b.xpf[i].w;
+    V3 pf = *(const volatile uint32_t*)&b.status->np_unsafe == 0u
+                ? group_pci_force_walk<L, true>(g, P, b, i, b.xpf, xi, tf, list)
+                : group_pci_force_walk<L, false>(g, P, b, i, b.xpf, xi, tf, list);
+    pf *= -(P.mass * rhoi);
+    return pf;
 }
 
 }  // namespace lsp

@@ -37,6 +37,7 @@ struct GridBuildArgs {
     float* rho;
     float* pres;
     float4* vrho;          // {v, rho} per particle for the non-pressure pass's gathers
+    float4* xpf;           // SPH: {x, p / rho^2} for the pressure pass's gathers, else null
 };
 
 struct MlpPacked;
@@ -73,6 +74,7 @@ struct StepBuffers {
     // {v.x, v.y, v.z, rho} of each particle, written by the neighbour build once rho is known:
     // the non-pressure pass gathers a neighbour's velocity and density with one 16-byte load.
     const float4* vrho;
+    const float4* xpf;        // SPH: {x, p / rho^2}, written by the neighbour build
     // tables (5 x 1001) and colliders
     const float* tables;
     const Collider* colliders;

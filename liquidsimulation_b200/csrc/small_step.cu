@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
         float sum;
         const int c = group_neighbors(own, P, b.pos, b.tables, g.cell_start, g.nbr, i, valid, list, &sum);
         const bool first = valid && own.lane == 0;
-        if (first) store_density(P, i, c, sum, b.vel, g.nbr_count, g.rho, g.pres, g.vrho, st);
+        if (first) store_density(P, i, c, sum, b.pos, b.vel, g.nbr_count, g.rho, g.pres, g.vrho, g.xpf, st);
         record_neighbor_count(P, c, first, st);
     }
     if (threadIdx.x == 0) block_max = 0u;
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
 
     if (!a.pcisph) {
         const float pres = b.pres[i];
-        F += group_sph_pressure(grp, P, b, i, x0, rho, pres, list);
+        F += group_sph_pressure(grp, P, b, i, x0, rho, list);
         if (!barrier()) return;   // the positions are read by other groups until here
         integrate(F, pres);
         if (tid == 0) *a.host = *st;
