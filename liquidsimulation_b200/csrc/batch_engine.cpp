@@ -136,7 +136,7 @@ void BatchEngine::build()
 {
     if (sc_.empty()) throw Error(LSP_ERR_STATE, "the batch has no scenes");
     activate();
-    int64_t cell_base = 0;
+    int64_t cell_base = 0, cells = 0;
     int coll_off = 0, max_it = 1;
     for (Scene& s : sc_) {
         float lo[3], hi[3];
@@ -170,12 +170,15 @@ void BatchEngine::build()
         }
         s.cells = grid_from_box(lo, hi, s.hk.h, s.org, s.dim);
         s.cell_base = cell_base;
-        cell_base += s.cells;
+        // Each scene's cell table has an end entry of its own and starts at a multiple of 8 entries,
+        // so that a scene's blocks can scan it alone.
+        cells += s.cells;
+        cell_base += scan_entries(s.cells + 1);
         s.coll_off = coll_off;
         coll_off += (int)s.cols.size();
         max_it = std::max(max_it, s.prm.pci_max_iterations);
     }
-    if (cell_base + 1 > ((int64_t)1 << 31)) throw Error(LSP_ERR_CAPACITY, "batch grid boxes hold more than 2^31 cells");
+    if (cells + 1 > ((int64_t)1 << 31)) throw Error(LSP_ERR_CAPACITY, "batch grid boxes hold more than 2^31 cells");
     cells_ = cell_base;
     mstride_ = max_it + 4;
     const int S = (int)sc_.size();
@@ -193,9 +196,7 @@ void BatchEngine::build()
     hist_.alloc(scan_entries(cells_ + 1));
     cell_start_.alloc(scan_entries(cells_ + 1));
     tile_sums_.alloc(scan_tiles(cells_ + 1) + 1);
-    loop_sync_.alloc(4);
-    maxerr_.alloc((size_t)S * mstride_);
-    status_.alloc(S + 1);
+    control_.alloc(control_words());
     dparams_.alloc(S);
     tables_.alloc((size_t)S * kSceneTableStride);
     dcols_.alloc(std::max(coll_off, 1));
@@ -242,6 +243,21 @@ void BatchEngine::build()
     ensure_neighbors(cap0);
     upload_colliders();
     build_items();
+    std::vector<int64_t> scene_n, scene_cells;
+    for (const Scene& s : sc_) {
+        scene_n.push_back(s.n);
+        scene_cells.push_back(s.cells);
+    }
+    std::vector<SmallBatchBlock> blocks;
+    small_lanes_ = small_batch_plan(scene_n, scene_cells, &blocks);
+    small_count_ = (int)blocks.size();
+    if (small_lanes_) {
+        if (tile_sums_.n < blocks.size()) tile_sums_.alloc(blocks.size());
+        small_blocks_.alloc(blocks.size());
+        CK(cudaMemcpyAsync(small_blocks_.p, blocks.data(), blocks.size() * sizeof(SmallBatchBlock), cudaMemcpyHostToDevice,
+                           stream_));
+        CK(cudaStreamSynchronize(stream_));
+    }
 }
 
 void BatchEngine::ensure_neighbors(int cap)
@@ -339,7 +355,7 @@ BatchArgs BatchEngine::args()
     a.items_count = items_count_;
     a.scenes = (int)sc_.size();
     a.threads = threads_;
-    a.st = status_.p;
+    a.st = status();
     return a;
 }
 
@@ -351,10 +367,49 @@ StepBuffers BatchEngine::buffers(int c)
     b.ppos = ppos_.p; b.phalf = phalf_.p; b.pforce = pforce_.p; b.prho = prho_.p; b.err = err_.p;
     b.nbr = nbr_.p; b.nbr_count = nbr_count_.p; b.vrho = vrho_.p;
     b.xpf = ppos_alt_.p;   // SPH has no predicted positions
-    b.tables = tables_.p; b.colliders = dcols_.p; b.status = status_.p + sc_.size();
+    b.tables = tables_.p; b.colliders = dcols_.p; b.status = status() + sc_.size();
     b.hist = history_on() ? phist_[c].p : nullptr;
     b.gradrho = features_on() ? gradrho_.p : nullptr;
     return b;
+}
+
+GridBuildArgs BatchEngine::grid_args(int c)
+{
+    const int S = (int)sc_.size();
+    GridBuildArgs g{};
+    g.P.n = (int)n_;
+    g.P.cells = (uint32_t)cells_;
+    g.pos_in = pos_[c].p; g.vel_in = vel_[c].p; g.half_in = half_[c].p; g.old_in = old_[c].p;
+    g.pos_out = pos_[1 - c].p; g.vel_out = vel_[1 - c].p; g.half_out = half_[1 - c].p; g.old_out = old_[1 - c].p;
+    g.key = key_.p; g.slot = slot_.p; g.hist = hist_.p; g.tile_sums = tile_sums_.p; g.cell_start = cell_start_.p;
+    g.tmp = tmp_.p; g.slot_of_id = slot_of_id_.p; g.sorted_key = sorted_key_.p;
+    g.hist_in = history_on() ? phist_[c].p : nullptr;
+    g.hist_out = history_on() ? phist_[1 - c].p : nullptr;
+    g.status = status() + S;
+    return g;
+}
+
+bool BatchEngine::enqueue_small(int c)
+{
+    SmallStepArgs a{};
+    a.g = grid_args(c);
+    a.g.nbr = nbr_.p; a.g.nbr_count = nbr_count_.p; a.g.rho = rho_.p; a.g.pres = pres_.p; a.g.vrho = vrho_.p;
+    a.g.xpf = pcisph_ ? nullptr : ppos_alt_.p;
+    a.b = buffers(1 - c);
+    a.b.status = status();
+    a.ppos_alt = ppos_alt_.p;
+    a.sync = loop_sync();
+    a.maxerr = maxerr();
+    a.host = hstatus_;
+    a.pcisph = pcisph_ ? 1 : 0;
+    SmallBatchArgs sb{};
+    sb.sp = dparams_.p;
+    sb.blocks = small_blocks_.p;
+    sb.mstride = mstride_;
+    sb.table_stride = kSceneTableStride;
+    if (launch_small_batch(a, sb, small_lanes_, small_count_, stream_)) return true;
+    cudaGetLastError();
+    return false;
 }
 
 // The step of every scene from buffer parity c into 1 - c (the grid build gathers the
@@ -365,34 +420,28 @@ int BatchEngine::enqueue_step(int c, int grid)
 {
     const int S = (int)sc_.size();
     int launches = 0;
-    CK(cudaMemsetAsync(status_.p, 0, (S + 1) * sizeof(DevStatus), stream_));
+    CK(cudaMemsetAsync(control_.p, 0, control_words() * sizeof(uint32_t), stream_));
+    if (one_launch()) {
+        if (enqueue_small(c)) return 1;
+        small_lanes_ = 0;   // refused by the device
+        grid = pcisph_ ? loop_grid() : 0;
+    }
     BatchArgs a = args();
     launches += launch_batch_keys(a, pos_[c].p, key_.p, slot_.p, hist_.p, stream_);
-    GridBuildArgs g{};
-    g.P.n = (int)n_;
-    g.P.cells = (uint32_t)cells_;
-    g.pos_in = pos_[c].p; g.vel_in = vel_[c].p; g.half_in = half_[c].p; g.old_in = old_[c].p;
-    g.pos_out = pos_[1 - c].p; g.vel_out = vel_[1 - c].p; g.half_out = half_[1 - c].p; g.old_out = old_[1 - c].p;
-    g.key = key_.p; g.slot = slot_.p; g.hist = hist_.p; g.tile_sums = tile_sums_.p; g.cell_start = cell_start_.p;
-    g.tmp = tmp_.p; g.slot_of_id = slot_of_id_.p; g.sorted_key = sorted_key_.p;
+    GridBuildArgs g = grid_args(c);
     const bool feats = features_on();
-    g.hist_in = history_on() ? phist_[c].p : nullptr;
-    g.hist_out = history_on() ? phist_[1 - c].p : nullptr;
-    g.status = status_.p + S;
     launches += launch_grid_order(g, stream_);
     StepBuffers b = buffers(1 - c);
     launches += launch_batch_neighbors_density(a, pos_[1 - c].p, cell_start_.p, nbr_.p, nbr_count_.p, rho_.p,
                                                pres_.p, vel_[1 - c].p, vrho_.p, pcisph_ ? nullptr : ppos_alt_.p, stream_);
     launches += launch_batch_nonpressure(a, b, stream_);
     if (pcisph_) {
-        CK(cudaMemsetAsync(loop_sync_.p, 0, 4 * sizeof(uint32_t), stream_));
-        CK(cudaMemsetAsync(maxerr_.p, 0, (size_t)S * mstride_ * sizeof(uint32_t), stream_));
         if (feats) {
             // Iteration 0 outside the persistent kernel: predict, then density with the
             // features and (warm start) the network's guess.
             BatchWarmArgs w{};
             w.feat = feat_.p;
-            w.maxerr = maxerr_.p;
+            w.maxerr = maxerr();
             w.mstride = mstride_;
             launches += launch_batch_pci_predict0(a, b, stream_);
             launches += launch_batch_density_first(a, b, w, stream_);
@@ -400,15 +449,15 @@ int BatchEngine::enqueue_step(int c, int grid)
                 // The network's guess on the tensor cores, one block per item (in
                 // LSP_WARM_AUTO only for the scenes switched on).
                 launch_batch_warm_guess_tc(mlp_.umma(), dparams_.p, items_.p, items_count_, b, feat_.p,
-                                           warm_ == LSP_WARM_AUTO ? warm_scene_.p : nullptr, status_.p + S,
+                                           warm_ == LSP_WARM_AUTO ? warm_scene_.p : nullptr, status() + S,
                                            stream_);
                 launches++;
             }
         }
         BatchLoopArgs l{};
         l.ppos_alt = ppos_alt_.p;
-        l.sync = loop_sync_.p;
-        l.maxerr = maxerr_.p;
+        l.sync = loop_sync();
+        l.maxerr = maxerr();
         l.mstride = mstride_;
         l.first_done = feats ? 1 : 0;
         l.warm = guess_on() ? 1 : 0;
@@ -421,7 +470,7 @@ int BatchEngine::enqueue_step(int c, int grid)
         launches += launch_batch_integrate(a, b, false, stream_);
     }
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(hstatus_, status_.p, (S + 1) * sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
+    CK(cudaMemcpyAsync(hstatus_, status(), (S + 1) * sizeof(DevStatus), cudaMemcpyDeviceToHost, stream_));
     return launches;
 }
 
@@ -429,7 +478,8 @@ void BatchEngine::run_once(int c)
 {
     activate();
     // Occupancy queries stay outside the stream capture.
-    const int grid = pcisph_ ? loop_grid() : 0;
+    const int grid = pcisph_ && !one_launch() ? loop_grid() : 0;
+    if (one_launch()) hstatus_[sc_.size()] = DevStatus{};   // the separate kernels' batch-wide entry
     if (use_graph_ && graph_ok_ && !graph_[c]) {
         cudaGraph_t g = nullptr;
         int l = 0;
@@ -552,6 +602,7 @@ void BatchEngine::set_launch(int use_graph, int threads, int loop_blocks)
     if (loop_blocks < 0) throw Error(LSP_ERR_INVALID, "loop_blocks must be >= 0");
     use_graph_ = use_graph != 0;
     loop_blocks_ = loop_blocks;
+    shaped_ = threads != 256 || loop_blocks != 0;
     if (threads != threads_) {
         threads_ = threads;
         if (built_) build_items();
@@ -565,6 +616,22 @@ void BatchEngine::get_launch(int* use_graph, int* threads, int* loop_blocks, int
     if (threads) *threads = threads_;
     if (loop_blocks) *loop_blocks = loop_blocks_;
     if (graph_active) *graph_active = (use_graph_ && graph_ok_ && (graph_[0] || graph_[1])) ? 1 : 0;
+}
+
+float BatchEngine::time_step(int repeats, cudaEvent_t e0, cudaEvent_t e1)
+{
+    run_checked();   // capture (and list growth, if the step needs it)
+    float best = std::numeric_limits<float>::infinity();
+    for (int r = 0; r < repeats; r++) {
+        CK(cudaEventRecord(e0, stream_));
+        run_once(cur_);
+        CK(cudaEventRecord(e1, stream_));
+        CK(cudaEventSynchronize(e1));
+        float ms = 0.f;
+        CK(cudaEventElapsedTime(&ms, e0, e1));
+        best = std::min(best, ms);
+    }
+    return best;
 }
 
 // Candidates: every supported block size, with the persistent kernel at full residency and
@@ -605,20 +672,15 @@ void BatchEngine::autotune(float dt, int repeats, lsp_batch_tuning* out, lsp_ste
     try {
         for (size_t k = 0; k < cands.size(); k++) {
             set_launch(graph ? 1 : 0, cands[k].threads, cands[k].blocks);
-            run_checked();   // capture (and list growth, if the step needs it)
-            float bestms = std::numeric_limits<float>::infinity();
-            for (int r = 0; r < repeats; r++) {
-                CK(cudaEventRecord(e0, stream_));
-                run_once(cur_);
-                CK(cudaEventRecord(e1, stream_));
-                CK(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                CK(cudaEventElapsedTime(&ms, e0, e1));
-                bestms = std::min(bestms, ms);
-            }
-            cands[k].ms = bestms;
-            if (bestms < cands[best].ms) best = k;
+            shaped_ = true;
+            cands[k].ms = time_step(repeats, e0, e1);
+            if (cands[k].ms < cands[best].ms) best = k;
         }
+        set_launch(graph ? 1 : 0, cands[best].threads, cands[best].blocks);
+        // A small batch's one-launch step has no shape: it stays when no shape is faster.
+        shaped_ = false;
+        shaped_ = !one_launch() || time_step(repeats, e0, e1) > cands[best].ms;
+        drop_graphs();
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -626,7 +688,6 @@ void BatchEngine::autotune(float dt, int repeats, lsp_batch_tuning* out, lsp_ste
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    set_launch(graph ? 1 : 0, cands[best].threads, cands[best].blocks);
     // The chosen shape runs the step once more; that run's results become the step.
     if (!run_checked()) {
         finish_step(stats);   // reports the persisting overflow

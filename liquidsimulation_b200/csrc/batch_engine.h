@@ -1,7 +1,7 @@
 // Host engine of a batch of independent scenes (lsp_batch_* in include/lsp.h): one set of
 // device arrays for all scenes, one stream, and a step that is one CUDA graph (grid build,
 // neighbour lists, density, non-pressure forces, the persistent PCISPH loop of every
-// scene, integration) per buffer parity.
+// scene, integration) per buffer parity. A small batch's step is one kernel (small_step.cu).
 #pragma once
 
 #include <cstdint>
@@ -9,6 +9,7 @@
 
 #include "batch_kernels.h"
 #include "engine.h"
+#include "small_step.h"
 
 namespace lsp {
 
@@ -84,6 +85,13 @@ private:
     void drop_graphs();
     int loop_grid() const;
     int enqueue_step(int c, int grid);   // returns the number of kernels launched
+    // Whether the step runs as one launch (small_step.cu): the batch is small enough, no features
+    // are computed and no other launch shape was asked for.
+    bool one_launch() const { return small_lanes_ && !features_on() && !shaped_; }
+    bool enqueue_small(int c);
+    GridBuildArgs grid_args(int c);
+    // Shortest of `repeats` runs of the pending step, ms (e0, e1: events to time it with).
+    float time_step(int repeats, cudaEvent_t e0, cudaEvent_t e1);
     void run_once(int c);           // one step attempt from buffer parity c (graph or direct)
     // Runs the step from parity cur_ until no list overflows; false if it still overflowed.
     bool run_checked();
@@ -116,7 +124,7 @@ private:
     DevArray<float4> force_, ppos_, ppos_alt_, phalf_, pforce_;
     DevArray<float> rho_, pres_, prho_, err_;
     DevArray<float4> vrho_;   // {v, rho} for the non-pressure pass (StepBuffers::vrho)
-    DevArray<uint32_t> key_, slot_, sorted_key_, hist_, cell_start_, tile_sums_, loop_sync_, maxerr_;
+    DevArray<uint32_t> key_, slot_, sorted_key_, hist_, cell_start_, tile_sums_;
     DevArray<int2> tmp_;
     DevArray<int32_t> slot_of_id_, nbr_, nbr_count_;
     DevArray<float> tables_, stage_;
@@ -124,7 +132,15 @@ private:
     DevArray<Collider> dcols_;
     DevArray<DevParams> dparams_;
     DevArray<BatchItem> items_;
-    DevArray<DevStatus> status_;
+    // What a step clears at its start, in one block: barrier words [scenes][4], maxima
+    // [scenes][mstride_], status [scenes + 1].
+    DevArray<uint32_t> control_;
+    size_t control_words() const { return sc_.size() * (4 + (size_t)mstride_) + (sc_.size() + 1) * sizeof(DevStatus) / 4; }
+    uint32_t* loop_sync() { return control_.p; }
+    uint32_t* maxerr() { return control_.p + 4 * sc_.size(); }
+    DevStatus* status() { return reinterpret_cast<DevStatus*>(control_.p + sc_.size() * (4 + (size_t)mstride_)); }
+    DevArray<SmallBatchBlock> small_blocks_;
+    int small_lanes_ = 0, small_count_ = 0;   // of the one-launch step; 0: the batch is too large for it
     DevParams* hparams_ = nullptr;   // pinned
     DevStatus* hstatus_ = nullptr;   // pinned
     int items_count_ = 0;
@@ -132,6 +148,7 @@ private:
     int64_t nbr_stride_ = 0;
 
     int threads_ = 256, loop_blocks_ = 0;
+    bool shaped_ = false;   // a launch shape of the separate kernels was chosen
     bool use_graph_ = true, graph_ok_ = true;
     cudaGraphExec_t graph_[2] = {nullptr, nullptr};
     int graph_launches_[2] = {0, 0};

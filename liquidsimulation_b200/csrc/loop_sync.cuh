@@ -49,16 +49,16 @@ static __device__ __forceinline__ bool barrier_wait(LoopSync* sy, DevStatus* st,
     return ld_volatile(&sy->abort) == 0u;
 }
 
-// Returns false when the loop must stop (a barrier gave up somewhere). The arrival counter
-// only grows during a launch (the host clears it before each one): the e-th barrier of a launch
-// is over when the counter reaches e times the grid size, so one reduction per block and barrier
-// is all the traffic; epoch counts the barriers this block has passed. The arrival releases and
-// the last poll acquires at device scope; block barriers on both sides carry that to the other
-// threads.
-static __device__ bool grid_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch)
+// Barrier of the `blocks` blocks that share sy. Returns false when the loop must stop (a barrier
+// gave up somewhere). The arrival counter only grows during a launch (the host clears it before each
+// one): the e-th barrier of a launch is over when the counter reaches e times the number of blocks,
+// so one reduction per block and barrier is all the traffic; epoch counts the barriers this block
+// has passed. The arrival releases and the last poll acquires at device scope; block barriers on
+// both sides carry that to the other threads.
+static __device__ bool blocks_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch, uint32_t blocks)
 {
     __shared__ int ok;
-    const uint32_t target = ++epoch * gridDim.x;
+    const uint32_t target = ++epoch * blocks;
     __syncthreads();
     if (threadIdx.x == 0) {
         add_release(&sy->count);
@@ -66,6 +66,11 @@ static __device__ bool grid_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch
     }
     __syncthreads();
     return ok != 0;
+}
+
+static __device__ __forceinline__ bool grid_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch)
+{
+    return blocks_barrier(sy, st, epoch, gridDim.x);
 }
 
 }  // namespace lsp

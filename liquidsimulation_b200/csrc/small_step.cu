@@ -1,4 +1,4 @@
-// The whole step of a small scene in one cooperative launch: grid build, neighbour lists,
+// The whole step of a small scene, or of a batch of small scenes, in one cooperative launch: grid build, neighbour lists,
 // non-pressure forces, the pressure (SPH force or the PCISPH loop) and the integration, separated
 // by grid barriers, with a group of L lanes per particle where a neighbour list is walked
 // (group_ops.cuh). Each result carries the bits of the separate kernels (grid.cu, sph.cu,
@@ -30,6 +30,9 @@ namespace lsp {
 
 // 512 threads per SM leave each 128 registers: the groups keep their particle's list and state there.
 constexpr int kMaxThreads = 512;
+// A batch's blocks: small, so that a scene's last one wastes little. 16 scenes, 20,071 particles, four
+// steps with their transfers: 464 us with 128 threads, 475 with 256, 495 with 64.
+constexpr int kBatchThreads = 128;
 // Shared memory of a group in the build: one row of terms and the list.
 template <int L>
 constexpr int build_words()
@@ -37,25 +40,36 @@ constexpr int build_words()
     return group_pitch(L) + kGroupList;
 }
 
-template <int L>
-__global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
+// The blocks of one scene: this block's place among them, and what they share.
+struct SceneBlocks {
+    int block, blocks;
+    LoopSync* sync;
+    uint32_t* maxerr;
+    uint32_t* tile_sums;
+    DevStatus* host;
+};
+
+// The step of one scene by its blocks. kBatch: the scene's particles start at slot P.base and its
+// cells at P.cell_base, a multiple of 8.
+template <int L, bool kBatch>
+__device__ __forceinline__ void small_step(const DevParams& P, const GridBuildArgs& g, const StepBuffers& b, float4* ppos_alt,
+                                           int pcisph, const SceneBlocks& own_blocks)
 {
     extern __shared__ float4 dyn[];   // the groups' terms; in the build also their lists
     __shared__ uint32_t ws[32];
     __shared__ Collider cols[kMaxColliders];
     __shared__ uint32_t block_max;
-    const GridBuildArgs& g = a.g;
-    const StepBuffers& b = a.b;
-    const DevParams& P = g.P;
     DevStatus* st = b.status;
-    LoopSync* sy = reinterpret_cast<LoopSync*>(a.sync);
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int block = own_blocks.block, blocks = own_blocks.blocks;
+    uint32_t* const maxerr = own_blocks.maxerr;
+    const int tid = block * blockDim.x + threadIdx.x;
     const int n = P.n;
+    const int base = kBatch ? P.base : 0;
     uint32_t epoch = 0;
     // A barrier that gave up tells the host at once: the status copy at the end is not reached.
     auto barrier = [&]() {
-        const bool ok = grid_barrier(sy, st, epoch);
-        if (!ok && threadIdx.x == 0) a.host->error_flags = kErrTimeout;
+        const bool ok = blocks_barrier(own_blocks.sync, st, epoch, (uint32_t)blocks);
+        if (!ok && threadIdx.x == 0) own_blocks.host->error_flags = kErrTimeout;
         return ok;
     };
     for (int w = threadIdx.x; w < P.ncoll * (int)(sizeof(Collider) / 4); w += blockDim.x)
@@ -67,43 +81,46 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
     float4 x4 = make_float4(0.f, 0.f, 0.f, 0.f);
     bool escaped = false, bad = false;
     if (mine) {
-        x4 = __ldg(g.pos_in + tid);
+        x4 = __ldg(g.pos_in + base + tid);
         key = cell_key(P, x4, escaped, bad);
     }
     const uint32_t slot = hist_slot(key, mine, g.hist);
     record_key_flags(mine, escaped, bad, st);
     if (!barrier()) return;
 
-    // ---- scan: each block owns a contiguous run of cells
+    // ---- scan: each block owns a contiguous run of the scene's cells
+    uint32_t* const hist = kBatch ? g.hist + P.cell_base : g.hist;
+    uint32_t* const cell_start = kBatch ? g.cell_start + P.cell_base : g.cell_start;
     const int64_t n8 = scan_entries((int64_t)P.cells + 1);
-    const int64_t per = (n8 / kScanItems + gridDim.x - 1) / gridDim.x * kScanItems;
-    const int64_t c0 = min((int64_t)blockIdx.x * per, n8), c1 = min(c0 + per, n8);
+    const int64_t per = (n8 / kScanItems + blocks - 1) / blocks * kScanItems;
+    const int64_t c0 = min((int64_t)block * per, n8), c1 = min(c0 + per, n8);
     {
         uint32_t s = 0;
         for (int64_t e = c0 + (int64_t)threadIdx.x * kScanItems; e < c1; e += (int64_t)blockDim.x * kScanItems) {
             uint32_t v[kScanItems];
-            load8(g.hist + e, v);
+            load8(hist + e, v);
 #pragma unroll
             for (int j = 0; j < kScanItems; j++) s += v[j];
         }
         uint32_t total;
         block_exclusive_scan(s, ws, &total);
-        if (threadIdx.x == 0) g.tile_sums[blockIdx.x] = total;
+        if (threadIdx.x == 0) own_blocks.tile_sums[block] = total;
     }
     if (!barrier()) return;
     {
         uint32_t s = 0, carry;
-        for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) s += __ldcg(g.tile_sums + k);
+        for (int k = threadIdx.x; k < block; k += blockDim.x) s += __ldcg(own_blocks.tile_sums + k);
         block_exclusive_scan(s, ws, &carry);
+        carry += (uint32_t)base;
         for (int64_t e0 = c0; e0 < c1; e0 += (int64_t)blockDim.x * kScanItems) {
             const int64_t e = e0 + (int64_t)threadIdx.x * kScanItems;
             uint32_t v[kScanItems] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (e < c1) load8(g.hist + e, v);
+            if (e < c1) load8(hist + e, v);
             uint32_t sum = 0, total;
 #pragma unroll
             for (int j = 0; j < kScanItems; j++) sum += v[j];
             const uint32_t ex = block_exclusive_scan(sum, ws, &total) + carry;
-            if (e < c1) store8_scan(g.cell_start + e, g.hist + e, v, ex);
+            if (e < c1) store8_scan(cell_start + e, hist + e, v, ex);
             carry += total;
         }
     }
@@ -115,11 +132,12 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
     if (mine) {
         beg = __ldcg(g.cell_start + key);
         end = __ldcg(g.cell_start + key + 1);
-        g.tmp[beg + slot] = make_int2(tid, id_of(x4));
+        g.tmp[beg + slot] = make_int2(base + tid, id_of(x4));
     }
     if (!barrier()) return;
     if (mine) {
-        const float4 v4 = __ldg(g.vel_in + tid), h4 = __ldg(g.half_in + tid), o4 = __ldg(g.old_in + tid);
+        const int from = base + tid;
+        const float4 v4 = __ldg(g.vel_in + from), h4 = __ldg(g.half_in + from), o4 = __ldg(g.old_in + from);
         const int id = id_of(x4);
         uint32_t rank = 0;
         if (end - beg <= (uint32_t)kMaxCellOccupancy) {
@@ -130,13 +148,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
         }
         const uint32_t dest = beg + rank;
         store_sorted(g, dest, id, key, x4, v4, h4, o4);
-        if (g.hist_out) g.hist_out[dest] = __ldg(g.hist_in + tid);
+        if (g.hist_out) g.hist_out[dest] = __ldg(g.hist_in + from);
     }
     if (!barrier()) return;
 
     // ---- neighbour lists, density, pressure (k_neighbors_density); from here a group holds
     // sorted particle i
-    const int i = min(tid / L, n - 1);
+    const int i = base + min(tid / L, n - 1);
     const bool valid = tid / L < n;
     {
         Group<L> own(reinterpret_cast<float*>(dyn));
@@ -175,18 +193,18 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
         }
     };
 
-    if (!a.pcisph) {
+    if (!pcisph) {
         const float pres = b.pres[i];
         F += group_sph_pressure(grp, P, b, i, x0, rho, list);
         if (!barrier()) return;   // the positions are read by other groups until here
         integrate(F, pres);
-        if (tid == 0) *a.host = *st;
+        if (tid == 0) *own_blocks.host = *st;
         return;
     }
 
     // ---- PCISPH: the loop of k_pci_loop from zero pressure. All lanes follow the particle's
     // predicted state.
-    auto pp = [&](int parity) { return parity ? a.ppos_alt : b.ppos; };
+    auto pp = [&](int parity) { return parity ? ppos_alt : b.ppos; };
     V3 px, ph;
     predict_motion(P, cols, st, F, v3(0.f, 0.f, 0.f), rho, x0, v, v4.w, half0, px, ph);
     if (lead) pp(0)[i] = f4(px, 0.f);
@@ -204,11 +222,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
         if ((threadIdx.x & 31) == 0 && mb) atomicMax(&block_max, mb);
         __syncthreads();
         if (threadIdx.x == 0) {
-            if (block_max) atomicMax(&a.maxerr[k], block_max);
+            if (block_max) atomicMax(&maxerr[k], block_max);
             block_max = 0u;
         }
         if (!barrier()) return;
-        const uint32_t me = ld_volatile(&a.maxerr[k]);
+        const uint32_t me = ld_volatile(&maxerr[k]);
         // PCISPHSolver.cpp:152-162: ratio = max|e| / rho0 in float, exit when below eta.
         const bool conv = fabsf(__uint_as_float(me) / P.rho0) < P.eta;
         const bool done = (conv && k + 1 >= P.min_it) || k + 1 >= P.max_it;
@@ -229,7 +247,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
                 st->max_err_bits = me;
                 st->warm_used = 0;
                 st->last_k = k;
-                *a.host = *st;
+                *own_blocks.host = *st;
             }
             return;
         }
@@ -237,6 +255,35 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
         if (lead) pp((k + 1) & 1)[i] = f4(px, 0.f);
         if (!barrier()) return;
     }
+}
+
+template <int L>
+__global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
+{
+    small_step<L, false>(a.g.P, a.g, a.b, a.ppos_alt, a.pcisph,
+                         {(int)blockIdx.x, (int)gridDim.x, reinterpret_cast<LoopSync*>(a.sync), a.maxerr, a.g.tile_sums, a.host});
+}
+
+// The same for a batch of scenes in one launch. A scene has blocks and a barrier of its own, so it
+// takes its iterations without waiting for the others. Four steps of 16 scenes (20,071 particles)
+// with their transfers: 650 us as separate kernels over all scenes, whose loop runs in lockstep
+// rounds with one thread per particle; 464 us here.
+template <int L>
+__global__ void __launch_bounds__(kBatchThreads, kMaxThreads / kBatchThreads) k_small_batch(SmallStepArgs a, SmallBatchArgs sb)
+{
+    __shared__ DevParams P;
+    const SmallBatchBlock me = sb.blocks[blockIdx.x];
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(sb.sp + me.scene);
+    for (int w = threadIdx.x; w < (int)(sizeof(DevParams) / 4); w += blockDim.x) reinterpret_cast<uint32_t*>(&P)[w] = from[w];
+    __syncthreads();
+    GridBuildArgs g = a.g;
+    StepBuffers b = a.b;
+    b.status += me.scene;
+    g.status = b.status;
+    b.tables += (size_t)me.scene * sb.table_stride;
+    small_step<L, true>(P, g, b, a.ppos_alt, a.pcisph,
+                        {(int)blockIdx.x - me.first, me.count, reinterpret_cast<LoopSync*>(a.sync) + me.scene,
+                         a.maxerr + (size_t)me.scene * sb.mstride, g.tile_sums + me.first, a.host + me.scene});
 }
 
 // ------------------------------------------------------------------ launch
@@ -262,6 +309,9 @@ static size_t step_smem(int choice, int threads)
 // different host threads may launch at once).
 static bool g_fits[kMaxDevices][kLaneChoices], g_ready[kMaxDevices];
 static std::mutex g_mutex;
+
+// A scene's blocks scan its cells; a block's share of a single scene's largest box.
+constexpr int64_t kBatchBlockCells = kSmallStepCells / 128;
 
 // As many lanes per particle as the threads allow: fewer lanes take longer walks (12,000 particles:
 // 93 us a step with 4 lanes). Beyond two lanes per particle the separate kernels, with one thread
@@ -312,6 +362,59 @@ bool launch_small_step(const SmallStepArgs& a, int lanes, cudaStream_t s)
     void* args[] = {&ac};
     return cudaLaunchCooperativeKernel(g_kernel[c], dim3(grid), dim3(block), args, step_smem(c, block), s) ==
            cudaSuccess;
+}
+
+static const void* const g_batch_kernel[kLaneChoices] = {(const void*)k_small_batch<16>, (const void*)k_small_batch<8>,
+                                                         (const void*)k_small_batch<4>, (const void*)k_small_batch<2>};
+
+// Resident blocks of a choice's batch kernel on the current device, 0 when it cannot run.
+static int64_t batch_block_limit(int c)
+{
+    int dev = 0, coop = 0, per = 0;
+    const size_t smem = step_smem(c, kBatchThreads);
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        !coop ||
+        cudaFuncSetAttribute(g_batch_kernel[c], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, g_batch_kernel[c], kBatchThreads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (int64_t)per * device_sm_count();
+}
+
+// The rule of small_step_lanes for all scenes together, in whole blocks. A PCISPH step, separate
+// kernels -> one launch: 4 scenes of 250 particles 99 -> 52 us, 48 of 71 104 -> 58, 16 of 500
+// 113 -> 103, 16 of 1,040 115 -> 79, 16 of 2,070 116 -> 96, 2 of 17,400 122 -> 106 us.
+int small_batch_plan(const std::vector<int64_t>& n, const std::vector<int64_t>& cells, std::vector<SmallBatchBlock>* blocks)
+{
+    blocks->clear();
+    for (int c = 0; c < kLaneChoices; c++) {
+        const int64_t lanes = 16 >> c;
+        int64_t total = 0;
+        bool fits = true;
+        for (size_t s = 0; s < n.size() && fits; s++) {
+            const int64_t count = (n[s] * lanes + kBatchThreads - 1) / kBatchThreads;
+            total += count;
+            fits = n[s] > 0 && cells[s] <= count * kBatchBlockCells;
+        }
+        if (!fits || total > (int64_t)device_sm_count() * (kMaxThreads / kBatchThreads) || total > batch_block_limit(c)) continue;
+        for (size_t s = 0; s < n.size(); s++) {
+            const int count = (int)((n[s] * lanes + kBatchThreads - 1) / kBatchThreads), first = (int)blocks->size();
+            for (int q = 0; q < count; q++) blocks->push_back({(int)s, first, count, 0});
+        }
+        return (int)lanes;
+    }
+    return 0;
+}
+
+bool launch_small_batch(const SmallStepArgs& a, const SmallBatchArgs& sb, int lanes, int blocks, cudaStream_t s)
+{
+    const int c = lanes == 16 ? 0 : lanes == 8 ? 1 : lanes == 4 ? 2 : 3;
+    SmallStepArgs ac = a;
+    SmallBatchArgs bc = sb;
+    void* args[] = {&ac, &bc};
+    return cudaLaunchCooperativeKernel(g_batch_kernel[c], dim3(blocks), dim3(kBatchThreads), args,
+                                       step_smem(c, kBatchThreads), s) == cudaSuccess;
 }
 
 }  // namespace lsp

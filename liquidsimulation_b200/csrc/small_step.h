@@ -1,6 +1,8 @@
 // Launch interface of the one-launch step of small scenes (small_step.cu).
 #pragma once
 
+#include <vector>
+
 #include "lsp_kernels.h"
 
 namespace lsp {
@@ -26,5 +28,24 @@ constexpr int kSmallStepTiles = 1024;
 int small_step_lanes(int64_t n, int64_t cells);
 // False when the device refuses the launch (the caller then runs the separate kernels).
 bool launch_small_step(const SmallStepArgs& a, int lanes, cudaStream_t s);
+
+// The one-launch step of a batch: block q of the launch belongs to blocks[q].scene, whose blocks are
+// [first, first + count).
+struct SmallBatchBlock {
+    int scene, first, count, pad;
+};
+struct SmallBatchArgs {
+    const DevParams* sp;             // [scenes]
+    const SmallBatchBlock* blocks;   // device
+    int mstride;                     // words of maxerr per scene
+    int table_stride;                // floats of tables per scene
+};
+
+// Lanes per particle of a batch's one-launch step, and its blocks; 0 (and no blocks) when the
+// separate kernels are used. n, cells: particles and grid cells of each scene.
+int small_batch_plan(const std::vector<int64_t>& n, const std::vector<int64_t>& cells, std::vector<SmallBatchBlock>* blocks);
+// a: b.status and host hold an entry per scene, sync 16 zeroed bytes per scene, g.tile_sums a word
+// per block. False when the device refuses the launch.
+bool launch_small_batch(const SmallStepArgs& a, const SmallBatchArgs& sb, int lanes, int blocks, cudaStream_t s);
 
 }  // namespace lsp
