@@ -20,6 +20,7 @@
 //                 the 64-byte persistent state into the new order
 //   k_neighbors_density  the start-of-step neighbour lists, reference order, with the density
 //                 and pressure summed over the accepted pairs
+#include "chained.cuh"
 #include "lsp_kernels.h"
 #include "particle_ops.cuh"
 #include "scan_ops.cuh"
@@ -32,7 +33,7 @@ constexpr int kScanTile = kScanThreads * kScanItems;
 __global__ void k_keys_hist(DevParams P, const float4* __restrict__ pos, uint32_t* __restrict__ key,
                             uint32_t* __restrict__ slot, uint32_t* __restrict__ hist, DevStatus* st)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     const bool valid = i < P.n;
     uint32_t k = 0xffffffffu;
     bool escaped = false, bad = false;
@@ -49,7 +50,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const uint32_t* __r
                                                              uint32_t* __restrict__ tile_sums)
 {
     __shared__ uint32_t ws[32];
-    const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+    const int64_t base = (int64_t)chained(blockIdx.x * kScanThreads + threadIdx.x) * kScanItems;
     uint32_t s = 0;
     if (base < n8) {
         uint32_t v[kScanItems];
@@ -68,8 +69,9 @@ __global__ void __launch_bounds__(1024) k_scan_top(uint32_t* tile_sums, int tile
 {
     __shared__ uint32_t ws[32];
     uint32_t carry = 0;
+    const int t = chained((int)threadIdx.x);
     for (int b = 0; b < tiles; b += blockDim.x) {
-        int i = b + threadIdx.x;
+        int i = b + t;
         uint32_t v = i < tiles ? tile_sums[i] : 0u;
         uint32_t total;
         uint32_t ex = block_exclusive_scan(v, ws, &total);
@@ -88,15 +90,17 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(uint32_t* __restric
                                                              uint32_t* __restrict__ out)
 {
     __shared__ uint32_t ws[32];
+    const int g = chained((int)(blockIdx.x * kScanThreads + threadIdx.x));
+    const int tile = g / kScanThreads;
     uint32_t prefix;
     if (fold) {
         uint32_t s = 0;
-        for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) s += tile_sums[k];
+        for (int k = g % kScanThreads; k < tile; k += kScanThreads) s += tile_sums[k];
         block_exclusive_scan(s, ws, &prefix);
     } else {
-        prefix = tile_sums[blockIdx.x];
+        prefix = tile_sums[tile];
     }
-    const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+    const int64_t base = (int64_t)g * kScanItems;
     uint32_t v[kScanItems] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (base < n8) load8(hist + base, v);
     uint32_t s = 0;
@@ -110,7 +114,7 @@ __global__ void k_scatter(DevParams P, const float4* __restrict__ pos, const uin
                           const uint32_t* __restrict__ slot, const uint32_t* __restrict__ cell_start,
                           int2* __restrict__ tmp)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     if (i >= P.n) return;
     uint32_t k = key[i];
     tmp[cell_start[k] + slot[i]] = make_int2(i, id_of(pos[i]));
@@ -119,7 +123,7 @@ __global__ void k_scatter(DevParams P, const float4* __restrict__ pos, const uin
 // rank_gather_one (particle_ops.cuh) for every sorted slot.
 __global__ void k_rank_gather(GridBuildArgs g)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const int p = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     if (p < g.P.n) rank_gather_one(g, p);
 }
 
@@ -137,7 +141,7 @@ __global__ void k_neighbors_density(DevParams P, const float4* __restrict__ pos,
                                     float4* __restrict__ xpf)
 {
     extern __shared__ uint2 masks[];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     const bool valid = i < P.n;
     int c = 0;
     if (valid) {
@@ -155,7 +159,7 @@ static inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t -
 int launch_grid_keys(const GridBuildArgs& a, cudaStream_t s)
 {
     if (a.P.n <= 0) return 0;
-    k_keys_hist<<<blocks_for(a.P.n, 256), 256, 0, s>>>(a.P, a.pos_in, a.key, a.slot, a.hist, a.status);
+    launch_chained(k_keys_hist, blocks_for(a.P.n, 256), 256, 0, s, a.P, a.pos_in, a.key, a.slot, a.hist, a.status);
     return 1;
 }
 
@@ -163,24 +167,24 @@ int launch_grid_scan(const GridBuildArgs& a, cudaStream_t s)
 {
     const int64_t n8 = scan_entries((int64_t)a.P.cells + 1);
     const int tiles = (int)scan_tiles((int64_t)a.P.cells + 1);
-    k_scan_tiles<<<tiles, kScanThreads, 0, s>>>(a.hist, n8, a.tile_sums);
+    launch_chained(k_scan_tiles, tiles, kScanThreads, 0, s, a.hist, n8, a.tile_sums);
     const int fold = tiles <= kFoldTiles ? 1 : 0;
-    if (!fold) k_scan_top<<<1, 1024, 0, s>>>(a.tile_sums, tiles);
-    k_scan_apply<<<tiles, kScanThreads, 0, s>>>(a.hist, n8, a.tile_sums, fold, a.cell_start);
+    if (!fold) launch_chained(k_scan_top, 1, 1024, 0, s, a.tile_sums, tiles);
+    launch_chained(k_scan_apply, tiles, kScanThreads, 0, s, a.hist, n8, a.tile_sums, fold, a.cell_start);
     return fold ? 2 : 3;
 }
 
 int launch_grid_scatter(const GridBuildArgs& a, cudaStream_t s)
 {
     if (a.P.n <= 0) return 0;
-    k_scatter<<<blocks_for(a.P.n, 256), 256, 0, s>>>(a.P, a.pos_in, a.key, a.slot, a.cell_start, a.tmp);
+    launch_chained(k_scatter, blocks_for(a.P.n, 256), 256, 0, s, a.P, a.pos_in, a.key, a.slot, a.cell_start, a.tmp);
     return 1;
 }
 
 int launch_grid_gather(const GridBuildArgs& a, cudaStream_t s)
 {
     if (a.P.n <= 0) return 0;
-    k_rank_gather<<<blocks_for(a.P.n, 256), 256, 0, s>>>(a);
+    launch_chained(k_rank_gather, blocks_for(a.P.n, 256), 256, 0, s, a);
     return 1;
 }
 
@@ -190,8 +194,8 @@ int launch_grid_order(const GridBuildArgs& a, cudaStream_t s)
     const DevParams& P = a.P;
     int launches = launch_grid_scan(a, s);
     if (P.n > 0) {
-        k_scatter<<<blocks_for(P.n, T), T, 0, s>>>(P, a.pos_in, a.key, a.slot, a.cell_start, a.tmp);
-        k_rank_gather<<<blocks_for(P.n, T), T, 0, s>>>(a);
+        launch_chained(k_scatter, blocks_for(P.n, T), T, 0, s, P, a.pos_in, a.key, a.slot, a.cell_start, a.tmp);
+        launch_chained(k_rank_gather, blocks_for(P.n, T), T, 0, s, a);
         launches += 2;
     }
     return launches;
@@ -203,7 +207,7 @@ int launch_grid_sort(const GridBuildArgs& a, cudaStream_t s)
     const DevParams& P = a.P;
     int launches = 0;
     if (P.n > 0) {
-        k_keys_hist<<<blocks_for(P.n, T), T, 0, s>>>(P, a.pos_in, a.key, a.slot, a.hist, a.status);
+        launch_chained(k_keys_hist, blocks_for(P.n, T), T, 0, s, P, a.pos_in, a.key, a.slot, a.hist, a.status);
         launches++;
     }
     return launches + launch_grid_order(a, s);
@@ -213,7 +217,7 @@ int launch_neighbors(const GridBuildArgs& a, cudaStream_t s)
 {
     const int T = 256;
     if (a.P.n <= 0) return 0;
-    k_neighbors_density<<<blocks_for(a.P.n, T), T, scan_smem(T), s>>>(a.P, a.pos_out, a.cell_start, a.nbr,
+    launch_chained(k_neighbors_density, blocks_for(a.P.n, T), T, scan_smem(T), s, a.P, a.pos_out, a.cell_start, a.nbr,
                                                                       a.nbr_count, a.status, a.tables, a.rho, a.pres,
                                                                       a.vel_out, a.vrho, a.xpf);
     return 1;

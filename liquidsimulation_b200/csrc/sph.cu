@@ -4,6 +4,7 @@
 //
 // Thread per particle; each thread walks its own neighbour list in the reference's
 // order, so its sums round exactly as the reference CPU solver's do.
+#include "chained.cuh"
 #include "lsp_device.cuh"
 #include "lsp_kernels.h"
 #include "particle_ops.cuh"
@@ -19,14 +20,14 @@ constexpr int kThreads = 256;
 template <bool kGrad>
 __global__ void __launch_bounds__(kThreads) k_nonpressure(DevParams P, StepBuffers b)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     if (i < P.n) nonpressure_one<kGrad>(P, b, i);
 }
 
 // SPHSolver::accumulatePressureForces, CPU branch (SPHSolver.cpp:268-290).
 __global__ void __launch_bounds__(kThreads) k_sph_pressure(DevParams P, StepBuffers b)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     if (i >= P.n) return;
     sph_pressure_one(P, b, i);
 }
@@ -36,7 +37,7 @@ __global__ void __launch_bounds__(kThreads) k_sph_pressure(DevParams P, StepBuff
 // added first (PCISPHSolver.cpp:166-169).
 __global__ void __launch_bounds__(kThreads) k_integrate_collide(DevParams P, StepBuffers b, int add_pforce)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     if (i >= P.n) return;
     integrate_one(P, b, i, add_pforce);
 }
@@ -47,17 +48,17 @@ void launch_nonpressure(const DevParams& P, const StepBuffers& b, cudaStream_t s
 {
     if (!P.n) return;
     if (b.gradrho)
-        k_nonpressure<true><<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, b);
+        launch_chained(k_nonpressure<true>, blocks_for(P.n, kThreads), kThreads, 0, s, P, b);
     else
-        k_nonpressure<false><<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, b);
+        launch_chained(k_nonpressure<false>, blocks_for(P.n, kThreads), kThreads, 0, s, P, b);
 }
 void launch_sph_pressure(const DevParams& P, const StepBuffers& b, cudaStream_t s)
 {
-    if (P.n) k_sph_pressure<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, b);
+    if (P.n) launch_chained(k_sph_pressure, blocks_for(P.n, kThreads), kThreads, 0, s, P, b);
 }
 void launch_integrate_collide(const DevParams& P, const StepBuffers& b, bool add_pforce, cudaStream_t s)
 {
-    if (P.n) k_integrate_collide<<<blocks_for(P.n, kThreads), kThreads, 0, s>>>(P, b, add_pforce ? 1 : 0);
+    if (P.n) launch_chained(k_integrate_collide, blocks_for(P.n, kThreads), kThreads, 0, s, P, b, add_pforce ? 1 : 0);
 }
 
 }  // namespace lsp
