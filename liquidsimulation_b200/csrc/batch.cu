@@ -83,10 +83,11 @@ __global__ void __launch_bounds__(T) kb_neighbors_density(BatchArgs a, const flo
     extern __shared__ uint2 masks[];
     const int i = it.begin + (int)threadIdx.x;
     const bool valid = i < it.end;
-    int c = 0;
+    float* stage = reinterpret_cast<float*>(masks + T * kScanChunks) + (threadIdx.x >> 5) * kStageFloats;
+    float sum;
+    const int c = neighbors_one<true>(P, pos, cell_start, nbr, min(i, it.end - 1), scene_tables(a, it.scene),
+                                      masks + threadIdx.x, T, &sum, stage, valid);
     if (valid) {
-        float sum;
-        c = neighbors_one(P, pos, cell_start, nbr, i, scene_tables(a, it.scene), masks + threadIdx.x, T, &sum);
         // The range check of the density is batch-wide, like the rest of the non-pressure pass's
         // (rank_gather_one).
         store_density(P, i, c, sum, pos, vel, count, rho, pres, vrho, xpf, a.st + a.scenes);

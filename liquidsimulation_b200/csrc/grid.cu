@@ -143,10 +143,11 @@ __global__ void k_neighbors_density(DevParams P, const float4* __restrict__ pos,
     extern __shared__ uint2 masks[];
     const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
     const bool valid = i < P.n;
-    int c = 0;
+    float* stage = reinterpret_cast<float*>(masks + blockDim.x * kScanChunks) + (threadIdx.x >> 5) * kStageFloats;
+    float sum;
+    const int c = neighbors_one<true>(P, pos, cell_start, nbr, min(i, P.n - 1), tables, masks + threadIdx.x, blockDim.x, &sum,
+                                      stage, valid);
     if (valid) {
-        float sum;
-        c = neighbors_one(P, pos, cell_start, nbr, i, tables, masks + threadIdx.x, blockDim.x, &sum);
         store_density(P, i, c, sum, pos, vel, count, rho, pres, vrho, xpf, st);
     }
     record_neighbor_count(P, c, valid, st);
@@ -215,11 +216,10 @@ int launch_grid_sort(const GridBuildArgs& a, cudaStream_t s)
 
 int launch_neighbors(const GridBuildArgs& a, cudaStream_t s)
 {
-    const int T = 256;
+    const int T = 128;
     if (a.P.n <= 0) return 0;
     launch_chained(k_neighbors_density, blocks_for(a.P.n, T), T, scan_smem(T), s, a.P, a.pos_out, a.cell_start, a.nbr,
-                                                                      a.nbr_count, a.status, a.tables, a.rho, a.pres,
-                                                                      a.vel_out, a.vrho, a.xpf);
+                   a.nbr_count, a.status, a.tables, a.rho, a.pres, a.vel_out, a.vrho, a.xpf);
     return 1;
 }
 

@@ -85,9 +85,15 @@ struct StepBuffers {
 // that many more.
 constexpr int kPosPad = 8;
 // Masks per thread that the neighbour scan keeps in dynamic shared memory (9 rows, and some to
-// spare), and their bytes for a block.
+// spare); the candidates of a row that a warp stages behind them, as three arrays kStagePitch apart;
+// and the bytes of both for a block.
 constexpr int kScanChunks = 12;
-inline size_t scan_smem(int threads) { return (size_t)threads * kScanChunks * sizeof(uint2); }
+constexpr int kStage = 96, kStagePitch = kStage + 4;
+constexpr int kStageFloats = 3 * kStagePitch;
+inline size_t scan_smem(int threads)
+{
+    return (size_t)threads * kScanChunks * sizeof(uint2) + (size_t)(threads / 32) * kStageFloats * sizeof(float);
+}
 
 // Entries of the histogram and cell-table buffers for `n` live entries: the scan moves them
 // 8 at a time, so both are padded to a multiple of 8 (the padding stays zero); and the scan's

@@ -66,6 +66,31 @@ __device__ __forceinline__ uint32_t scan_row(const float4* pos, V3 xi, float abo
     return bits & (0xffffffffu << over);
 }
 
+// scan_row over candidates staged as x[], y[], z[] (kStagePitch apart): those in [o, o + len), two at
+// a time from the even place at or below o, len <= 32 - (o & 1). Reads up to 3 past the end. `last`
+// is the staged index of the mask's bit 0. above - s is formed negated, s - above, for its sign.
+__device__ __forceinline__ uint32_t scan_staged(const float* st, F2 nx, F2 ny, F2 nz, F2 nabove, int o, int len, int& last)
+{
+    const int c = o & ~1, n = len + (o & 1);
+    const float* p = st + c;
+    uint32_t bits = 0;
+    for (int k = 0; k < n; k += 4, p += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+            const float2 x = *reinterpret_cast<const float2*>(p + u);
+            const float2 y = *reinterpret_cast<const float2*>(p + u + kStagePitch);
+            const float2 z = *reinterpret_cast<const float2*>(p + u + 2 * kStagePitch);
+            const F2 s = fma2(neg_sqmag(f2(x.x, x.y) + nx, f2(y.x, y.y) + ny, f2(z.x, z.y) + nz), f2(-1.f), nabove);
+            bits = __funnelshift_l(__float_as_uint(lo(s)), bits, 1);
+            bits = __funnelshift_l(__float_as_uint(hi(s)), bits, 1);
+        }
+    }
+    const int over = -n & 3;
+    last = c + n + over - 1;
+    if (o & 1) bits &= ~(1u << (last - c));
+    return bits & (0xffffffffu << over);
+}
+
 // Start-of-step neighbour list and density sum of particle i: every j with
 // |x_i - x_j|^2 <= h^2, including i, in the reference's order (SPHSpatialGrid::findNeighborParticles,
 // SPHSpatialGrid.cpp:39-76): cell ranges from (x -+ h) / h per axis, x then y rows, each row a
@@ -84,13 +109,23 @@ __device__ __forceinline__ uint32_t scan_row(const float4* pos, V3 xi, float abo
 // on average and scatters its 4-byte stores over as many lines, and its lists had to be regrouped
 // by the next pass. Build 0.254 -> 0.229 ms, non-pressure pass without the regrouping and loop
 // with the filled-up groups 1.16 -> 1.11 ms a step at 991,440 particles; 12,000 particles: build
-// 39 -> 21 us. It is bound by the L1 data pipe (84 % of its wavefronts: a candidate's 16-byte load takes
-// four to eight of them); 40 or 32 registers instead of 50 (6 or 8 blocks of 256 threads per SM) are
-// slower (0.238, 0.289 ms), the larger working set missing more in L1.
+// 39 -> 21 us.
+//
+// The scan is bound by the L1 data pipe: a candidate's 16-byte load by lanes in four or five cells
+// takes four to eight wavefronts (84 % of the pipe's rate). kWarp (every lane calls, `valid` or not;
+// stage: kStageFloats of the warp): a warp whose particles all search the same rows, as four of five
+// do, first copies the candidates of a row, all lanes' ranges together, to shared memory as x[], y[],
+// z[]; the lanes then read two candidates' coordinate by an 8-byte load, which is half the
+// wavefronts, and test them with packed arithmetic. A row of more than kStage candidates is scanned
+// from memory. Build 229 -> 182 us at 991,440 particles, 80 -> 58 at 250,000, 31 -> 29 at 102,400;
+// 174, 57 and 29 in blocks of 128 instead of 256 threads. Slower: a warp's two row groups one after
+// the other (216, 81, 31), a row's table entries fetched a row ahead (179, 58, 31). 64 or 128 staged
+// candidates make no difference.
+template <bool kWarp = false>
 __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* __restrict__ pos,
                                              const uint32_t* __restrict__ cell_start, int32_t* __restrict__ nbr,
                                              int i, const float* __restrict__ tables, uint2* col, int pitch,
-                                             float* wsum)
+                                             float* wsum, float* stage = nullptr, bool valid = true)
 {
     const V3 xi = v3(pos[i]);
     int lo_[3], hi_[3];
@@ -125,21 +160,69 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
         }
         next = chunks = 0;
     };
-    if (lo_[2] <= hi_[2]) {
+    auto keep = [&](uint32_t bits, int last_q) {
+        if (!bits) return;
+        if (chunks == kScanChunks) drain();
+        col[chunks * pitch] = make_uint2((uint32_t)last_q, bits);
+        chunks++;
+        pending += __popc(bits);
+    };
+    auto scan_own = [&](int beg, int end) {
+        for (; beg < end; beg += 32) {
+            int last_q;
+            const uint32_t bits = scan_row<4>(pos, xi, above, beg, min(end - beg, 32), last_q);
+            keep(bits, last_q);
+        }
+    };
+    valid = valid && lo_[2] <= hi_[2];
+    bool together = false;
+    if (kWarp) {
+        const uint32_t all = 0xffffffffu;
+        const uint32_t active = __ballot_sync(all, valid);
+        const int lead = active ? __ffs((int)active) - 1 : 0;   // the others compare their rows with its
+        const int x0 = __shfl_sync(all, lo_[0], lead), x1 = __shfl_sync(all, hi_[0], lead);
+        const int y0 = __shfl_sync(all, lo_[1], lead), y1 = __shfl_sync(all, hi_[1], lead);
+        together = __all_sync(all, !valid || (lo_[0] == x0 && hi_[0] == x1 && lo_[1] == y0 && hi_[1] == y1)) && active;
+        if (together) {
+            const int lane = threadIdx.x & 31;
+            const F2 nx = f2(-xi.x), ny = f2(-xi.y), nz = f2(-xi.z), nabove = f2(-above);
+            for (int cx = x0; cx <= x1; cx++) {
+                for (int cy = y0; cy <= y1; cy++) {
+                    const uint32_t row = P.cell_base + ((uint32_t)cx * (uint32_t)P.ny + (uint32_t)cy) * (uint32_t)P.nz;
+                    int beg = 0, end = 0;
+                    if (valid) {
+                        beg = (int)cell_start[row + lo_[2]];
+                        end = (int)cell_start[row + hi_[2] + 1];
+                    }
+                    const int ub = __reduce_min_sync(all, valid ? beg : 0x7fffffff), ue = __reduce_max_sync(all, end);
+                    if (ue - ub > kStage) {
+                        scan_own(beg, end);
+                        continue;
+                    }
+                    for (int k = lane; k < ue - ub; k += 32) {
+                        const float4 p = pos[ub + k];
+                        stage[k] = p.x;
+                        stage[k + kStagePitch] = p.y;
+                        stage[k + 2 * kStagePitch] = p.z;
+                    }
+                    __syncwarp();
+                    for (int o = beg - ub; o < end - ub;) {
+                        const int len = min(end - ub - o, 32 - (o & 1));
+                        int last_o;
+                        const uint32_t bits = scan_staged(stage, nx, ny, nz, nabove, o, len, last_o);
+                        keep(bits, ub + last_o);
+                        o += len;
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    }
+    if (!together && valid) {
         for (int cx = lo_[0]; cx <= hi_[0]; cx++) {
             for (int cy = lo_[1]; cy <= hi_[1]; cy++) {
                 const uint32_t row = P.cell_base + ((uint32_t)cx * (uint32_t)P.ny + (uint32_t)cy) * (uint32_t)P.nz;
-                const int end = (int)cell_start[row + hi_[2] + 1];
-                for (int beg = (int)cell_start[row + lo_[2]]; beg < end; beg += 32) {
-                    int last_q;
-                    const uint32_t bits = scan_row<4>(pos, xi, above, beg, min(end - beg, 32), last_q);
-                    if (bits) {
-                        if (chunks == kScanChunks) drain();
-                        col[chunks * pitch] = make_uint2((uint32_t)last_q, bits);
-                        chunks++;
-                        pending += __popc(bits);
-                    }
-                }
+                scan_own((int)cell_start[row + lo_[2]], (int)cell_start[row + hi_[2] + 1]);
             }
         }
     }
