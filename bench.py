@@ -81,7 +81,7 @@ ALGO_BYTES = {
     "neighbors": 16 + 4 + 4 + 4,     # read x; write count, rho, p (the list itself is not algorithmic)
     "density": 24,                   # read x; write rho, p
     "nonpressure": 52,               # read x, v, rho; write F
-    "sph_pressure": 56,
+    "sph_pressure": 56,              # all forces of SPH: read x, p / rho^2, v, rho; write F
     "pci_predict": 84,               # read x, v, v_half, F, F_p, rho (write x*, v_half*)
     "pci_density": 28,               # read x*, p; write rho*, p
     "pci_force": 44,                 # read x*, p/rho*^2, rho; write F_p

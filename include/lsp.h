@@ -254,7 +254,7 @@ int lsp_timer_elapsed(lsp_solver* s, int slot_a, int slot_b, float* ms);
 #define LSP_PROF_NEIGHBORS     1
 #define LSP_PROF_DENSITY       2
 #define LSP_PROF_NONPRESSURE   3
-#define LSP_PROF_SPH_PRESSURE  4
+#define LSP_PROF_SPH_PRESSURE  4   /* SPH: all forces, the non-pressure ones included */
 #define LSP_PROF_PCI_PREDICT   5
 #define LSP_PROF_PCI_DENSITY   6
 #define LSP_PROF_PCI_FORCE     7

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(T) kb_nonpressure(BatchArgs a, StepBuffers b)
 }
 
 template <int T>
-__global__ void __launch_bounds__(T) kb_sph_pressure(BatchArgs a, StepBuffers b)
+__global__ void __launch_bounds__(T) kb_sph_forces(BatchArgs a, StepBuffers b)
 {
     __shared__ DevParams P;
     const BatchItem it = a.items[blockIdx.x];
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(T) kb_sph_pressure(BatchArgs a, StepBuffers b)
     __syncthreads();
     const int i = it.begin + (int)threadIdx.x;
     if (i >= it.end) return;
-    sph_pressure_one(P, b, i);
+    sph_forces_one(P, b, i);
 }
 
 template <int T>
@@ -441,10 +441,10 @@ int launch_batch_nonpressure(const BatchArgs& a, const StepBuffers& b, cudaStrea
     return 1;
 }
 
-int launch_batch_sph_pressure(const BatchArgs& a, const StepBuffers& b, cudaStream_t s)
+int launch_batch_sph_forces(const BatchArgs& a, const StepBuffers& b, cudaStream_t s)
 {
     if (!a.items_count) return 0;
-    LSP_BATCH_DISPATCH(a.threads, (kb_sph_pressure<T><<<a.items_count, T, 0, s>>>(a, b)));
+    LSP_BATCH_DISPATCH(a.threads, (kb_sph_forces<T><<<a.items_count, T, 0, s>>>(a, b)));
     return 1;
 }
 

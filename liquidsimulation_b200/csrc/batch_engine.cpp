@@ -434,8 +434,8 @@ int BatchEngine::enqueue_step(int c, int grid)
     StepBuffers b = buffers(1 - c);
     launches += launch_batch_neighbors_density(a, pos_[1 - c].p, cell_start_.p, nbr_.p, nbr_count_.p, rho_.p,
                                                pres_.p, vel_[1 - c].p, vrho_.p, pcisph_ ? nullptr : ppos_alt_.p, stream_);
-    launches += launch_batch_nonpressure(a, b, stream_);
     if (pcisph_) {
+        launches += launch_batch_nonpressure(a, b, stream_);
         if (feats) {
             // Iteration 0 outside the persistent kernel: predict, then density with the
             // features and (warm start) the network's guess.
@@ -466,7 +466,7 @@ int BatchEngine::enqueue_step(int c, int grid)
             throw Error(LSP_ERR_CUDA, "the cooperative launch of the batch's PCISPH loop was refused");
         launches++;   // the loop integrates each scene in its last pass
     } else {
-        launches += launch_batch_sph_pressure(a, b, stream_);
+        launches += launch_batch_sph_forces(a, b, stream_);
         launches += launch_batch_integrate(a, b, false, stream_);
     }
     CK(cudaGetLastError());

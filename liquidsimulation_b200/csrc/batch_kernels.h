@@ -49,7 +49,7 @@ int launch_batch_neighbors_density(const BatchArgs& a, const float4* pos, const 
                                    int32_t* count, float* rho, float* pres, const float4* vel, float4* vrho,
                                    float4* xpf, cudaStream_t s);
 int launch_batch_nonpressure(const BatchArgs& a, const StepBuffers& b, cudaStream_t s);
-int launch_batch_sph_pressure(const BatchArgs& a, const StepBuffers& b, cudaStream_t s);
+int launch_batch_sph_forces(const BatchArgs& a, const StepBuffers& b, cudaStream_t s);
 int launch_batch_integrate(const BatchArgs& a, const StepBuffers& b, bool add_pforce, cudaStream_t s);
 
 // Learned warm start of a batch: iteration 0's predict, then its density pass with the

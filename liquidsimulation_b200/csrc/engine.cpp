@@ -830,13 +830,13 @@ void Engine::run_step(float dt, lsp_step_stats* st)
         timed(LSP_PROF_GRID_SCATTER, [&] { return launch_grid_scatter(g, stream_); });
         timed(LSP_PROF_GRID_GATHER, [&] { return launch_grid_gather(g, stream_); });
         timed(LSP_PROF_NEIGHBORS, [&] { return launch_neighbors(g, stream_); });
-        timed(LSP_PROF_NONPRESSURE, [&] { launch_nonpressure(P, b, stream_); return 1; });
         if (prm_.solver == LSP_SOLVER_SPH) {
-            timed(LSP_PROF_SPH_PRESSURE, [&] { launch_sph_pressure(P, b, stream_); return 1; });
+            timed(LSP_PROF_SPH_PRESSURE, [&] { launch_sph_forces(P, b, stream_); return 1; });
             timed(LSP_PROF_INTEGRATE, [&] { launch_integrate_collide(P, b, false, stream_); return 1; });
             local.iterations = 0;
             local.converged = 1;
         } else {
+            timed(LSP_PROF_NONPRESSURE, [&] { launch_nonpressure(P, b, stream_); return 1; });
             device_loop = pcisph_loop(P, b, &local);
             // The persistent loop integrates in its last pass; the per-phase loop does not.
             if (!device_loop)

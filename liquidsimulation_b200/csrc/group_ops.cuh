@@ -295,7 +295,7 @@ __device__ __forceinline__ V3 group_pci_force(const Group<L>& g, const DevParams
                                   ? group_pci_force_walk<L, true>(g, P, b, i, ppos, xi, tf, list)
                                   : group_pci_force_walk<L, false>(g, P, b, i, ppos, xi, tf, list));
 }
-// The SPH pressure force of particle i (sph_pressure_one), in every lane.
+// The SPH pressure force of particle i (its part of sph_forces_walk), in every lane.
 template <int L>
 __device__ __forceinline__ V3 group_sph_pressure(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i, V3 xi,
                                                  float rhoi, const HeldList<L>& list)

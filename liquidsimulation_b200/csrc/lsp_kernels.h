@@ -116,7 +116,7 @@ int launch_grid_gather(const GridBuildArgs& a, cudaStream_t s);
 
 // With b.gradrho set, also stores |grad rho| (a warm-start feature).
 void launch_nonpressure(const DevParams& P, const StepBuffers& b, cudaStream_t s);
-void launch_sph_pressure(const DevParams& P, const StepBuffers& b, cudaStream_t s);
+void launch_sph_forces(const DevParams& P, const StepBuffers& b, cudaStream_t s);
 void launch_integrate_collide(const DevParams& P, const StepBuffers& b, bool add_pforce, cudaStream_t s);
 
 void launch_pci_predict(const DevParams& P, const StepBuffers& b, int iteration, cudaStream_t s);

@@ -687,20 +687,64 @@ __device__ __forceinline__ void pci_force_one(const DevParams& P, const StepBuff
     b.pforce[i] = f4(pci_pressure_force(P, b.rho[i], pci_force_sum(P, b, i, ppos)), 0.f);
 }
 
-// SPHSolver::accumulatePressureForces, CPU branch (SPHSolver.cpp:268-290): the PCISPH pressure force's
-// sum over the positions and factors p / rho^2 (StepBuffers::xpf; the factor is the quotient the
+// All forces of SPH in one walk of the list: nonpressure_walk's sums and, beside them, the pressure
+// force's (SPHSolver::accumulatePressureForces, CPU branch, SPHSolver.cpp:268-290), which is the PCISPH
+// force's sum over the positions and factors p / rho^2 (StepBuffers::xpf; the factor is the quotient the
 // reference takes per pair), without its test for NaN. Where the step's positions are in range, the
-// distance and direction come from the exact forms, two pairs at a time: 54 -> 25 us at 250,047
-// particles against one pair at a time with IEEE square root and four IEEE divisions.
-__device__ __forceinline__ void sph_pressure_one(const DevParams& P, const StepBuffers& b, int i)
+// distance and direction come from the exact forms, two pairs at a time. Two walks, each fetching the
+// list and the neighbours' positions, took 37 + 25 us at 250,047 particles; this one 45.5 in blocks
+// of 128 threads with the 94 registers it asks for (47.5 with 80, 60 with 64 and spills, 50 in blocks
+// of 256).
+template <bool kExactDiv>
+__device__ __forceinline__ void sph_forces_walk(const DevParams& P, const StepBuffers& b, int i)
 {
-    V3 pf = *(const volatile uint32_t*)&b.status->np_unsafe == 0u ? pci_force_walk<true>(P, b, i, b.xpf)
-                                                                  : pci_force_walk<false>(P, b, i, b.xpf);
-    const float4 f = b.force[i];
-    pf *= -(P.mass * f.w);
-    V3 F = v3(f);
+    const float4 xi4 = b.xpf[i];
+    const V3 xi = v3(xi4);
+    const float tf = xi4.w;
+    const V3 vi = v3(b.vel[i]);
+    const float rhoi = b.rho[i];
+    V3 normal = v3(0.f, 0.f, 0.f), visc = v3(0.f, 0.f, 0.f), pf = v3(0.f, 0.f, 0.f);
+    float lap = 0.f;
+    auto one = [&](int j, const NonpressureRec& r) {
+        const NonpressureTerms t = nonpressure_term<false>(P, b.tables, xi, vi, rhoi, r);
+        normal += t.normal;
+        lap += t.lap;
+        if (j == i) return;
+        visc += t.visc;
+        pf += pci_force_term(P, b.tables, xi, tf, r.x);
+    };
+    auto pair = [&](int j0, const NonpressureRec& r0, int j1, const NonpressureRec& r1, bool two) {
+        if (!kExactDiv) {
+            one(j0, r0);
+            if (two) one(j1, r1);
+            return;
+        }
+        const NonpressureTerms2 t = nonpressure_pair<false>(P, b.tables, xi, vi, rhoi, r0, r1);
+        const V3x2 f = pci_force_pair(P, b.tables, xi, tf, r0.x, r1.x);
+        normal += v3(lo(t.nx), lo(t.ny), lo(t.nz));
+        lap += lo(t.lap);
+        visc += v3(lo(t.vx), lo(t.vy), lo(t.vz));
+        if (j0 != i) pf += v3(lo(f.x), lo(f.y), lo(f.z));
+        if (two) {
+            normal += v3(hi(t.nx), hi(t.ny), hi(t.nz));
+            lap += hi(t.lap);
+            visc += v3(hi(t.vx), hi(t.vy), hi(t.vz));
+            if (j1 != i) pf += v3(hi(f.x), hi(f.y), hi(f.z));
+        }
+    };
+    for_each_neighbor<2>(b.nbr, i, P.nbr_stride, __ldg(b.nbr_count + i),
+                         [&](int j) { return NonpressureRec{b.xpf[j], b.vrho[j]}; }, pair);
+    V3 F = nonpressure_force(P, rhoi, normal, lap, visc);
+    pf *= -(P.mass * rhoi);
     F += pf;
-    b.force[i] = f4(F, f.w);
+    b.force[i] = f4(F, rhoi);
+}
+__device__ __forceinline__ void sph_forces_one(const DevParams& P, const StepBuffers& b, int i)
+{
+    if (P.exact_tables && *(const volatile uint32_t*)&b.status->np_unsafe == 0u)
+        sph_forces_walk<true>(P, b, i);
+    else
+        sph_forces_walk<false>(P, b, i);
 }
 
 // The persistent loops' fused pass: the pressure force of iteration k - 1 at positions `from`, then

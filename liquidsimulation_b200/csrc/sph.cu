@@ -1,6 +1,5 @@
-// SPH passes over the start-of-step neighbour lists: non-pressure forces (gravity,
-// surface tension, viscosity), the SPH pressure force, and the fused leapfrog integration +
-// collision pass (the density and pressure are summed in the neighbour build, grid.cu).
+// Passes over the start-of-step neighbour lists: non-pressure forces (gravity, surface tension,
+// viscosity) of PCISPH, all forces of SPH, and the fused leapfrog integration + collision pass (the density and pressure are summed in the neighbour build, grid.cu).
 //
 // Thread per particle; each thread walks its own neighbour list in the reference's
 // order, so its sums round exactly as the reference CPU solver's do.
@@ -24,12 +23,12 @@ __global__ void __launch_bounds__(kThreads) k_nonpressure(DevParams P, StepBuffe
     if (i < P.n) nonpressure_one<kGrad>(P, b, i);
 }
 
-// SPHSolver::accumulatePressureForces, CPU branch (SPHSolver.cpp:268-290).
-__global__ void __launch_bounds__(kThreads) k_sph_pressure(DevParams P, StepBuffers b)
+// All forces of SPH (sph_forces_walk).
+constexpr int kForceThreads = 128;
+__global__ void __launch_bounds__(kForceThreads) k_sph_forces(DevParams P, StepBuffers b)
 {
     const int i = chained((int)(blockIdx.x * blockDim.x + threadIdx.x));
-    if (i >= P.n) return;
-    sph_pressure_one(P, b, i);
+    if (i < P.n) sph_forces_one(P, b, i);
 }
 
 // SPHParticle::integrate (SPHParticle.cpp:30-44) then SPHSolver::handleCollisions
@@ -52,9 +51,9 @@ void launch_nonpressure(const DevParams& P, const StepBuffers& b, cudaStream_t s
     else
         launch_chained(k_nonpressure<false>, blocks_for(P.n, kThreads), kThreads, 0, s, P, b);
 }
-void launch_sph_pressure(const DevParams& P, const StepBuffers& b, cudaStream_t s)
+void launch_sph_forces(const DevParams& P, const StepBuffers& b, cudaStream_t s)
 {
-    if (P.n) launch_chained(k_sph_pressure, blocks_for(P.n, kThreads), kThreads, 0, s, P, b);
+    if (P.n) launch_chained(k_sph_forces, blocks_for(P.n, kForceThreads), kForceThreads, 0, s, P, b);
 }
 void launch_integrate_collide(const DevParams& P, const StepBuffers& b, bool add_pforce, cudaStream_t s)
 {
