@@ -347,14 +347,16 @@ int lsp_batch_write_state(lsp_batch* b, const float* x, const float* v, const fl
                           const float* v_half_old, const int32_t* first_step, int64_t n);
 /* Launch shape: use_graph (0/1), threads (128, 256, 512 or 1024 particles per block), loop_blocks
  * (blocks of the persistent kernel, 0 = all that fit). At the default shape (256, 0) a small batch
- * steps in one kernel, which has no shape; any other shape selects the separate kernels. get also
- * reports whether the step currently runs as a captured graph. */
+ * steps in one kernel, which has no shape, and the persistent kernel of a batch of large scenes takes
+ * blocks of its own size; any other shape is used as given. get also reports whether the step
+ * currently runs as a captured graph. */
 int lsp_batch_set_launch(lsp_batch* b, int use_graph, int threads, int loop_blocks);
 int lsp_batch_get_launch(const lsp_batch* b, int* use_graph, int* threads, int* loop_blocks, int* graph_active);
 /* Autotuner: runs the next step under each candidate launch shape (particles per block x
  * persistent-kernel blocks), re-running that same step from the same state `repeats` times
- * per candidate, keeps the fastest shape (a small batch stays in one kernel when no shape is
- * faster), and leaves the batch advanced by exactly that one step (results do not depend on the shape). result and stats may be NULL. */
+ * per candidate, keeps the fastest shape (or, when no shape is faster, what the default shape
+ * runs), and leaves the batch advanced by exactly that one step (results do not depend on the
+ * shape). result and stats may be NULL. */
 int lsp_batch_autotune(lsp_batch* b, float dt, int repeats, lsp_batch_tuning* result, lsp_step_stats* stats);
 /* Learned warm start for the scenes of a PCISPH batch (LSP_WARM_ZERO, LSP_WARM_MLP or
  * LSP_WARM_AUTO; AUTO switches each scene on by itself, at that scene's

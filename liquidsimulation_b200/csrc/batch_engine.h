@@ -83,6 +83,7 @@ private:
     void build_items();
     void ensure_neighbors(int cap);
     void drop_graphs();
+    int loop_threads() const;
     int loop_grid() const;
     int enqueue_step(int c, int grid);   // returns the number of kernels launched
     // Whether the step runs as one launch (small_step.cu): the batch is small enough, no features

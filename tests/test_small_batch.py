@@ -110,3 +110,9 @@ def test_autotune_and_direct_launches():
             assert np.array_equal(bits(a.read(k, f)), bits(b.read(k, f))), (k, f)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("counts", [(8192,) * 5, (8191,) * 5, (30000, 9000, 1025)])
+def test_blocks_of_the_loop_over_large_scenes(counts):
+    """Scenes of 8,192 particles on average take the loop's 1024-thread blocks at the default shape."""
+    compare(boxes(counts), 2, small=False, lists=False)
