@@ -50,7 +50,14 @@ __device__ __forceinline__ void load8(const uint32_t* p, uint32_t (&v)[kScanItem
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// Writes the exclusive scan of v, starting at ex, to out[0..7] and clears hist[0..7].
+__device__ __forceinline__ void clear8(uint32_t* p)
+{
+    *reinterpret_cast<uint4*>(p) = make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(p + 4) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Writes the exclusive scan of v, starting at ex, to out[0..7] and clears hist[0..7] (hist: may be
+// null).
 __device__ __forceinline__ void store8_scan(uint32_t* out, uint32_t* hist, const uint32_t (&v)[kScanItems], uint32_t ex)
 {
     uint32_t o[kScanItems];
@@ -61,8 +68,7 @@ __device__ __forceinline__ void store8_scan(uint32_t* out, uint32_t* hist, const
     }
     *reinterpret_cast<uint4*>(out) = make_uint4(o[0], o[1], o[2], o[3]);
     *reinterpret_cast<uint4*>(out + 4) = make_uint4(o[4], o[5], o[6], o[7]);
-    *reinterpret_cast<uint4*>(hist) = make_uint4(0u, 0u, 0u, 0u);
-    *reinterpret_cast<uint4*>(hist + 4) = make_uint4(0u, 0u, 0u, 0u);
+    if (hist) clear8(hist);
 }
 
 }  // namespace lsp

@@ -10,9 +10,10 @@
 // list and state in registers for the whole step, so a pass is one dependent fetch (the neighbours'
 // positions) and a barrier. A PCISPH step with 4 iterations, wall clock, separate kernels -> this:
 // 1,200 particles 89 -> 42 us, 4,700 145 -> 73, 9,400 156 -> 93, 18,900 177 -> 118, 30,000 203 ->
-// 180, 37,800 219 -> 188 us. About 1.2 us of it is each grid barrier (7 + 2 per iteration).
+// 180, 37,800 219 -> 188 us. About 1.2 us of it is each grid barrier (6 + 2 per iteration, 7 in a
+// large grid).
 //
-//   keys | scan sums | scan apply | scatter | rank + gather | lists + density |
+//   keys | (scan sums |) scan | scatter | rank + gather | lists + density |
 //   non-pressure + predict(0), then the loop of k_pci_loop       (PCISPH)
 //   non-pressure + pressure | integrate                          (SPH)
 //
@@ -30,6 +31,9 @@ namespace lsp {
 
 // 512 threads per SM leave each 128 registers: the groups keep their particle's list and state there.
 constexpr int kMaxThreads = 512;
+// Rounds of the block over the counts that cost less than the barrier they save. A step of 12,000
+// particles in 4,000 cells takes 1.7 us less, 1,200 in 15,600 cells 1.5 us less (4 rounds: not taken).
+constexpr int kFewRounds = 12;
 // A batch's blocks: small, so that a scene's last one wastes little. 16 scenes, 20,071 particles, four
 // steps with their transfers: 464 us with 128 threads, 475 with 256, 495 with 64.
 constexpr int kBatchThreads = 128;
@@ -94,37 +98,48 @@ __device__ __forceinline__ void small_step(const DevParams& P, const GridBuildAr
     const int64_t n8 = scan_entries((int64_t)P.cells + 1);
     const int64_t per = (n8 / kScanItems + blocks - 1) / blocks * kScanItems;
     const int64_t c0 = min((int64_t)block * per, n8), c1 = min(c0 + per, n8);
-    {
+    const int64_t stride = (int64_t)blockDim.x * kScanItems, own = (int64_t)threadIdx.x * kScanItems;
+    auto sum_of = [&](int64_t from, int64_t to) {
         uint32_t s = 0;
-        for (int64_t e = c0 + (int64_t)threadIdx.x * kScanItems; e < c1; e += (int64_t)blockDim.x * kScanItems) {
+#pragma unroll 4
+        for (int64_t e = from + own; e < to; e += stride) {
             uint32_t v[kScanItems];
             load8(hist + e, v);
 #pragma unroll
             for (int j = 0; j < kScanItems; j++) s += v[j];
         }
+        return s;
+    };
+    // Few cells: each block adds up the counts before its run itself, which saves a barrier; the counts
+    // are then cleared once every block has read them.
+    const bool few = n8 <= kFewRounds * stride;
+    uint32_t carry;
+    if (few) {
+        block_exclusive_scan(sum_of(0, c0), ws, &carry);
+    } else {
         uint32_t total;
-        block_exclusive_scan(s, ws, &total);
+        block_exclusive_scan(sum_of(c0, c1), ws, &total);
         if (threadIdx.x == 0) own_blocks.tile_sums[block] = total;
-    }
-    if (!barrier()) return;
-    {
-        uint32_t s = 0, carry;
+        if (!barrier()) return;
+        uint32_t s = 0;
         for (int k = threadIdx.x; k < block; k += blockDim.x) s += __ldcg(own_blocks.tile_sums + k);
         block_exclusive_scan(s, ws, &carry);
-        carry += (uint32_t)base;
-        for (int64_t e0 = c0; e0 < c1; e0 += (int64_t)blockDim.x * kScanItems) {
-            const int64_t e = e0 + (int64_t)threadIdx.x * kScanItems;
-            uint32_t v[kScanItems] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (e < c1) load8(hist + e, v);
-            uint32_t sum = 0, total;
+    }
+    carry += (uint32_t)base;
+    for (int64_t e0 = c0; e0 < c1; e0 += stride) {
+        const int64_t e = e0 + own;
+        uint32_t v[kScanItems] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (e < c1) load8(hist + e, v);
+        uint32_t sum = 0, total;
 #pragma unroll
-            for (int j = 0; j < kScanItems; j++) sum += v[j];
-            const uint32_t ex = block_exclusive_scan(sum, ws, &total) + carry;
-            if (e < c1) store8_scan(cell_start + e, hist + e, v, ex);
-            carry += total;
-        }
+        for (int j = 0; j < kScanItems; j++) sum += v[j];
+        const uint32_t ex = block_exclusive_scan(sum, ws, &total) + carry;
+        if (e < c1) store8_scan(cell_start + e, few ? nullptr : hist + e, v, ex);
+        carry += total;
     }
     if (!barrier()) return;
+    if (few)
+        for (int64_t e = c0 + own; e < c1; e += stride) clear8(hist + e);
 
     // ---- scatter (k_scatter), then rank by caller id inside the cell and move the state
     // (rank_gather_one, from the particle's side)
