@@ -15,7 +15,7 @@
 //
 //   keys | (scan sums |) scan | scatter | rank + gather | lists + density |
 //   non-pressure + predict(0), then the loop of k_pci_loop       (PCISPH)
-//   non-pressure + pressure | integrate                          (SPH)
+//   all forces | integrate                                       (SPH)
 //
 // Everything one phase writes and a later one reads goes through plain or L2 loads; the grid
 // barrier orders them.
@@ -191,7 +191,7 @@ __device__ __forceinline__ void small_step(const DevParams& P, const GridBuildAr
     const V3 x0 = v3(p4), half0 = v3(h4);
     V3 v = v3(v4);
     const bool lead = valid && grp.lane == 0;   // the lane that stores the particle's results
-    V3 F = group_nonpressure(grp, P, b, i, x0, v, rho, list);
+    V3 F = pcisph ? group_nonpressure(grp, P, b, i, x0, v, rho, list) : group_sph_forces(grp, P, b, i, x0, v, rho, list);
     auto integrate = [&](V3 total, float p) {
         V3 x = x0, half = half0, old;
         float first = v4.w;
@@ -210,7 +210,6 @@ __device__ __forceinline__ void small_step(const DevParams& P, const GridBuildAr
 
     if (!pcisph) {
         const float pres = b.pres[i];
-        F += group_sph_pressure(grp, P, b, i, x0, rho, list);
         if (!barrier()) return;   // the positions are read by other groups until here
         integrate(F, pres);
         if (tid == 0) *own_blocks.host = *st;
