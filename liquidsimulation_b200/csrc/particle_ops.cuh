@@ -116,11 +116,20 @@ __device__ __forceinline__ uint32_t scan_staged(const float* st, F2 nx, F2 ny, F
 // stage: kStageFloats of the warp): a warp whose particles all search the same rows, as four of five
 // do, first copies the candidates of a row, all lanes' ranges together, to shared memory as x[], y[],
 // z[]; the lanes then read two candidates' coordinate by an 8-byte load, which is half the
-// wavefronts, and test them with packed arithmetic. A row of more than kStage candidates is scanned
-// from memory. Build 229 -> 182 us at 991,440 particles, 80 -> 58 at 250,000, 31 -> 29 at 102,400;
+// wavefronts, and test them with packed arithmetic; a row of more than kStage candidates goes through
+// in pieces. Build 229 -> 182 us at 991,440 particles, 80 -> 58 at 250,000, 31 -> 29 at 102,400;
 // 174, 57 and 29 in blocks of 128 instead of 256 threads. Slower: a warp's two row groups one after
 // the other (216, 81, 31), a row's table entries fetched a row ahead (179, 58, 31). 64 or 128 staged
 // candidates make no difference.
+//
+// Rows of more than 32 particles (kernels wider than about 4 radii, compressed fluid) need more masks
+// than a column holds. A full column is emptied in the same groups of four, by a whole warp at once
+// where it scans together: `room` counts the free masks that every lane has at least, so that rows
+// of usual length cost one vote in six. Emptied one entry at a time, 64,000 particles with 117
+// neighbours took 426 us and with 207 neighbours 795, now 119 and 248; 250,047 with 458 neighbours
+// 5.42 -> 1.16 ms. A check per lane instead of the warp's took 264 us at 117 neighbours; scanning
+// that can be left and resumed, so that the groups are taken in one place, 92 us there, but 193 us
+// instead of 180 at 991,440 particles with 29.
 template <bool kWarp = false>
 __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* __restrict__ pos,
                                              const uint32_t* __restrict__ cell_start, int32_t* __restrict__ nbr,
@@ -149,30 +158,46 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
         m ^= 1u << b;
         return last - b;
     };
-    // Takes every waiting entry one by one; only when a list needs more masks than the column
-    // holds (rows of more than 32 particles).
-    auto drain = [&]() {
-        for (; pending > 0; pending--) {
-            const int q = take();
-            sum += weight_w(sqmag(xi - v3(pos[q])), P, tables);
-            if (stored < P.nbr_cap) reinterpret_cast<int32_t*>(out + (int64_t)(stored >> 2) * stride)[stored & 3] = q;
-            stored++;
-        }
-        next = chunks = 0;
-    };
     auto keep = [&](uint32_t bits, int last_q) {
         if (!bits) return;
-        if (chunks == kScanChunks) drain();
         col[chunks * pitch] = make_uint2((uint32_t)last_q, bits);
         chunks++;
         pending += __popc(bits);
     };
-    auto scan_own = [&](int beg, int end) {
-        for (; beg < end; beg += 32) {
-            int last_q;
-            const uint32_t bits = scan_row<4>(pos, xi, above, beg, min(end - beg, 32), last_q);
-            keep(bits, last_q);
+    // Takes the waiting entries, four at a time, while at least `least` of them wait (1: all of them,
+    // the last group filled up).
+    auto emit = [&](int least) {
+        for (; pending >= least; out += stride) {
+            const int left = pending;
+            int4 q = make_int4(i, i, i, i);
+            q.x = take();
+            if (left > 1) q.y = take();
+            if (left > 2) q.z = take();
+            if (left > 3) q.w = take();
+            const float4 a = pos[q.x], b = pos[q.y], c = pos[q.z], e = pos[q.w];
+            if (stored < P.nbr_cap) *out = q;
+            const F2 w0 = weight_w(neg_sqmag(f2(a.x - xi.x, b.x - xi.x), f2(a.y - xi.y, b.y - xi.y), f2(a.z - xi.z, b.z - xi.z)),
+                                   P, tables);
+            const F2 w1 = weight_w(neg_sqmag(f2(c.x - xi.x, e.x - xi.x), f2(c.y - xi.y, e.y - xi.y), f2(c.z - xi.z, e.z - xi.z)),
+                                   P, tables);
+            sum += lo(w0);
+            if (left > 1) sum += hi(w0);
+            if (left > 2) sum += lo(w1);
+            if (left > 3) sum += hi(w1);
+            stored += min(left, 4);
+            pending -= min(left, 4);
         }
+    };
+    // Makes room in the column: takes the whole groups of the waiting entries; the masks of the up to
+    // three that are left move to its front.
+    auto drain = [&]() {
+        emit(4);
+        int kept = 0;
+        if (m) col[kept++ * pitch] = make_uint2((uint32_t)last, m);
+        for (; next < chunks; next++) col[kept++ * pitch] = col[next * pitch];
+        m = 0u;
+        next = 0;
+        chunks = kept;
     };
     valid = valid && lo_[2] <= hi_[2];
     bool together = false;
@@ -186,6 +211,7 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
         if (together) {
             const int lane = threadIdx.x & 31;
             const F2 nx = f2(-xi.x), ny = f2(-xi.y), nz = f2(-xi.z), nabove = f2(-above);
+            int room = kScanChunks;   // masks that every lane's column still holds, at least
             for (int cx = x0; cx <= x1; cx++) {
                 for (int cy = y0; cy <= y1; cy++) {
                     const uint32_t row = P.cell_base + ((uint32_t)cx * (uint32_t)P.ny + (uint32_t)cy) * (uint32_t)P.nz;
@@ -195,25 +221,35 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
                         end = (int)cell_start[row + hi_[2] + 1];
                     }
                     const int ub = __reduce_min_sync(all, valid ? beg : 0x7fffffff), ue = __reduce_max_sync(all, end);
-                    if (ue - ub > kStage) {
-                        scan_own(beg, end);
-                        continue;
+                    for (int from = ub; from < ue; from += kStage) {
+                        const int staged = min(ue - from, kStage);
+                        const int to = min(end - from, staged);   // this lane's candidates: [o, to)
+                        int o = max(beg - from, 0);
+                        const int masks = (staged + 32) >> 5;   // most that a lane adds
+                        if (room < masks) {
+                            room = kScanChunks - __reduce_max_sync(all, chunks);
+                            if (room < masks) {
+                                drain();
+                                room = kScanChunks - 3;
+                            }
+                        }
+                        room -= masks;
+                        for (int k = lane; k < staged; k += 32) {
+                            const float4 p = pos[from + k];
+                            stage[k] = p.x;
+                            stage[k + kStagePitch] = p.y;
+                            stage[k + 2 * kStagePitch] = p.z;
+                        }
+                        __syncwarp();
+                        while (o < to) {
+                            const int len = min(to - o, 32 - (o & 1));
+                            int last_o;
+                            const uint32_t bits = scan_staged(stage, nx, ny, nz, nabove, o, len, last_o);
+                            keep(bits, from + last_o);
+                            o += len;
+                        }
+                        __syncwarp();
                     }
-                    for (int k = lane; k < ue - ub; k += 32) {
-                        const float4 p = pos[ub + k];
-                        stage[k] = p.x;
-                        stage[k + kStagePitch] = p.y;
-                        stage[k + 2 * kStagePitch] = p.z;
-                    }
-                    __syncwarp();
-                    for (int o = beg - ub; o < end - ub;) {
-                        const int len = min(end - ub - o, 32 - (o & 1));
-                        int last_o;
-                        const uint32_t bits = scan_staged(stage, nx, ny, nz, nabove, o, len, last_o);
-                        keep(bits, ub + last_o);
-                        o += len;
-                    }
-                    __syncwarp();
                 }
             }
         }
@@ -222,39 +258,19 @@ __device__ __forceinline__ int neighbors_one(const DevParams& P, const float4* _
         for (int cx = lo_[0]; cx <= hi_[0]; cx++) {
             for (int cy = lo_[1]; cy <= hi_[1]; cy++) {
                 const uint32_t row = P.cell_base + ((uint32_t)cx * (uint32_t)P.ny + (uint32_t)cy) * (uint32_t)P.nz;
-                scan_own((int)cell_start[row + lo_[2]], (int)cell_start[row + hi_[2] + 1]);
+                const int end = (int)cell_start[row + hi_[2] + 1];
+                for (int beg = (int)cell_start[row + lo_[2]]; beg < end; beg += 32) {
+                    if (chunks == kScanChunks) drain();
+                    int last_q;
+                    const uint32_t bits = scan_row<4>(pos, xi, above, beg, min(end - beg, 32), last_q);
+                    keep(bits, last_q);
+                }
             }
         }
     }
-    if (stored) {
-        drain();
-        const int rest = -stored & 3;
-        for (int k = stored; k < stored + rest && k < P.nbr_cap; k++)
-            reinterpret_cast<int32_t*>(out + (int64_t)(k >> 2) * stride)[k & 3] = i;
-        *wsum = sum;
-        return stored;
-    }
-    for (int k = 0; k < pending; k += 4) {
-        const int left = pending - k;
-        int4 q = make_int4(i, i, i, i);
-        q.x = take();
-        if (left > 1) q.y = take();
-        if (left > 2) q.z = take();
-        if (left > 3) q.w = take();
-        const float4 a = pos[q.x], b = pos[q.y], c = pos[q.z], e = pos[q.w];
-        if (k < P.nbr_cap) *out = q;
-        out += stride;
-        const F2 w0 = weight_w(neg_sqmag(f2(a.x - xi.x, b.x - xi.x), f2(a.y - xi.y, b.y - xi.y), f2(a.z - xi.z, b.z - xi.z)),
-                               P, tables);
-        const F2 w1 = weight_w(neg_sqmag(f2(c.x - xi.x, e.x - xi.x), f2(c.y - xi.y, e.y - xi.y), f2(c.z - xi.z, e.z - xi.z)),
-                               P, tables);
-        sum += lo(w0);
-        if (left > 1) sum += hi(w0);
-        if (left > 2) sum += lo(w1);
-        if (left > 3) sum += hi(w1);
-    }
+    emit(1);
     *wsum = sum;
-    return pending;
+    return stored;
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt()
