@@ -172,6 +172,12 @@ int lsp_step(lsp_solver* s, float dt, lsp_step_stats* stats);
  * the next is queued (a step whose neighbour lists overflow is redone with larger lists), so
  * this saves the per-call overhead, not the per-step synchronisation. */
 int lsp_step_many(lsp_solver* s, float dt, int steps, lsp_step_stats* stats);
+/* Check of a step that gives up (no counterpart in the reference): the next step, as one launch, whose
+ * barrier-th grid barrier (from 1) waits for an arrival that does not come, for a short time. A step
+ * of one launch that gives up returns LSP_ERR_TIMEOUT and leaves the state as it was before the call
+ * (its lists and grid are refused until the next step). LSP_ERR_STATE when the step would not run as
+ * one launch; LSP_OK, and an ordinary step, when it has fewer barriers. */
+int lsp_stalled_step(lsp_solver* s, float dt, int barrier);
 int lsp_synchronize(lsp_solver* s);
 
 /* ---- read-back / state (caller order) ---- */
@@ -331,6 +337,8 @@ int lsp_batch_scene_count(const lsp_batch* b, int32_t scene, int64_t* n);
 int lsp_batch_particle_mass(const lsp_batch* b, int32_t scene, float* mass);
 /* One step of every scene. stats: NULL or an array of one lsp_step_stats per scene. */
 int lsp_batch_step(lsp_batch* b, float dt, lsp_step_stats* stats);
+/* lsp_stalled_step at a barrier of one scene; all scenes stay as they were. */
+int lsp_batch_stalled_step(lsp_batch* b, float dt, int32_t scene, int barrier);
 /* Per-scene read-back in the scene's caller order (n = the scene's particle count). */
 int lsp_batch_read_particles(lsp_batch* b, int32_t scene, float* xyz, float* vel, int64_t n);
 int lsp_batch_read_field(lsp_batch* b, int32_t scene, int field, float* out, int64_t n);

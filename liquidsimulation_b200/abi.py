@@ -193,6 +193,7 @@ def _declare(lib):
         "lsp_last_error": (c_char_p, []),
         "lsp_device_info": (c_int, [POINTER(c_int), POINTER(c_int), POINTER(c_int)]),
         "lsp_barrier_probe": (c_int, [c_int, c_int, c_int, POINTER(c_int32), POINTER(c_uint32)]),
+        "lsp_stalled_step": (c_int, [S, c_float, c_int]),
         "lsp_create": (c_int, [POINTER(LspParams), c_int, POINTER(c_void_p)]),
         "lsp_destroy": (c_int, [S]),
         "lsp_set_params": (c_int, [S, POINTER(LspParams)]),
@@ -259,6 +260,7 @@ def _declare(lib):
         "lsp_batch_read_grid": (c_int, [c_void_p, c_int32, u32p, i32p, c_int64, u32p, c_int64]),
         "lsp_batch_read_state": (c_int, [c_void_p, fp, fp, fp, fp, i32p, c_int64]),
         "lsp_batch_write_state": (c_int, [c_void_p, fp, fp, fp, fp, i32p, c_int64]),
+        "lsp_batch_stalled_step": (c_int, [c_void_p, c_float, c_int32, c_int]),
         "lsp_batch_set_launch": (c_int, [c_void_p, c_int, c_int, c_int]),
         "lsp_batch_get_launch": (c_int, [c_void_p, POINTER(c_int), POINTER(c_int), POINTER(c_int), POINTER(c_int)]),
         "lsp_batch_autotune": (c_int, [c_void_p, c_float, c_int, POINTER(LspBatchTuning), POINTER(LspStepStats)]),

@@ -238,6 +238,10 @@ int lsp_step(lsp_solver* s, float dt, lsp_step_stats* stats)
 {
     return lsp::guard([&] { E(s).step(dt, stats); });
 }
+int lsp_stalled_step(lsp_solver* s, float dt, int barrier)
+{
+    return lsp::guard([&] { E(s).stalled_step(dt, barrier); });
+}
 int lsp_step_many(lsp_solver* s, float dt, int steps, lsp_step_stats* stats)
 {
     return lsp::guard([&] { E(s).step_many(dt, steps, stats); });

@@ -183,6 +183,11 @@ int lsp_batch_write_state(lsp_batch* b, const float* x, const float* v, const fl
     return lsp::guard([&] { B(b).write_state(x, v, v_half, v_half_old, first_step, n); });
 }
 
+int lsp_batch_stalled_step(lsp_batch* b, float dt, int32_t scene, int barrier)
+{
+    return lsp::guard([&] { B(b).stalled_step(dt, scene, barrier); });
+}
+
 int lsp_batch_set_launch(lsp_batch* b, int use_graph, int threads, int loop_blocks)
 {
     return lsp::guard([&] { B(b).set_launch(use_graph, threads, loop_blocks); });

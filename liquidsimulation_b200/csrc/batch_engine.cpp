@@ -411,6 +411,7 @@ bool BatchEngine::enqueue_small(int c)
     a.maxerr = maxerr();
     a.host = hstatus_;
     a.pcisph = pcisph_ ? 1 : 0;
+    a.stall = stall_;
     SmallBatchArgs sb{};
     sb.sp = dparams_.p;
     sb.blocks = small_blocks_.p;
@@ -489,8 +490,11 @@ void BatchEngine::run_once(int c)
     activate();
     // Occupancy queries stay outside the stream capture.
     const int grid = pcisph_ && !one_launch() ? loop_grid() : 0;
-    if (one_launch()) hstatus_[sc_.size()] = DevStatus{};   // the separate kernels' batch-wide entry
-    if (use_graph_ && graph_ok_ && !graph_[c]) {
+    // The batch-wide entry is the separate kernels', gave_up the one launch's.
+    if (one_launch()) hstatus_[sc_.size()] = DevStatus{};
+    for (size_t s = 0; s < sc_.size(); s++) hstatus_[s].gave_up = 0;
+    const bool graph = use_graph_ && !stall_.barrier;
+    if (graph && graph_ok_ && !graph_[c]) {
         cudaGraph_t g = nullptr;
         int l = 0;
         bool ok = true;
@@ -512,13 +516,25 @@ void BatchEngine::run_once(int c)
             graph_launches_[c] = l;
         }
     }
-    if (use_graph_ && graph_ok_ && graph_[c]) {
+    if (graph && graph_ok_ && graph_[c]) {
         CK(cudaGraphLaunch(graph_[c], stream_));
         launches_ += graph_launches_[c];
     } else {
         launches_ += enqueue_step(c, grid);
     }
     CK(cudaStreamSynchronize(stream_));
+    for (size_t s = 0; s < sc_.size(); s++)
+        if (hstatus_[s].gave_up) abandon_step(c);
+}
+
+void BatchEngine::abandon_step(int c)
+{
+    stepped_ = false;
+    CK(cudaMemsetAsync(hist_.p, 0, hist_.n * sizeof(uint32_t), stream_));
+    launch_slots_of_ids(pos_[c].p, slot_of_id_.p, n_, stream_);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(stream_));
+    throw Error(LSP_ERR_TIMEOUT, "a barrier of the batch's one-launch step gave up; the state is that before the step");
 }
 
 bool BatchEngine::run_checked()
@@ -546,6 +562,7 @@ void BatchEngine::finish_step(lsp_step_stats* stats)
 {
     const int S = (int)sc_.size();
     cur_ = 1 - cur_;
+    stepped_ = true;
     features_valid_ = features_on();
     uint32_t errors = hstatus_[S].error_flags;
     bool not_converged = false;
@@ -604,6 +621,22 @@ void BatchEngine::step(float dt, lsp_step_stats* stats)
     if (cols_dirty_) upload_colliders();
     run_checked();
     finish_step(stats);
+}
+
+void BatchEngine::stalled_step(float dt, int scene, int barrier)
+{
+    at(scene);
+    if (barrier < 1) throw Error(LSP_ERR_INVALID, "barrier must be >= 1");
+    if (!built_) build();
+    if (!one_launch()) throw Error(LSP_ERR_STATE, "the step does not run as one launch");
+    stall_ = {(uint32_t)barrier, kStallSpins, scene};
+    try {
+        step(dt, nullptr);
+    } catch (...) {
+        stall_ = {};
+        throw;
+    }
+    stall_ = {};
 }
 
 void BatchEngine::set_launch(int use_graph, int threads, int loop_blocks)
@@ -786,6 +819,7 @@ void BatchEngine::read_neighbors(int scene, int64_t* offsets, int32_t* index, in
     check_scene(scene);
     const Scene& s = sc_[scene];
     if (n != s.n || !offsets) throw Error(LSP_ERR_INVALID, "read_neighbors: bad arguments");
+    if (!stepped_) throw Error(LSP_ERR_STATE, "read_neighbors: no step has run");
     std::vector<float> counts(n);
     read_field(scene, LSP_FIELD_NEIGHBOR_COUNT, counts.data(), n);
     offsets[0] = 0;
@@ -812,6 +846,7 @@ void BatchEngine::read_grid(int scene, uint32_t* keys, int32_t* ids, int64_t n, 
     check_scene(scene);
     const Scene& s = sc_[scene];
     if (n != s.n) throw Error(LSP_ERR_INVALID, "read_grid: n must equal the scene's particle count");
+    if (!stepped_) throw Error(LSP_ERR_STATE, "read_grid: no step has run");
     activate();
     if (keys) {
         CK(cudaMemcpyAsync(keys, sorted_key_.p + s.base, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream_));

@@ -43,6 +43,7 @@ public:
 
     void set_launch(int use_graph, int threads, int loop_blocks);
     void get_launch(int* use_graph, int* threads, int* loop_blocks, int* graph_active) const;
+    void stalled_step(float dt, int scene, int barrier);
     void autotune(float dt, int repeats, lsp_batch_tuning* out, lsp_step_stats* stats);
 
     void timer_mark(int slot);
@@ -97,6 +98,8 @@ private:
     // Runs the step from parity cur_ until no list overflows; false if it still overflowed.
     bool run_checked();
     void finish_step(lsp_step_stats* stats);
+    // Engine::abandon_step for a step from parity c.
+    [[noreturn]] void abandon_step(int c);
     StepBuffers buffers(int c);
     BatchArgs args();
     void stage(size_t floats);
@@ -115,6 +118,8 @@ private:
     std::vector<Scene> sc_;
     std::vector<float4> init_pos_, init_vel_;   // host copies until the first step
     bool built_ = false, pcisph_ = true;
+    bool stepped_ = false;     // the lists and the grid are those of the last step
+    BarrierStall stall_{};     // of the next step
     int64_t n_ = 0, cells_ = 0;
     int cur_ = 0;
     int mstride_ = 0;

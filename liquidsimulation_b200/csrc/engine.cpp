@@ -2,7 +2,6 @@
 #include "engine.h"
 #include "mlp.cuh"
 #include "mlp_tc.cuh"
-#include "small_step.h"
 
 #include <algorithm>
 #include <cmath>
@@ -744,10 +743,24 @@ int grown_neighbor_capacity(int needed, int current)
 bool Engine::retry_step(int attempt)
 {
     CK(cudaStreamSynchronize(stream_));
+    if (hstatus_->gave_up) abandon_step();
     if (!(hstatus_->error_flags & kErrNeighborOverflow) || attempt >= 3) return false;
     cur_ = 1 - cur_;
     ensure_neighbors(grown_neighbor_capacity((int)hstatus_->max_neighbors, nbr_cap_));
     return true;
+}
+
+// A one-launch step may give up before the counts are cleared or the state is gathered, so its
+// output buffers hold nothing to go on from; those it read are untouched.
+void Engine::abandon_step()
+{
+    cur_ = 1 - cur_;
+    stepped_ = false;   // the lists and the grid are unfinished too
+    CK(cudaMemsetAsync(hist_.p, 0, hist_.n * sizeof(uint32_t), stream_));
+    launch_slots_of_ids(pos_[cur_].p, slot_of_id_.p, n_, stream_);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(stream_));
+    throw Error(LSP_ERR_TIMEOUT, "a grid barrier of the one-launch step gave up; the state is that before the step");
 }
 
 // Small scenes take the whole step in one launch (small_step_lanes has the rule); the per-class
@@ -767,6 +780,7 @@ bool Engine::run_small(const GridBuildArgs& g, const StepBuffers& b)
     a.maxerr = ctl_.p->maxerr;
     a.host = hstatus_;
     a.pcisph = pci ? 1 : 0;
+    a.stall = stall_;
     std::memset(hstatus_, 0, sizeof(DevStatus));
     if (!launch_small_step(a, lanes, stream_)) {
         cudaGetLastError();   // the device refused the cooperative launch
@@ -825,6 +839,10 @@ void Engine::run_step(float dt, lsp_step_stats* st)
             if (retry_step(attempt)) continue;
             break;
         }
+        if (stall_.barrier) {
+            cur_ = 1 - cur_;
+            throw Error(LSP_ERR_STATE, "the step does not run as one launch");
+        }
         timed(LSP_PROF_GRID_SORT, [&] { return launch_grid_keys(g, stream_); });
         timed(LSP_PROF_GRID_SCAN, [&] { return launch_grid_scan(g, stream_); });
         timed(LSP_PROF_GRID_SCATTER, [&] { return launch_grid_scatter(g, stream_); });
@@ -879,6 +897,19 @@ void Engine::run_step(float dt, lsp_step_stats* st)
 }
 
 void Engine::step(float dt, lsp_step_stats* st) { run_step(dt, st); }
+
+void Engine::stalled_step(float dt, int barrier)
+{
+    if (barrier < 1) throw Error(LSP_ERR_INVALID, "barrier must be >= 1");
+    stall_ = {(uint32_t)barrier, kStallSpins, 0};
+    try {
+        run_step(dt, nullptr);
+    } catch (...) {
+        stall_ = {};
+        throw;
+    }
+    stall_ = {};
+}
 
 void Engine::step_many(float dt, int steps, lsp_step_stats* st)
 {

@@ -14,6 +14,7 @@
 #include "host_view.h"
 #include "lsp_kernels.h"
 #include "mlp_model.h"
+#include "small_step.h"
 
 namespace lsp {
 
@@ -94,6 +95,7 @@ public:
     void write_history(const float* in, int64_t n);
 
     void step(float dt, lsp_step_stats* st);
+    void stalled_step(float dt, int barrier);
     void step_many(float dt, int steps, lsp_step_stats* st);
     void synchronize();
 
@@ -141,6 +143,8 @@ private:
     void ensure_neighbors(int cap);
     void upload_colliders();
     void run_step(float dt, lsp_step_stats* st);
+    // After a one-launch step that gave up: the solver as it was before the step, and the error.
+    [[noreturn]] void abandon_step();
     // Waits for a step; true when it is to be redone. The one-launch step of a small scene; false when this step runs as separate kernels.
     bool retry_step(int attempt);
     bool run_small(const GridBuildArgs& g, const StepBuffers& b);
@@ -190,6 +194,7 @@ private:
     DevStatus* hstatus_ = nullptr;   // pinned
     DevArray<float> stage_;
     HostStage hstage_;
+    BarrierStall stall_{};   // of the next step
 
     // Launch bracketing for the per-class profile.
     template <typename F>

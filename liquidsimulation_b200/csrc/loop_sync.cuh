@@ -54,15 +54,16 @@ static __device__ __forceinline__ bool barrier_wait(LoopSync* sy, DevStatus* st,
 // one): the e-th barrier of a launch is over when the counter reaches e times the number of blocks,
 // so one reduction per block and barrier is all the traffic; epoch counts the barriers this block
 // has passed. The arrival releases and the last poll acquires at device scope; block barriers on
-// both sides carry that to the other threads.
-static __device__ bool blocks_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch, uint32_t blocks)
+// both sides carry that to the other threads. missing: arrivals waited for that do not come.
+static __device__ bool blocks_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch, uint32_t blocks, uint32_t missing = 0,
+                                      unsigned long long spin_limit = kBarrierSpinLimit)
 {
     __shared__ int ok;
-    const uint32_t target = ++epoch * blocks;
+    const uint32_t target = ++epoch * blocks + missing;
     __syncthreads();
     if (threadIdx.x == 0) {
         add_release(&sy->count);
-        ok = barrier_wait(sy, st, target, kBarrierSpinLimit) ? 1 : 0;
+        ok = barrier_wait(sy, st, target, spin_limit) ? 1 : 0;
     }
     __syncthreads();
     return ok != 0;

@@ -55,7 +55,7 @@ struct DevStatus {
     uint32_t np_unsafe;         // a start-of-step position, velocity or density left the range
                                 // where the non-pressure pass divides with div_by
     uint32_t any_first;         // a particle is on its first step
-    uint32_t pad;
+    uint32_t gave_up;           // host copy only: a barrier of the one-launch step gave up (last word)
 };
 
 struct DevParams {

@@ -153,6 +153,8 @@ void launch_gather_field(const void* src, int comps, int w_as_flag, const int32_
 // Positions and velocities of a field read-back in one launch.
 void launch_gather_particles(const float4* pos, const float4* vel, const int32_t* slot_of_id, float* x, float* v,
                              int64_t n, cudaStream_t s);
+// slot_of_id of n particles from the ids in their positions' w.
+void launch_slots_of_ids(const float4* pos, int32_t* slot_of_id, int64_t n, cudaStream_t s);
 void launch_gather_count(const int32_t* count, const int32_t* slot_of_id, float* out, int64_t n, cudaStream_t s);
 // Scatters caller-order state (x, v, v_half, v_half_old, first) into device slots.
 void launch_scatter_state(const float* x, const float* v, const float* half, const float* old,

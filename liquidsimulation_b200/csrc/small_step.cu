@@ -25,6 +25,7 @@
 #include "scan_ops.cuh"
 #include "small_step.h"
 
+#include <cstddef>
 #include <mutex>
 
 namespace lsp {
@@ -51,6 +52,7 @@ struct SceneBlocks {
     uint32_t* maxerr;
     uint32_t* tile_sums;
     DevStatus* host;
+    BarrierStall stall;
 };
 
 // The step of one scene by its blocks. kBatch: the scene's particles start at slot P.base and its
@@ -70,11 +72,21 @@ __device__ __forceinline__ void small_step(const DevParams& P, const GridBuildAr
     const int n = P.n;
     const int base = kBatch ? P.base : 0;
     uint32_t epoch = 0;
-    // A barrier that gave up tells the host at once: the status copy at the end is not reached.
+    // A barrier that gave up tells the host in a word of its own, which the status copy at the end of
+    // a block that got further leaves alone. The step's buffers are unfinished then, and the counts
+    // may not be cleared: the host goes back to the buffers that the step read (abandon_step).
     auto barrier = [&]() {
-        const bool ok = blocks_barrier(own_blocks.sync, st, epoch, (uint32_t)blocks);
-        if (!ok && threadIdx.x == 0) own_blocks.host->error_flags = kErrTimeout;
+        const BarrierStall& stall = own_blocks.stall;
+        const bool ok = stall.barrier ? blocks_barrier(own_blocks.sync, st, epoch, (uint32_t)blocks,
+                                                       epoch + 1 == stall.barrier ? 1u : 0u, stall.spins)
+                                      : blocks_barrier(own_blocks.sync, st, epoch, (uint32_t)blocks);
+        if (!ok && threadIdx.x == 0) own_blocks.host->gave_up = 1u;
         return ok;
+    };
+    auto report = [&]() {
+        static_assert(offsetof(DevStatus, gave_up) == sizeof(DevStatus) - sizeof(uint32_t), "the last word");
+        for (int w = 0; w < (int)(offsetof(DevStatus, gave_up) / sizeof(uint32_t)); w++)
+            reinterpret_cast<uint32_t*>(own_blocks.host)[w] = reinterpret_cast<const uint32_t*>(st)[w];
     };
     for (int w = threadIdx.x; w < P.ncoll * (int)(sizeof(Collider) / 4); w += blockDim.x)
         reinterpret_cast<uint32_t*>(cols)[w] = reinterpret_cast<const uint32_t*>(b.colliders + P.coll_off)[w];
@@ -212,7 +224,7 @@ __device__ __forceinline__ void small_step(const DevParams& P, const GridBuildAr
         const float pres = b.pres[i];
         if (!barrier()) return;   // the positions are read by other groups until here
         integrate(F, pres);
-        if (tid == 0) *own_blocks.host = *st;
+        if (tid == 0) report();
         return;
     }
 
@@ -261,7 +273,7 @@ __device__ __forceinline__ void small_step(const DevParams& P, const GridBuildAr
                 st->max_err_bits = me;
                 st->warm_used = 0;
                 st->last_k = k;
-                *own_blocks.host = *st;
+                report();
             }
             return;
         }
@@ -275,7 +287,8 @@ template <int L>
 __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
 {
     small_step<L, false>(a.g.P, a.g, a.b, a.ppos_alt, a.pcisph,
-                         {(int)blockIdx.x, (int)gridDim.x, reinterpret_cast<LoopSync*>(a.sync), a.maxerr, a.g.tile_sums, a.host});
+                         {(int)blockIdx.x, (int)gridDim.x, reinterpret_cast<LoopSync*>(a.sync), a.maxerr, a.g.tile_sums, a.host,
+                          a.stall});
 }
 
 // The same for a batch of scenes in one launch. A scene has blocks and a barrier of its own, so it
@@ -297,7 +310,8 @@ __global__ void __launch_bounds__(kBatchThreads, kMaxThreads / kBatchThreads) k_
     b.tables += (size_t)me.scene * sb.table_stride;
     small_step<L, true>(P, g, b, a.ppos_alt, a.pcisph,
                         {(int)blockIdx.x - me.first, me.count, reinterpret_cast<LoopSync*>(a.sync) + me.scene,
-                         a.maxerr + (size_t)me.scene * sb.mstride, g.tile_sums + me.first, a.host + me.scene});
+                         a.maxerr + (size_t)me.scene * sb.mstride, g.tile_sums + me.first, a.host + me.scene,
+                         me.scene == a.stall.scene ? a.stall : BarrierStall{}});
 }
 
 // ------------------------------------------------------------------ launch

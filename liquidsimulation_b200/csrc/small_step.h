@@ -7,6 +7,14 @@
 
 namespace lsp {
 
+// A step made to give up (lsp_stalled_step): its `barrier`-th barrier (from 1; 0: none) of scene
+// `scene` waits for an arrival that does not come, `spins` polls long.
+struct BarrierStall {
+    uint32_t barrier, spins;
+    int scene;
+};
+constexpr uint32_t kStallSpins = 1u << 14;   // some 10 ms
+
 struct SmallStepArgs {
     GridBuildArgs g;
     StepBuffers b;       // the buffers the grid build gathers into
@@ -15,6 +23,7 @@ struct SmallStepArgs {
     uint32_t* maxerr;    // max_it zeroed words
     DevStatus* host;     // pinned: the step's status, written at its end
     int pcisph;
+    BarrierStall stall;
 };
 
 // Largest grid box of the one-launch step, whose blocks scan a contiguous share of the cells each:

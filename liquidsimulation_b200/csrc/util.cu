@@ -132,6 +132,17 @@ __global__ void k_gather_count(const int32_t* __restrict__ count, const int32_t*
     out[id] = (float)count[slot_of_id[id]];
 }
 
+__global__ void k_slots_of_ids(const float4* __restrict__ pos, int32_t* __restrict__ slot_of_id, int64_t n)
+{
+    const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot < n) slot_of_id[id_of(pos[slot])] = (int32_t)slot;
+}
+
+void launch_slots_of_ids(const float4* pos, int32_t* slot_of_id, int64_t n, cudaStream_t s)
+{
+    if (n) k_slots_of_ids<<<blocks_for(n), kThreads, 0, s>>>(pos, slot_of_id, n);
+}
+
 void launch_gather_field(const void* src, int comps, int mode, const int32_t* slot_of_id, float* out, int64_t n,
                          cudaStream_t s)
 {
