@@ -27,9 +27,10 @@ GetAttributes pointer_attributes()
 }
 }  // namespace
 
-void* pinned_view(const void* p, size_t bytes)
+void* pinned_view(const void* p, size_t bytes, bool* host)
 {
     const GetAttributes get = pointer_attributes();
+    *host = false;
     if (!get || !p) return nullptr;
     unsigned type = 0;
     CUdeviceptr dev = 0, start = 0;
@@ -39,6 +40,7 @@ void* pinned_view(const void* p, size_t bytes)
     void* to[4] = {&type, &dev, &start, &size};
     const CUdeviceptr a = (CUdeviceptr)(uintptr_t)p;
     if (get(4, what, to, a) != CUDA_SUCCESS) return nullptr;
+    *host = type == 0 || type == CU_MEMORYTYPE_HOST;   // 0: not known to the driver, pageable
     if (type != CU_MEMORYTYPE_HOST || !dev) return nullptr;
     // The whole array lies in the allocation (its start is reported in the address space of p or of dev).
     const bool inside = (a >= start && a - start <= size && bytes <= size - (a - start)) ||
@@ -70,11 +72,14 @@ char* HostStage::get(size_t bytes)
 
 void HostTransfer::add(const void* p, size_t bytes)
 {
-    e_[n_++] = Entry{const_cast<void*>(p), bytes, pinned_view(p, bytes), nullptr};
+    bool host;
+    e_[n_++] = Entry{const_cast<void*>(p), bytes, pinned_view(p, bytes, &host), nullptr};
+    host_ = host_ && host;
 }
 
 bool HostTransfer::ready()
 {
+    if (!host_) return false;
     auto padded = [](size_t b) { return (b + 127) / 128 * 128; };
     size_t need = 0;
     for (int k = 0; k < n_; k++)

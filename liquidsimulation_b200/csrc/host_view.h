@@ -8,9 +8,10 @@
 
 namespace lsp {
 
-// Device address of the host memory [p, p + bytes) when all of it is one pinned, mapped allocation;
-// null otherwise.
-void* pinned_view(const void* p, size_t bytes);
+// Device address of the memory [p, p + bytes) when all of it is one pinned, mapped allocation of the
+// host; null otherwise. *host says whether the host may touch p: false for device memory, which
+// callers may pass as well, and when the driver cannot be asked.
+void* pinned_view(const void* p, size_t bytes, bool* host);
 
 // Pinned memory of a solver, kept between calls and at most kMaxBytes.
 class HostStage {
@@ -32,7 +33,8 @@ public:
     // to_device: the caller's data is read (staged arrays are copied in), else written.
     HostTransfer(HostStage& stage, bool to_device) : stage_(stage), in_(to_device) {}
     void add(const void* p, size_t bytes);
-    // False when some array can be reached neither way; the device addresses are view(k).
+    // False when some array can be reached neither way (device memory goes by copies); the device
+    // addresses are view(k).
     bool ready();
     void* view(int k) const { return e_[k].dev; }
     void finish();
@@ -47,6 +49,7 @@ private:
     };
     HostStage& stage_;
     bool in_;
+    bool host_ = true;   // every array is the host's
     int n_ = 0;
     Entry e_[kMost];
 };
