@@ -222,6 +222,14 @@ __device__ __forceinline__ int group_neighbors(const Group<L>& g, const DevParam
     return cnt;   // of the first lane where neighbors_one ran
 }
 
+// Whether the word is set, the same in every lane: the walks' two instances are full of warp-wide
+// operations, so a warp has to take one of them as a whole, and another block may be setting the
+// word (div_unsafe: predict_motion of a block that is a pass ahead). Both give the same bits then.
+__device__ __forceinline__ bool any_lane_sees(const uint32_t* word)
+{
+    return __any_sync(kFullWarp, *(const volatile uint32_t*)word != 0u);
+}
+
 // The non-pressure force of particle i (nonpressure_one without the warm-start feature), in every lane.
 template <int L, bool kExactDiv>
 __device__ __forceinline__ V3 group_nonpressure_walk(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i,
@@ -256,7 +264,7 @@ template <int L>
 __device__ __forceinline__ V3 group_nonpressure(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i, V3 xi,
                                                 V3 vi, float rhoi, const HeldList<L>& list)
 {
-    return P.exact_tables && *(const volatile uint32_t*)&b.status->np_unsafe == 0u
+    return P.exact_tables && !any_lane_sees(&b.status->np_unsafe)
                ? group_nonpressure_walk<L, true>(g, P, b, i, xi, vi, rhoi, list)
                : group_nonpressure_walk<L, false>(g, P, b, i, xi, vi, rhoi, list);
 }
@@ -291,9 +299,9 @@ __device__ __forceinline__ V3 group_pci_force(const Group<L>& g, const DevParams
                                               const float4* ppos, V3 xi, float tf, float rhoi, const HeldList<L>& list)
 {
     return pci_pressure_force(P, rhoi,
-                              *(const volatile uint32_t*)&b.status->div_unsafe == 0u
-                                  ? group_pci_force_walk<L, true>(g, P, b, i, ppos, xi, tf, list)
-                                  : group_pci_force_walk<L, false>(g, P, b, i, ppos, xi, tf, list));
+                              any_lane_sees(&b.status->div_unsafe)
+                                  ? group_pci_force_walk<L, false>(g, P, b, i, ppos, xi, tf, list)
+                                  : group_pci_force_walk<L, true>(g, P, b, i, ppos, xi, tf, list));
 }
 // All forces of SPH of particle i (sph_forces_walk), in every lane. In one walk instead of two, each with
 // its fetches and block of ordered sums, a step of 12,000 particles takes 1.6 us less.
@@ -341,7 +349,7 @@ template <int L>
 __device__ __forceinline__ V3 group_sph_forces(const Group<L>& g, const DevParams& P, const StepBuffers& b, int i, V3 xi,
                                                V3 vi, float rhoi, const HeldList<L>& list)
 {
-    return P.exact_tables && *(const volatile uint32_t*)&b.status->np_unsafe == 0u
+    return P.exact_tables && !any_lane_sees(&b.status->np_unsafe)
                ? group_sph_walk<L, true>(g, P, b, i, xi, vi, rhoi, list)
                : group_sph_walk<L, false>(g, P, b, i, xi, vi, rhoi, list);
 }
