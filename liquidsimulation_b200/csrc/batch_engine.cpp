@@ -629,7 +629,7 @@ void BatchEngine::stalled_step(float dt, int scene, int barrier)
     if (barrier < 1) throw Error(LSP_ERR_INVALID, "barrier must be >= 1");
     if (!built_) build();
     if (!one_launch()) throw Error(LSP_ERR_STATE, "the step does not run as one launch");
-    stall_ = {(uint32_t)barrier, kStallSpins, scene};
+    stall_ = {(uint32_t)barrier, scene};
     try {
         step(dt, nullptr);
     } catch (...) {

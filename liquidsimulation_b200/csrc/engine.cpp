@@ -901,7 +901,7 @@ void Engine::step(float dt, lsp_step_stats* st) { run_step(dt, st); }
 void Engine::stalled_step(float dt, int barrier)
 {
     if (barrier < 1) throw Error(LSP_ERR_INVALID, "barrier must be >= 1");
-    stall_ = {(uint32_t)barrier, kStallSpins, 0};
+    stall_ = {(uint32_t)barrier, 0};
     try {
         run_step(dt, nullptr);
     } catch (...) {

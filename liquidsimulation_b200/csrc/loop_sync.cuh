@@ -9,6 +9,7 @@
 namespace lsp {
 
 constexpr unsigned long long kBarrierSpinLimit = 1ull << 25;
+constexpr unsigned long long kStallSpinLimit = 1ull << 14;   // some 10 ms
 
 struct LoopSync {
     uint32_t count;   // barrier arrivals since the launch
@@ -54,16 +55,16 @@ static __device__ __forceinline__ bool barrier_wait(LoopSync* sy, DevStatus* st,
 // one): the e-th barrier of a launch is over when the counter reaches e times the number of blocks,
 // so one reduction per block and barrier is all the traffic; epoch counts the barriers this block
 // has passed. The arrival releases and the last poll acquires at device scope; block barriers on
-// both sides carry that to the other threads. missing: arrivals waited for that do not come.
-static __device__ bool blocks_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch, uint32_t blocks, uint32_t missing = 0,
-                                      unsigned long long spin_limit = kBarrierSpinLimit)
+// both sides carry that to the other threads. stalled: the barrier (from 1) that waits, for a short time, for
+// an arrival that does not come, 0: none.
+static __device__ bool blocks_barrier(LoopSync* sy, DevStatus* st, uint32_t& epoch, uint32_t blocks, uint32_t stalled = 0)
 {
     __shared__ int ok;
-    const uint32_t target = ++epoch * blocks + missing;
+    const uint32_t target = ++epoch * blocks + (stalled && epoch == stalled ? 1u : 0u);
     __syncthreads();
     if (threadIdx.x == 0) {
         add_release(&sy->count);
-        ok = barrier_wait(sy, st, target, spin_limit) ? 1 : 0;
+        ok = barrier_wait(sy, st, target, stalled ? kStallSpinLimit : kBarrierSpinLimit) ? 1 : 0;
     }
     __syncthreads();
     return ok != 0;

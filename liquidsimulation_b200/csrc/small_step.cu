@@ -52,7 +52,7 @@ struct SceneBlocks {
     uint32_t* maxerr;
     uint32_t* tile_sums;
     DevStatus* host;
-    BarrierStall stall;
+    uint32_t stalled;   // BarrierStall::barrier of this scene
 };
 
 // The step of one scene by its blocks. kBatch: the scene's particles start at slot P.base and its
@@ -76,17 +76,19 @@ __device__ __forceinline__ void small_step(const DevParams& P, const GridBuildAr
     // a block that got further leaves alone. The step's buffers are unfinished then, and the counts
     // may not be cleared: the host goes back to the buffers that the step read (abandon_step).
     auto barrier = [&]() {
-        const BarrierStall& stall = own_blocks.stall;
-        const bool ok = stall.barrier ? blocks_barrier(own_blocks.sync, st, epoch, (uint32_t)blocks,
-                                                       epoch + 1 == stall.barrier ? 1u : 0u, stall.spins)
-                                      : blocks_barrier(own_blocks.sync, st, epoch, (uint32_t)blocks);
+        const bool ok = blocks_barrier(own_blocks.sync, st, epoch, (uint32_t)blocks, own_blocks.stalled);
         if (!ok && threadIdx.x == 0) own_blocks.host->gave_up = 1u;
         return ok;
     };
+    // The status over PCIe, in as few stores as leave that word out.
     auto report = [&]() {
-        static_assert(offsetof(DevStatus, gave_up) == sizeof(DevStatus) - sizeof(uint32_t), "the last word");
-        for (int w = 0; w < (int)(offsetof(DevStatus, gave_up) / sizeof(uint32_t)); w++)
-            reinterpret_cast<uint32_t*>(own_blocks.host)[w] = reinterpret_cast<const uint32_t*>(st)[w];
+        static_assert(sizeof(DevStatus) == 64 && offsetof(DevStatus, gave_up) == 60, "gave_up is the last word");
+        const uint32_t* from = reinterpret_cast<const uint32_t*>(st);
+        uint4* to = reinterpret_cast<uint4*>(own_blocks.host);
+#pragma unroll
+        for (int q = 0; q < 3; q++) to[q] = make_uint4(from[4 * q], from[4 * q + 1], from[4 * q + 2], from[4 * q + 3]);
+        *reinterpret_cast<uint2*>(to + 3) = make_uint2(from[12], from[13]);
+        reinterpret_cast<uint32_t*>(to)[14] = from[14];
     };
     for (int w = threadIdx.x; w < P.ncoll * (int)(sizeof(Collider) / 4); w += blockDim.x)
         reinterpret_cast<uint32_t*>(cols)[w] = reinterpret_cast<const uint32_t*>(b.colliders + P.coll_off)[w];
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) k_small_step(SmallStepArgs a)
 {
     small_step<L, false>(a.g.P, a.g, a.b, a.ppos_alt, a.pcisph,
                          {(int)blockIdx.x, (int)gridDim.x, reinterpret_cast<LoopSync*>(a.sync), a.maxerr, a.g.tile_sums, a.host,
-                          a.stall});
+                          a.stall.barrier});
 }
 
 // The same for a batch of scenes in one launch. A scene has blocks and a barrier of its own, so it
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kBatchThreads, kMaxThreads / kBatchThreads) k_
     small_step<L, true>(P, g, b, a.ppos_alt, a.pcisph,
                         {(int)blockIdx.x - me.first, me.count, reinterpret_cast<LoopSync*>(a.sync) + me.scene,
                          a.maxerr + (size_t)me.scene * sb.mstride, g.tile_sums + me.first, a.host + me.scene,
-                         me.scene == a.stall.scene ? a.stall : BarrierStall{}});
+                         me.scene == a.stall.scene ? a.stall.barrier : 0u});
 }
 
 // ------------------------------------------------------------------ launch

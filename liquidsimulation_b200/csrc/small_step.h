@@ -8,12 +8,11 @@
 namespace lsp {
 
 // A step made to give up (lsp_stalled_step): its `barrier`-th barrier (from 1; 0: none) of scene
-// `scene` waits for an arrival that does not come, `spins` polls long.
+// `scene` waits for an arrival that does not come.
 struct BarrierStall {
-    uint32_t barrier, spins;
+    uint32_t barrier;
     int scene;
 };
-constexpr uint32_t kStallSpins = 1u << 14;   // some 10 ms
 
 struct SmallStepArgs {
     GridBuildArgs g;
