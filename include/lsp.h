@@ -362,9 +362,10 @@ int lsp_batch_set_launch(lsp_batch* b, int use_graph, int threads, int loop_bloc
 int lsp_batch_get_launch(const lsp_batch* b, int* use_graph, int* threads, int* loop_blocks, int* graph_active);
 /* Autotuner: runs the next step under each candidate launch shape (particles per block x
  * persistent-kernel blocks), re-running that same step from the same state `repeats` times
- * per candidate, keeps the fastest shape (or, when no shape is faster, what the default shape
- * runs), and leaves the batch advanced by exactly that one step (results do not depend on the
- * shape). result and stats may be NULL. */
+ * per candidate, keeps the fastest shape, and leaves the batch advanced by exactly that one step
+ * (results do not depend on the shape). The default shape (256, 0) with what runs there is a
+ * candidate too, so lsp_batch_set_launch with the chosen shape gives the same again. result and
+ * stats may be NULL. */
 int lsp_batch_autotune(lsp_batch* b, float dt, int repeats, lsp_batch_tuning* result, lsp_step_stats* stats);
 /* Learned warm start for the scenes of a PCISPH batch (LSP_WARM_ZERO, LSP_WARM_MLP or
  * LSP_WARM_AUTO; AUTO switches each scene on by itself, at that scene's

@@ -677,8 +677,8 @@ float BatchEngine::time_step(int repeats, cudaEvent_t e0, cudaEvent_t e1)
     return best;
 }
 
-// Candidates: every supported block size, with the persistent kernel at full residency and
-// at half of it. Each candidate runs the same step (from the same pre-step buffers) once to
+// Candidates: the default shape with the choices made for it (one_launch, loop_threads), then every
+// supported block size, with the persistent kernel at full residency and at half of it. Each candidate runs the same step (from the same pre-step buffers) once to
 // capture its graph, then `repeats` timed times; the state only advances at the end.
 void BatchEngine::autotune(float dt, int repeats, lsp_batch_tuning* out, lsp_step_stats* stats)
 {
@@ -694,10 +694,10 @@ void BatchEngine::autotune(float dt, int repeats, lsp_batch_tuning* out, lsp_ste
         int threads, blocks;
         float ms;
     };
-    std::vector<Cand> cands;
+    std::vector<Cand> cands{{256, 0, 0.f}};
     for (int T : {128, 256, 512, 1024}) {
         if (!pcisph_) {
-            cands.push_back({T, 0, 0.f});
+            if (T != 256) cands.push_back({T, 0, 0.f});
             continue;
         }
         const int most = batch_loop_max_blocks(T, (int)sc_.size());
@@ -706,27 +706,23 @@ void BatchEngine::autotune(float dt, int repeats, lsp_batch_tuning* out, lsp_ste
         const int per_sm = most / std::max(sms, 1);
         if (per_sm >= 2) cands.push_back({T, (per_sm / 2) * sms, 0.f});
     }
-    if (cands.empty()) throw Error(LSP_ERR_CUDA, "no launch shape can run the batch's persistent kernel");
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     const bool graph = use_graph_;
+    const Cand before{threads_, loop_blocks_, 0.f};
     size_t best = 0;
     try {
         for (size_t k = 0; k < cands.size(); k++) {
             set_launch(graph ? 1 : 0, cands[k].threads, cands[k].blocks);
-            shaped_ = true;
             cands[k].ms = time_step(repeats, e0, e1);
             if (cands[k].ms < cands[best].ms) best = k;
         }
         set_launch(graph ? 1 : 0, cands[best].threads, cands[best].blocks);
-        // The choices made without a shape (one_launch, loop_threads) stay when no shape is faster.
-        shaped_ = false;
-        shaped_ = time_step(repeats, e0, e1) > cands[best].ms;
-        drop_graphs();
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
+        set_launch(graph ? 1 : 0, before.threads, before.blocks);
         throw;
     }
     cudaEventDestroy(e0);
