@@ -341,7 +341,11 @@ void BatchEngine::drop_graphs()
 // Unless a shape was chosen, the loop of a batch of large scenes runs in the single scene's blocks, one
 // of 1024 threads per SM: its grid barriers have a quarter of the arrivals. Two steps of 64 scenes of
 // 21,000 particles on average with their transfers: 6.34 ms in four blocks of 256 per SM, 6.22 ms so.
-// Scenes below eight blocks would leave more than a sixteenth of their blocks' threads idle.
+// The line is at a mean of eight blocks a scene, where the last blocks leave about a sixteenth of the
+// threads idle; it holds for unequal scenes as well, since a small scene's block costs little beside
+// the barriers. Three steps with their transfers, 256 -> 1024: one scene of 600,000 particles with 60
+// of 100 2.71 -> 2.63 ms, one of 900,000 with 100 of 27 3.87 -> 3.73, one of 300,000 with 30 of 1,100
+// 1.62 -> 1.59, one of 120,000 with 13 of 1,000 0.78 -> 0.75.
 int BatchEngine::loop_threads() const
 {
     return !shaped_ && n_ >= (int64_t)sc_.size() * 8 * 1024 ? 1024 : threads_;
