@@ -233,9 +233,10 @@ __device__ void block_scan_counts(int* a, int n, int* warp_sums)
     __syncthreads();
 }
 
+// 1024 threads per SM at 64 registers, in one block by default where the scenes are large
+// (BatchEngine::loop_threads), else in four of 256: faster than the unconstrained allocation (about 112
+// registers, 512 threads per SM).
 template <int T>
-// 64 registers (four 256-thread blocks per SM): measured faster than the unconstrained
-// allocation (about 112 registers, two blocks per SM) despite a few spilled words.
 __global__ void __launch_bounds__(T, 1024 / T) kb_pci_loop(BatchArgs a, StepBuffers b, BatchLoopArgs l)
 {
     extern __shared__ int dyn[];

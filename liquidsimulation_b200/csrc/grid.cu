@@ -202,18 +202,6 @@ int launch_grid_order(const GridBuildArgs& a, cudaStream_t s)
     return launches;
 }
 
-int launch_grid_sort(const GridBuildArgs& a, cudaStream_t s)
-{
-    const int T = 256;
-    const DevParams& P = a.P;
-    int launches = 0;
-    if (P.n > 0) {
-        launch_chained(k_keys_hist, blocks_for(P.n, T), T, 0, s, P, a.pos_in, a.key, a.slot, a.hist, a.status);
-        launches++;
-    }
-    return launches + launch_grid_order(a, s);
-}
-
 int launch_neighbors(const GridBuildArgs& a, cudaStream_t s)
 {
     const int T = 128;

@@ -28,6 +28,7 @@ constexpr size_t group_smem(int threads, int lanes)
 
 template <int L>
 struct Group {
+    static_assert(L >= 2 && L <= 16 && (L & (L - 1)) == 0, "part of a warp");
     int lane;     // this thread's lane in its group
     float* row;   // the group's rows of terms in shared memory
     __device__ __forceinline__ Group(float* smem)
@@ -190,7 +191,7 @@ __device__ __forceinline__ int group_neighbors(const Group<L>& g, const DevParam
         cnt += __shfl_sync(kFullWarp, upto, L - 1, L);
     }
     plain = plain && cnt <= kGroupList;
-    const uint32_t lanes = (L == 32 ? kFullWarp : (1u << (L & 31)) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
+    const uint32_t lanes = ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
     const bool fast = (__ballot_sync(kFullWarp, !plain) & lanes) == 0u;
     if (fast) {
 #pragma unroll

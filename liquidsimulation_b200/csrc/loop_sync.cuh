@@ -13,9 +13,8 @@ constexpr unsigned long long kStallSpinLimit = 1ull << 14;   // some 10 ms
 
 struct LoopSync {
     uint32_t count;   // barrier arrivals since the launch
-    uint32_t unused;
     uint32_t abort;
-    uint32_t pad;
+    uint32_t pad[2];
 };
 
 static __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *(const volatile uint32_t*)p; }

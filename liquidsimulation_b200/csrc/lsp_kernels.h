@@ -102,13 +102,11 @@ __host__ __device__ inline int64_t scan_entries(int64_t n) { return (n + 7) / 8 
 inline int64_t scan_tiles(int64_t n) { return (scan_entries(n) + 2047) / 2048; }
 
 // All return the number of kernels launched.
-int launch_grid_sort(const GridBuildArgs& a, cudaStream_t s);
 // The part of the grid build after the keys: scan of a.hist (a.P.cells + 1 counters) into
 // the cell table, scatter, rank by caller id and gather of a.P.n particles.
 int launch_grid_order(const GridBuildArgs& a, cudaStream_t s);
 int launch_neighbors(const GridBuildArgs& a, cudaStream_t s);
-// The grid build's four passes one by one (launch_grid_sort = all four in order): cell keys
-// and histogram, scan into the cell table, scatter, rank + gather.
+// The grid build's four passes one by one: cell keys and histogram, scan into the cell table, scatter, rank + gather.
 int launch_grid_keys(const GridBuildArgs& a, cudaStream_t s);
 int launch_grid_scan(const GridBuildArgs& a, cudaStream_t s);
 int launch_grid_scatter(const GridBuildArgs& a, cudaStream_t s);
