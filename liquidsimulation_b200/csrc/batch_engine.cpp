@@ -331,11 +331,11 @@ void BatchEngine::build_items()
 
 void BatchEngine::drop_graphs()
 {
-    for (int c = 0; c < 2; c++) {
-        if (graph_[c]) cudaGraphExecDestroy(graph_[c]);
-        graph_[c] = nullptr;
-        graph_launches_[c] = 0;
-    }
+    for (auto& route : graph_)
+        for (Graph& g : route) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = Graph{};
+        }
 }
 
 // Unless a shape was chosen, the loop of a batch of large scenes runs in the single scene's blocks, one
@@ -498,7 +498,8 @@ void BatchEngine::run_once(int c)
     if (one_launch()) hstatus_[sc_.size()] = DevStatus{};
     for (size_t s = 0; s < sc_.size(); s++) hstatus_[s].gave_up = 0;
     const bool graph = use_graph_ && !stall_.barrier;
-    if (graph && graph_ok_ && !graph_[c]) {
+    Graph& kept = graph_[one_launch() ? 1 : 0][c];
+    if (graph && graph_ok_ && !kept.exec) {
         cudaGraph_t g = nullptr;
         int l = 0;
         bool ok = true;
@@ -516,13 +517,12 @@ void BatchEngine::run_once(int c)
             cudaGetLastError();   // capture refused: the step runs as direct launches
             graph_ok_ = false;
         } else {
-            graph_[c] = ex;
-            graph_launches_[c] = l;
+            kept = {ex, l};
         }
     }
-    if (graph && graph_ok_ && graph_[c]) {
-        CK(cudaGraphLaunch(graph_[c], stream_));
-        launches_ += graph_launches_[c];
+    if (graph && graph_ok_ && kept.exec) {
+        CK(cudaGraphLaunch(kept.exec, stream_));
+        launches_ += kept.launches;
     } else {
         launches_ += enqueue_step(c, grid);
     }
@@ -623,6 +623,9 @@ void BatchEngine::step(float dt, lsp_step_stats* stats)
     activate();
     if (params_dirty_ || dt != dt_) upload_params(dt);
     if (cols_dirty_) upload_colliders();
+    const StepInFlight in_flight(dev_, threads_in_flight());
+    fits_ = in_flight.fits();
+    if (stall_.barrier && !one_launch()) throw Error(LSP_ERR_STATE, "the step does not run as one launch");
     run_checked();
     finish_step(stats);
 }
@@ -631,8 +634,6 @@ void BatchEngine::stalled_step(float dt, int scene, int barrier)
 {
     at(scene);
     if (barrier < 1) throw Error(LSP_ERR_INVALID, "barrier must be >= 1");
-    if (!built_) build();
-    if (!one_launch()) throw Error(LSP_ERR_STATE, "the step does not run as one launch");
     stall_ = {(uint32_t)barrier, scene};
     try {
         step(dt, nullptr);
@@ -662,7 +663,11 @@ void BatchEngine::get_launch(int* use_graph, int* threads, int* loop_blocks, int
     if (use_graph) *use_graph = use_graph_ ? 1 : 0;
     if (threads) *threads = threads_;
     if (loop_blocks) *loop_blocks = loop_blocks_;
-    if (graph_active) *graph_active = (use_graph_ && graph_ok_ && (graph_[0] || graph_[1])) ? 1 : 0;
+    if (graph_active) *graph_active = 0;
+    if (graph_active && use_graph_ && graph_ok_)
+        for (const auto& route : graph_)
+            for (const Graph& g : route)
+                if (g.exec) *graph_active = 1;
 }
 
 float BatchEngine::time_step(int repeats, cudaEvent_t e0, cudaEvent_t e1)
@@ -710,6 +715,8 @@ void BatchEngine::autotune(float dt, int repeats, lsp_batch_tuning* out, lsp_ste
         const int per_sm = most / std::max(sms, 1);
         if (per_sm >= 2) cands.push_back({T, (per_sm / 2) * sms, 0.f});
     }
+    const StepInFlight in_flight(dev_, threads_in_flight());
+    fits_ = in_flight.fits();
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));

@@ -88,8 +88,10 @@ private:
     int loop_grid() const;
     int enqueue_step(int c, int grid);   // returns the number of kernels launched
     // Whether the step runs as one launch (small_step.cu): the batch is small enough, no features
-    // are computed and no other launch shape was asked for.
-    bool one_launch() const { return small_lanes_ && !features_on() && !shaped_; }
+    // are computed, no other launch shape was asked for and it fits beside the steps in flight.
+    bool may_be_one() const { return small_lanes_ && !features_on() && !shaped_; }
+    bool one_launch() const { return may_be_one() && fits_; }
+    int64_t threads_in_flight() const { return batch_step_threads(n_, may_be_one() ? small_count_ : 0); }
     bool enqueue_small(int c);
     GridBuildArgs grid_args(int c);
     // Shortest of `repeats` runs of the pending step, ms (e0, e1: events to time it with).
@@ -120,6 +122,7 @@ private:
     bool built_ = false, pcisph_ = true;
     bool stepped_ = false;     // the lists and the grid are those of the last step
     BarrierStall stall_{};     // of the next step
+    bool fits_ = true;         // StepInFlight::fits of this step
     int64_t n_ = 0, cells_ = 0;
     int cur_ = 0;
     int mstride_ = 0;
@@ -156,8 +159,12 @@ private:
     int threads_ = 256, loop_blocks_ = 0;
     bool shaped_ = false;   // a launch shape of the separate kernels was chosen
     bool use_graph_ = true, graph_ok_ = true;
-    cudaGraphExec_t graph_[2] = {nullptr, nullptr};
-    int graph_launches_[2] = {0, 0};
+    // The step's graphs: of the separate kernels and of the one launch, per buffer parity.
+    struct Graph {
+        cudaGraphExec_t exec = nullptr;
+        int launches = 0;
+    };
+    Graph graph_[2][2];
 
     cudaEvent_t marks_[16] = {};
     int64_t launches_ = 0;

@@ -763,12 +763,13 @@ void Engine::abandon_step()
     throw Error(LSP_ERR_TIMEOUT, "a grid barrier of the one-launch step gave up; the state is that before the step");
 }
 
-// Small scenes take the whole step in one launch (small_step_lanes has the rule); the per-class
-// profile, the per-phase loop and the warm start's features need the separate kernels.
+// Small scenes take the whole step in one launch (small_step_lanes has the rule) that fits beside the
+// steps in flight; the per-class profile, the per-phase loop and the warm start's features need the
+// separate kernels.
 bool Engine::run_small(const GridBuildArgs& g, const StepBuffers& b)
 {
     const bool pci = prm_.solver == LSP_SOLVER_PCISPH;
-    if (profile_ || features_on()) return false;
+    if (profile_ || features_on() || !fits_) return false;
     if (pci && (prm_.loop_mode != LSP_LOOP_PERSISTENT || g.P.max_it <= 0)) return false;
     const int lanes = small_step_lanes(n_, cells_);
     if (!lanes) return false;
@@ -813,6 +814,8 @@ void Engine::run_step(float dt, lsp_step_stats* st)
     if (nbr_cap_ == 0 || nbr_stride_ < cap_) ensure_neighbors(nbr_cap_ ? nbr_cap_ : initial_neighbor_capacity(prm_));
     lsp_step_stats local{};
     bool device_loop = false;
+    const StepInFlight in_flight(dev_, step_threads(n_, cells_));
+    fits_ = in_flight.fits();
     for (int attempt = 0;; attempt++) {
         device_loop = false;
         DevParams P = device_params(dt);

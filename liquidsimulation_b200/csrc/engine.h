@@ -195,6 +195,7 @@ private:
     DevArray<float> stage_;
     HostStage hstage_;
     BarrierStall stall_{};   // of the next step
+    bool fits_ = true;       // StepInFlight::fits of this step
 
     // Launch bracketing for the per-class profile.
     template <typename F>

@@ -25,6 +25,8 @@
 #include "scan_ops.cuh"
 #include "small_step.h"
 
+#include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <mutex>
 
@@ -355,6 +357,59 @@ int small_step_lanes(int64_t n, int64_t cells)
     return 0;
 }
 
+// One group per particle in one block per SM, as evenly as whole warps allow.
+static void small_shape(int64_t n, int lanes, int* block, int* grid)
+{
+    const int sms = device_sm_count();
+    const int64_t threads = n * lanes;
+    const int64_t per_sm = (threads + sms - 1) / sms;
+    *block = (int)((per_sm + 63) / 64 * 64 < 128 ? 128 : (per_sm + 63) / 64 * 64);
+    *grid = (int)((threads + *block - 1) / *block);
+}
+
+static int64_t chip_threads() { return (int64_t)device_sm_count() * kMaxThreads; }
+
+int64_t step_threads(int64_t n, int64_t cells)
+{
+    const int lanes = small_step_lanes(n, cells);
+    if (!lanes) return std::min(n, chip_threads()) / 2;
+    int block, grid;
+    small_shape(n, lanes, &block, &grid);
+    return (int64_t)block * grid;
+}
+
+int64_t batch_step_threads(int64_t n, int small_blocks)
+{
+    return small_blocks ? (int64_t)small_blocks * kBatchThreads : std::min(n, chip_threads()) / 2;
+}
+
+// Threads of the steps in flight per device. Separate kernels count half of theirs: they leave places
+// free at their ends and between them. us a step of a small and of a large solver stepped at once,
+// the small one in one launch / in separate kernels: PCISPH of 1,200 particles beside SPH of 250,047
+// 73 and 178 / 135 and 153; 12,167 beside the same 97 and 208 / 151 and 165; 29,791 122 and 358 / 167
+// and 172, beside PCISPH of 417,792 161 and 812 / 420 and 499.
+static std::atomic<int64_t> g_in_flight[kMaxDevices];
+
+// An eighth more than fits still counts as fitting: the last blocks then wait for the end of another
+// step, which costs less than the separate kernels do. us a step, T threads stepping a PCISPH (SPH)
+// solver each, one launch / separate kernels: 1,200 particles T = 4, 1.01 of the chip, 22.7 / 28.5 (16.3 /
+// 18.1); 4,913, T = 2, 1.04 of the chip, 46.3 / 54.7 (30.5 / 31.0); 12,167, T = 2, 1.29, 58.4 / 57.2 (36.0 /
+// 31.6); 29,791, T = 2, 1.6, 81.8 / 64.9 (46.3 / 34.6); 12,167, T = 8, 57.1 / 19.9 (36.2 / 12.6). A step of a
+// quarter of the chip, one block of 128 threads per SM, runs beside three like it and takes one launch
+// whatever is in flight: 512 particles T = 16 5.8 / 10.9 (4.3 / 10.2), 1,100 particles T = 24 11.9 / 11.8
+// (8.4 / 9.8); with 150 blocks, 1,200 particles, T = 16, it is 22.4 / 11.2 (15.6 / 9.7).
+StepInFlight::StepInFlight(int device, int64_t threads) : dev_(device), threads_(threads)
+{
+    if (dev_ < 0 || dev_ >= kMaxDevices) return;
+    const int64_t others = g_in_flight[dev_].fetch_add(threads_, std::memory_order_relaxed);
+    fits_ = threads_ * 4 <= chip_threads() || others + threads_ <= chip_threads() * 9 / 8;
+}
+
+StepInFlight::~StepInFlight()
+{
+    if (dev_ >= 0 && dev_ < kMaxDevices) g_in_flight[dev_].fetch_sub(threads_, std::memory_order_relaxed);
+}
+
 bool launch_small_step(const SmallStepArgs& a, int lanes, cudaStream_t s)
 {
     const int c = lanes == 16 ? 0 : lanes == 8 ? 1 : lanes == 4 ? 2 : 3;
@@ -381,13 +436,9 @@ bool launch_small_step(const SmallStepArgs& a, int lanes, cudaStream_t s)
         fits = g_fits[dev][c];
     }
     if (!fits) return false;
-    // One group per particle in one block per SM, as evenly as whole warps allow.
-    const int sms = device_sm_count();
-    const int64_t threads = (int64_t)a.g.P.n * lanes;
-    const int64_t per_sm = (threads + sms - 1) / sms;
-    const int block = (int)((per_sm + 63) / 64 * 64 < 128 ? 128 : (per_sm + 63) / 64 * 64);
+    int block, grid;
+    small_shape(a.g.P.n, lanes, &block, &grid);
     if (block > kMaxThreads) return false;
-    const int grid = (int)((threads + block - 1) / block);
     SmallStepArgs ac = a;
     void* args[] = {&ac};
     return cudaLaunchCooperativeKernel(g_kernel[c], dim3(grid), dim3(block), args, step_smem(c, block), s) ==

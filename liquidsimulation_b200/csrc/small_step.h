@@ -34,6 +34,29 @@ constexpr int kSmallStepTiles = 1024;
 // Lanes per particle of the one-launch step for n particles in a grid of `cells`, 0 when the
 // separate kernels are used.
 int small_step_lanes(int64_t n, int64_t cells);
+// Threads that a step counts for (StepInFlight): those of its one launch, else half of one per particle
+// (of no more than fit).
+int64_t step_threads(int64_t n, int64_t cells);
+int64_t batch_step_threads(int64_t n, int small_blocks);   // small_blocks: of a one-launch step, 0: separate
+
+// A step in flight on a device, for the solvers that other host threads step there at the same time: a
+// one-launch step takes all its blocks' places at once and keeps them to its end, so steps that do
+// not fit beside each other would run one after the other, where separate kernels share the chip.
+class StepInFlight {
+public:
+    StepInFlight(int device, int64_t threads);
+    ~StepInFlight();
+    StepInFlight(const StepInFlight&) = delete;
+    StepInFlight& operator=(const StepInFlight&) = delete;
+    // Whether the step fits beside those that were in flight when it began.
+    bool fits() const { return fits_; }
+
+private:
+    int dev_;
+    int64_t threads_;
+    bool fits_ = true;
+};
+
 // False when the device refuses the launch (the caller then runs the separate kernels).
 bool launch_small_step(const SmallStepArgs& a, int lanes, cudaStream_t s);
 
