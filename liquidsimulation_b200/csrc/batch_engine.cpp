@@ -251,6 +251,8 @@ void BatchEngine::build()
     std::vector<SmallBatchBlock> blocks;
     small_lanes_ = small_batch_plan(scene_n, scene_cells, &blocks);
     small_count_ = (int)blocks.size();
+    one_threads_ = batch_step_threads(n_, small_count_);
+    separate_threads_ = batch_step_threads(n_, 0);
     if (small_lanes_) {
         if (tile_sums_.n < blocks.size()) tile_sums_.alloc(blocks.size());
         small_blocks_.alloc(blocks.size());

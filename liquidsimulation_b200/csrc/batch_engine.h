@@ -91,7 +91,7 @@ private:
     // are computed, no other launch shape was asked for and it fits beside the steps in flight.
     bool may_be_one() const { return small_lanes_ && !features_on() && !shaped_; }
     bool one_launch() const { return may_be_one() && fits_; }
-    int64_t threads_in_flight() const { return batch_step_threads(n_, may_be_one() ? small_count_ : 0); }
+    int64_t threads_in_flight() const { return may_be_one() ? one_threads_ : separate_threads_; }
     bool enqueue_small(int c);
     GridBuildArgs grid_args(int c);
     // Shortest of `repeats` runs of the pending step, ms (e0, e1: events to time it with).
@@ -150,6 +150,7 @@ private:
     DevStatus* status() { return reinterpret_cast<DevStatus*>(control_.p + sc_.size() * (4 + (size_t)mstride_)); }
     DevArray<SmallBatchBlock> small_blocks_;
     int small_lanes_ = 0, small_count_ = 0;   // of the one-launch step; 0: the batch is too large for it
+    int64_t one_threads_ = 0, separate_threads_ = 0;   // that a step counts for (StepInFlight)
     DevParams* hparams_ = nullptr;   // pinned
     DevStatus* hstatus_ = nullptr;   // pinned
     int items_count_ = 0;

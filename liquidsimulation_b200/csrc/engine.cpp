@@ -771,8 +771,7 @@ bool Engine::run_small(const GridBuildArgs& g, const StepBuffers& b)
     const bool pci = prm_.solver == LSP_SOLVER_PCISPH;
     if (profile_ || features_on() || !fits_) return false;
     if (pci && (prm_.loop_mode != LSP_LOOP_PERSISTENT || g.P.max_it <= 0)) return false;
-    const int lanes = small_step_lanes(n_, cells_);
-    if (!lanes) return false;
+    if (!lanes_) return false;
     SmallStepArgs a{};
     a.g = g;
     a.b = b;
@@ -783,7 +782,7 @@ bool Engine::run_small(const GridBuildArgs& g, const StepBuffers& b)
     a.pcisph = pci ? 1 : 0;
     a.stall = stall_;
     std::memset(hstatus_, 0, sizeof(DevStatus));
-    if (!launch_small_step(a, lanes, stream_)) {
+    if (!launch_small_step(a, lanes_, stream_)) {
         cudaGetLastError();   // the device refused the cooperative launch
         return false;
     }
@@ -814,7 +813,13 @@ void Engine::run_step(float dt, lsp_step_stats* st)
     if (nbr_cap_ == 0 || nbr_stride_ < cap_) ensure_neighbors(nbr_cap_ ? nbr_cap_ : initial_neighbor_capacity(prm_));
     lsp_step_stats local{};
     bool device_loop = false;
-    const StepInFlight in_flight(dev_, step_threads(n_, cells_));
+    if (n_ != lanes_n_ || cells_ != lanes_cells_) {
+        lanes_ = small_step_lanes(n_, cells_);
+        step_threads_ = step_threads(n_, lanes_);
+        lanes_n_ = n_;
+        lanes_cells_ = cells_;
+    }
+    const StepInFlight in_flight(dev_, step_threads_);
     fits_ = in_flight.fits();
     for (int attempt = 0;; attempt++) {
         device_loop = false;

@@ -196,6 +196,10 @@ private:
     HostStage hstage_;
     BarrierStall stall_{};   // of the next step
     bool fits_ = true;       // StepInFlight::fits of this step
+    // Lanes of a one-launch step and the threads a step counts for, of lanes_n_ particles in
+    // lanes_cells_ cells.
+    int lanes_ = 0;
+    int64_t lanes_n_ = -1, lanes_cells_ = -1, step_threads_ = 0;
 
     // Launch bracketing for the per-class profile.
     template <typename F>

@@ -369,9 +369,8 @@ static void small_shape(int64_t n, int lanes, int* block, int* grid)
 
 static int64_t chip_threads() { return (int64_t)device_sm_count() * kMaxThreads; }
 
-int64_t step_threads(int64_t n, int64_t cells)
+int64_t step_threads(int64_t n, int lanes)
 {
-    const int lanes = small_step_lanes(n, cells);
     if (!lanes) return std::min(n, chip_threads()) / 2;
     int block, grid;
     small_shape(n, lanes, &block, &grid);
@@ -402,6 +401,7 @@ StepInFlight::StepInFlight(int device, int64_t threads) : dev_(device), threads_
 {
     if (dev_ < 0 || dev_ >= kMaxDevices) return;
     const int64_t others = g_in_flight[dev_].fetch_add(threads_, std::memory_order_relaxed);
+    if (others == 0) return;
     fits_ = threads_ * 4 <= chip_threads() || others + threads_ <= chip_threads() * 9 / 8;
 }
 

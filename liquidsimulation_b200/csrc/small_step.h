@@ -36,7 +36,7 @@ constexpr int kSmallStepTiles = 1024;
 int small_step_lanes(int64_t n, int64_t cells);
 // Threads that a step counts for (StepInFlight): those of its one launch, else half of one per particle
 // (of no more than fit).
-int64_t step_threads(int64_t n, int64_t cells);
+int64_t step_threads(int64_t n, int lanes);   // lanes: of the one launch, 0: separate kernels
 int64_t batch_step_threads(int64_t n, int small_blocks);   // small_blocks: of a one-launch step, 0: separate
 
 // A step in flight on a device, for the solvers that other host threads step there at the same time: a
@@ -52,8 +52,8 @@ public:
     bool fits() const { return fits_; }
 
 private:
-    int dev_;
-    int64_t threads_;
+    const int dev_;
+    const int64_t threads_;
     bool fits_ = true;
 };
 
