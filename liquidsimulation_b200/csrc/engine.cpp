@@ -512,7 +512,7 @@ StepBuffers Engine::buffers()
     b.force = force_.p; b.rho = rho_.p; b.pres = pres_.p;
     b.ppos = ppos_.p; b.phalf = phalf_.p; b.pforce = pforce_.p; b.prho = prho_.p; b.err = err_.p;
     b.nbr = nbr_.p; b.nbr_count = nbr_count_.p; b.vrho = vrho_.p;
-    b.xpf = ppos_alt_.p;   // SPH has no predicted positions
+    b.xpf = sph_records();
     b.tables = tables_.p; b.colliders = dcols_.p; b.status = status();
     b.hist = phist_[cur_].p;
     b.gradrho = features_on() ? gradrho_.p : nullptr;
@@ -787,7 +787,6 @@ bool Engine::run_small(const GridBuildArgs& g, const StepBuffers& b)
         return false;
     }
     launches_++;
-    ppos_final_ = ppos_.p;
     return true;
 }
 
@@ -838,7 +837,7 @@ void Engine::run_step(float dt, lsp_step_stats* st)
         g.nbr = nbr_.p; g.nbr_count = nbr_count_.p; g.status = status();
         // The neighbour build also sums the start-of-step density (k_neighbors_density).
         g.tables = tables_.p; g.rho = rho_.p; g.pres = pres_.p; g.vrho = vrho_.p;
-        g.xpf = prm_.solver == LSP_SOLVER_SPH ? ppos_alt_.p : nullptr;
+        g.xpf = prm_.solver == LSP_SOLVER_SPH ? sph_records() : nullptr;
         cur_ = 1 - cur_;
         StepBuffers b = buffers();
         if (run_small(g, b)) {

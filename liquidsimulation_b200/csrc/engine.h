@@ -162,6 +162,9 @@ private:
     DevArray<float4> pos_[2], vel_[2], half_[2], old_[2];
     DevArray<float4> force_, ppos_, ppos_alt_, phalf_, pforce_;
     const float4* ppos_final_ = nullptr;   // buffer holding the last iteration's x*
+    // SPH's {x, p / rho^2}: SPH has no predicted positions, but a solver that was PCISPH before still
+    // holds those of its last step, in one of the two buffers.
+    float4* sph_records() const { return ppos_final_ == ppos_alt_.p ? ppos_.p : ppos_alt_.p; }
     DevArray<float> rho_, pres_, prho_, err_;
     DevArray<float4> vrho_;   // {v, rho} for the non-pressure pass (StepBuffers::vrho)
     DevArray<uint32_t> key_, slot_, sorted_key_;
