@@ -968,7 +968,7 @@ void Engine::read_field(int field, float* out, int64_t n)
     if (field == LSP_FIELD_NEIGHBOR_COUNT)
         launch_gather_count(nbr_count_.p, slot_of_id_.p, to, n, stream_);
     else
-        launch_gather_field(src, comps, mode, slot_of_id_.p, to, n, stream_);
+        launch_gather_field(src, comps, mode, slot_of_id_.p, to, direct, n, stream_);
     CK(cudaGetLastError());
     if (!direct) CK(cudaMemcpyAsync(out, stage_.p, bytes, cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
@@ -1007,7 +1007,8 @@ void Engine::read_state(float* x, float* v, float* half, float* old, int32_t* fi
         h.add(first, (size_t)n * sizeof(int32_t));
         if (h.ready()) {
             launch_gather_state(pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, slot_of_id_.p, (float*)h.view(0),
-                                (float*)h.view(1), (float*)h.view(2), (float*)h.view(3), (int32_t*)h.view(4), n, stream_);
+                                (float*)h.view(1), (float*)h.view(2), (float*)h.view(3), (int32_t*)h.view(4), true, n,
+                                stream_);
             CK(cudaGetLastError());
             CK(cudaStreamSynchronize(stream_));
             h.finish();
@@ -1017,7 +1018,7 @@ void Engine::read_state(float* x, float* v, float* half, float* old, int32_t* fi
     stage((size_t)n * 13);
     float* s = stage_.p;
     launch_gather_state(pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, slot_of_id_.p, s, s + 3 * n,
-                        s + 6 * n, s + 9 * n, (int32_t*)(s + 12 * n), n, stream_);
+                        s + 6 * n, s + 9 * n, (int32_t*)(s + 12 * n), false, n, stream_);
     size_t b3 = (size_t)n * 3 * sizeof(float);
     CK(cudaMemcpyAsync(x, s, b3, cudaMemcpyDeviceToHost, stream_));
     CK(cudaMemcpyAsync(v, s + 3 * n, b3, cudaMemcpyDeviceToHost, stream_));
@@ -1040,7 +1041,7 @@ void Engine::write_state(const float* x, const float* v, const float* half, cons
         if (h.ready()) {
             launch_scatter_state((const float*)h.view(0), (const float*)h.view(1), (const float*)h.view(2),
                                  (const float*)h.view(3), (const int32_t*)h.view(4), slot_of_id_.p, pos_[cur_].p,
-                                 vel_[cur_].p, half_[cur_].p, old_[cur_].p, n, stream_);
+                                 vel_[cur_].p, half_[cur_].p, old_[cur_].p, true, n, stream_);
             CK(cudaGetLastError());
             CK(cudaStreamSynchronize(stream_));
             if (domain_from_particles_) grid_valid_ = false;
@@ -1056,7 +1057,7 @@ void Engine::write_state(const float* x, const float* v, const float* half, cons
     CK(cudaMemcpyAsync(s + 9 * n, old, b3, cudaMemcpyHostToDevice, stream_));
     CK(cudaMemcpyAsync(s + 12 * n, first, (size_t)n * sizeof(int32_t), cudaMemcpyHostToDevice, stream_));
     launch_scatter_state(s, s + 3 * n, s + 6 * n, s + 9 * n, (const int32_t*)(s + 12 * n), slot_of_id_.p,
-                         pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, n, stream_);
+                         pos_[cur_].p, vel_[cur_].p, half_[cur_].p, old_[cur_].p, false, n, stream_);
     CK(cudaStreamSynchronize(stream_));
     if (domain_from_particles_) grid_valid_ = false;
 }
@@ -1078,7 +1079,7 @@ void Engine::read_history(float* out, int64_t n)
     }
     activate();
     stage((size_t)n * 3);
-    launch_gather_field(phist_[cur_].p, 3, 0, slot_of_id_.p, stage_.p, n, stream_);
+    launch_gather_field(phist_[cur_].p, 3, 0, slot_of_id_.p, stage_.p, false, n, stream_);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, stage_.p, (size_t)n * 3 * sizeof(float), cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));

@@ -72,9 +72,8 @@ char* HostStage::get(size_t bytes)
 
 void HostTransfer::add(const void* p, size_t bytes)
 {
-    bool host;
-    e_[n_++] = Entry{const_cast<void*>(p), bytes, pinned_view(p, bytes, &host), nullptr};
-    host_ = host_ && host;
+    if (!host_) return;
+    e_[n_++] = Entry{const_cast<void*>(p), bytes, pinned_view(p, bytes, &host_), nullptr};
 }
 
 bool HostTransfer::ready()

@@ -145,10 +145,11 @@ void launch_mlp_adam(const float* partial, const float* loss_partial, int rows, 
                      cudaStream_t s);
 
 // Gathers a per-particle field from device order into caller order.
-// comps: 1 (float) or 3 (xyz of a float4); src is float* or float4* accordingly.
+// comps: 1 (float) or 3 (xyz of a float4); src is float* or float4* accordingly. host (here and below):
+// the caller-order arrays are the host's memory, not the device's.
 void launch_gather_field(const void* src, int comps, int w_as_flag, const int32_t* slot_of_id, float* out,
-                         int64_t n, cudaStream_t s);
-// Positions and velocities of a field read-back in one launch.
+                         bool host, int64_t n, cudaStream_t s);
+// Positions and velocities of a read-back into the host's memory in one launch.
 void launch_gather_particles(const float4* pos, const float4* vel, const int32_t* slot_of_id, float* x, float* v,
                              int64_t n, cudaStream_t s);
 // slot_of_id of n particles from the ids in their positions' w.
@@ -157,7 +158,7 @@ void launch_gather_count(const int32_t* count, const int32_t* slot_of_id, float*
 // Scatters caller-order state (x, v, v_half, v_half_old, first) into device slots.
 void launch_scatter_state(const float* x, const float* v, const float* half, const float* old,
                           const int32_t* first, const int32_t* slot_of_id, float4* pos, float4* vel,
-                          float4* hvel, float4* oldv, int64_t n, cudaStream_t s);
+                          float4* hvel, float4* oldv, bool host, int64_t n, cudaStream_t s);
 // dst[slot_of_id[id]] = (in[3 id], in[3 id + 1], in[3 id + 2], 0) for caller-order rows.
 void launch_scatter_vec(const float* in, const int32_t* slot_of_id, float4* dst, int64_t n, cudaStream_t s);
 
@@ -169,7 +170,7 @@ void barrier_probe(int blocks, int parties, int* completed, uint32_t* error_flag
 // Writes caller-order x, v, v_half, v_half_old, first from device slots.
 void launch_gather_state(const float4* pos, const float4* vel, const float4* hvel, const float4* oldv,
                          const int32_t* slot_of_id, float* x, float* v, float* half, float* old, int32_t* first,
-                         int64_t n, cudaStream_t s);
+                         bool host, int64_t n, cudaStream_t s);
 // Neighbour lists in caller order and caller ids.
 void launch_neighbor_export(const int32_t* nbr, const int32_t* count, int64_t stride, const float4* pos,
                             const int32_t* slot_of_id, const int64_t* offsets, int32_t* out, int64_t n,

@@ -12,11 +12,13 @@ namespace lsp {
 constexpr int kThreads = 256;
 static inline unsigned blocks_for(int64_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
-// Rows of three floats between caller order (packed, possibly host memory) and device slots: a
-// block moves 256 consecutive rows of up to four arrays and the first-step flags. The packed side
-// goes through shared memory, so that it is read and written contiguously, 16 bytes at a time where
-// every array's alignment allows (a row at a time it would be three strided accesses, each a
-// request of its own over PCIe).
+// Rows of three floats between caller order (packed) and device slots: a thread moves a row of up to
+// four arrays and its first-step flag. Packed arrays in the host's memory go through shared memory (the
+// _host kernels), 256 rows at a time, so that they are read and written contiguously, 16 bytes at a
+// time where every array's alignment allows: a row at a time it would be three strided accesses, each a
+// request of its own over PCIe. In device memory L2 merges those, and the block's wait for its slowest
+// row costs more than it saves: a field of 990,000 positions 25 us a row at a time, 35 through shared
+// memory, the state 88 and 106.
 struct RowArrays {
     const float4* slots[4];
     float* rows[4];
@@ -43,8 +45,28 @@ __device__ __forceinline__ void move_rows(float* packed, float* sm, int floats)
     }
 }
 
+template <int kCount>
+__global__ void __launch_bounds__(kThreads) k_gather_rows(RowArrays a, const int32_t* __restrict__ slot_of_id, int64_t n)
+{
+    const int64_t id = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (id >= n) return;
+    const int32_t s = slot_of_id[id];
+    float4 v[kCount];
+#pragma unroll
+    for (int c = 0; c < kCount; c++) v[c] = __ldg(a.slots[c] + s);
+    const float flag = a.flag_slots ? __ldg(&a.flag_slots[s].w) : 0.f;
+#pragma unroll
+    for (int c = 0; c < kCount; c++) {
+        float* to = a.rows[c] + 3 * id;
+        to[0] = v[c].x;
+        to[1] = v[c].y;
+        to[2] = v[c].z;
+    }
+    if (a.flag_slots) a.flags[id] = flag != 0.f ? 1 : 0;
+}
+
 template <bool kVector>
-__global__ void __launch_bounds__(kThreads) k_gather_rows3(RowArrays a, const int32_t* __restrict__ slot_of_id, int64_t n)
+__global__ void __launch_bounds__(kThreads) k_gather_rows_host(RowArrays a, const int32_t* __restrict__ slot_of_id, int64_t n)
 {
     __shared__ alignas(16) float sm[4][3 * kThreads];
     const int64_t base = (int64_t)blockIdx.x * kThreads, id = base + threadIdx.x;
@@ -65,9 +87,27 @@ __global__ void __launch_bounds__(kThreads) k_gather_rows3(RowArrays a, const in
 
 // The other way for the whole state: positions (w: caller id), velocities (w: flag), half and old
 // half velocities (w kept).
-template <bool kVector>
-__global__ void __launch_bounds__(kThreads) k_scatter_state(RowArrays a, float4* pos, float4* vel, float4* hv, float4* ov,
+__global__ void __launch_bounds__(kThreads) k_scatter_state(RowArrays a, float4* __restrict__ pos, float4* __restrict__ vel,
+                                                            float4* __restrict__ hv, float4* __restrict__ ov,
                                                             const int32_t* __restrict__ slot_of_id, int64_t n)
+{
+    const int64_t id = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (id >= n) return;
+    const int32_t s = slot_of_id[id], flag = __ldg(a.flags + id);
+    auto row = [&](int c, float w) {
+        const float* from = a.rows[c] + 3 * id;
+        return make_float4(__ldg(from), __ldg(from + 1), __ldg(from + 2), w);
+    };
+    const float hw = hv[s].w, ow = ov[s].w;
+    pos[s] = row(0, __int_as_float((int)id));
+    vel[s] = row(1, flag ? 1.f : 0.f);
+    hv[s] = row(2, hw);
+    ov[s] = row(3, ow);
+}
+
+template <bool kVector>
+__global__ void __launch_bounds__(kThreads) k_scatter_state_host(RowArrays a, float4* pos, float4* vel, float4* hv, float4* ov,
+                                                                 const int32_t* __restrict__ slot_of_id, int64_t n)
 {
     __shared__ alignas(16) float sm[4][3 * kThreads];
     const int64_t base = (int64_t)blockIdx.x * kThreads, id = base + threadIdx.x;
@@ -93,11 +133,11 @@ static bool aligned_rows(const RowArrays& a)
         if ((uintptr_t)a.rows[c] % sizeof(float4)) return false;
     return true;
 }
-static void gather_rows3(const RowArrays& a, const int32_t* slot_of_id, int64_t n, cudaStream_t s)
+static void gather_rows_host(const RowArrays& a, const int32_t* slot_of_id, int64_t n, cudaStream_t s)
 {
     if (!n) return;
-    if (aligned_rows(a)) k_gather_rows3<true><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
-    else k_gather_rows3<false><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
+    if (aligned_rows(a)) k_gather_rows_host<true><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
+    else k_gather_rows_host<false><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
 }
 
 __global__ void k_gather_w(const float4* __restrict__ src, const int32_t* __restrict__ slot_of_id,
@@ -143,7 +183,7 @@ void launch_slots_of_ids(const float4* pos, int32_t* slot_of_id, int64_t n, cuda
     if (n) k_slots_of_ids<<<blocks_for(n), kThreads, 0, s>>>(pos, slot_of_id, n);
 }
 
-void launch_gather_field(const void* src, int comps, int mode, const int32_t* slot_of_id, float* out, int64_t n,
+void launch_gather_field(const void* src, int comps, int mode, const int32_t* slot_of_id, float* out, bool host, int64_t n,
                          cudaStream_t s)
 {
     if (!n) return;
@@ -152,7 +192,8 @@ void launch_gather_field(const void* src, int comps, int mode, const int32_t* sl
         a.slots[0] = (const float4*)src;
         a.rows[0] = out;
         a.count = 1;
-        gather_rows3(a, slot_of_id, n, s);
+        if (host) gather_rows_host(a, slot_of_id, n, s);
+        else k_gather_rows<1><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
     } else if (mode == 1)
         k_gather_w<<<blocks_for(n), kThreads, 0, s>>>((const float4*)src, slot_of_id, out, n);
     else if (mode == 2)
@@ -175,12 +216,12 @@ void launch_gather_particles(const float4* pos, const float4* vel, const int32_t
     a.rows[0] = x;
     a.rows[1] = v;
     a.count = 2;
-    gather_rows3(a, slot_of_id, n, s);
+    gather_rows_host(a, slot_of_id, n, s);
 }
 
 void launch_scatter_state(const float* x, const float* v, const float* half, const float* old, const int32_t* first,
                           const int32_t* slot_of_id, float4* pos, float4* vel, float4* hvel, float4* oldv,
-                          int64_t n, cudaStream_t s)
+                          bool host, int64_t n, cudaStream_t s)
 {
     if (!n) return;
     RowArrays a{};
@@ -188,8 +229,10 @@ void launch_scatter_state(const float* x, const float* v, const float* half, con
     for (int c = 0; c < 4; c++) a.rows[c] = const_cast<float*>(rows[c]);
     a.count = 4;
     a.flags = const_cast<int32_t*>(first);
-    if (aligned_rows(a)) k_scatter_state<true><<<blocks_for(n), kThreads, 0, s>>>(a, pos, vel, hvel, oldv, slot_of_id, n);
-    else k_scatter_state<false><<<blocks_for(n), kThreads, 0, s>>>(a, pos, vel, hvel, oldv, slot_of_id, n);
+    const unsigned blocks = blocks_for(n);
+    if (!host) k_scatter_state<<<blocks, kThreads, 0, s>>>(a, pos, vel, hvel, oldv, slot_of_id, n);
+    else if (aligned_rows(a)) k_scatter_state_host<true><<<blocks, kThreads, 0, s>>>(a, pos, vel, hvel, oldv, slot_of_id, n);
+    else k_scatter_state_host<false><<<blocks, kThreads, 0, s>>>(a, pos, vel, hvel, oldv, slot_of_id, n);
 }
 
 __global__ void k_scatter_vec(const float* __restrict__ in, const int32_t* __restrict__ slot_of_id,
@@ -207,8 +250,9 @@ void launch_scatter_vec(const float* in, const int32_t* slot_of_id, float4* dst,
 
 void launch_gather_state(const float4* pos, const float4* vel, const float4* hvel, const float4* oldv,
                          const int32_t* slot_of_id, float* x, float* v, float* half, float* old, int32_t* first,
-                         int64_t n, cudaStream_t s)
+                         bool host, int64_t n, cudaStream_t s)
 {
+    if (!n) return;
     RowArrays a{};
     const float4* slots[4] = {pos, vel, hvel, oldv};
     float* rows[4] = {x, v, half, old};
@@ -219,7 +263,8 @@ void launch_gather_state(const float4* pos, const float4* vel, const float4* hve
     a.count = 4;
     a.flag_slots = vel;
     a.flags = first;
-    gather_rows3(a, slot_of_id, n, s);
+    if (host) gather_rows_host(a, slot_of_id, n, s);
+    else k_gather_rows<4><<<blocks_for(n), kThreads, 0, s>>>(a, slot_of_id, n);
 }
 
 __global__ void k_neighbor_export(const int32_t* __restrict__ nbr, const int32_t* __restrict__ count, int64_t stride,
