@@ -175,7 +175,7 @@ int lsp_step_many(lsp_solver* s, float dt, int steps, lsp_step_stats* stats);
 /* Check of a step that gives up (no counterpart in the reference): the next step, as one launch, whose
  * barrier-th grid barrier (from 1) waits for an arrival that does not come, for a short time. A step
  * of one launch that gives up returns LSP_ERR_TIMEOUT and leaves the state as it was before the call
- * (its lists and grid are refused until the next step). LSP_ERR_STATE when the step would not run as
+ * (its lists, grid and other results are refused until the next step). LSP_ERR_STATE when the step would not run as
  * one launch; LSP_OK, and an ordinary step, when it has fewer barriers. */
 int lsp_stalled_step(lsp_solver* s, float dt, int barrier);
 int lsp_synchronize(lsp_solver* s);

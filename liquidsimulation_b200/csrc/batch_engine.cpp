@@ -536,6 +536,7 @@ void BatchEngine::run_once(int c)
 void BatchEngine::abandon_step(int c)
 {
     stepped_ = false;
+    unfinished_ = true;
     CK(cudaMemsetAsync(hist_.p, 0, hist_.n * sizeof(uint32_t), stream_));
     launch_slots_of_ids(pos_[c].p, slot_of_id_.p, n_, stream_);
     CK(cudaGetLastError());
@@ -569,6 +570,7 @@ void BatchEngine::finish_step(lsp_step_stats* stats)
     const int S = (int)sc_.size();
     cur_ = 1 - cur_;
     stepped_ = true;
+    unfinished_ = false;
     features_valid_ = features_on();
     uint32_t errors = hstatus_[S].error_flags;
     bool not_converged = false;
@@ -786,6 +788,7 @@ void BatchEngine::read_field(int scene, int field, float* out, int64_t n)
     check_scene(scene);
     const Scene& s = sc_[scene];
     if (!out || n != s.n) throw Error(LSP_ERR_INVALID, "read_field: n must equal the scene's particle count");
+    if (unfinished_ && step_result_field(field)) throw Error(LSP_ERR_STATE, "read_field: the last step gave up");
     activate();
     const void* src = nullptr;
     int comps = 1, mode = 0;

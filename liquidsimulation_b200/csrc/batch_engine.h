@@ -121,6 +121,7 @@ private:
     std::vector<float4> init_pos_, init_vel_;   // host copies until the first step
     bool built_ = false, pcisph_ = true;
     bool stepped_ = false;     // the lists and the grid are those of the last step
+    bool unfinished_ = false;  // Engine::unfinished_
     BarrierStall stall_{};     // of the next step
     bool fits_ = true;         // StepInFlight::fits of this step
     int64_t n_ = 0, cells_ = 0;

@@ -325,6 +325,7 @@ void Engine::remove_particles()
     n_ = 0;
     if (domain_from_particles_) grid_valid_ = false;
     stepped_ = false;
+    unfinished_ = false;
 }
 
 int Engine::add_collider(const Collider& c)
@@ -732,6 +733,16 @@ int warm_auto_switch(const lsp_params& p)
     return p.warm_auto_iterations > 0 ? p.warm_auto_iterations : std::max(12, p.pci_max_iterations / 2);
 }
 
+bool step_result_field(int field)
+{
+    switch (field) {
+    case LSP_FIELD_DENSITY: case LSP_FIELD_PRESSURE: case LSP_FIELD_PRED_DENSITY: case LSP_FIELD_DENSITY_ERROR:
+    case LSP_FIELD_PRED_POSITION: case LSP_FIELD_PRED_HALF_VELOCITY: case LSP_FIELD_PRED_PRESSURE_FORCE:
+    case LSP_FIELD_NEIGHBOR_COUNT: return true;
+    default: return false;
+    }
+}
+
 int grown_neighbor_capacity(int needed, int current)
 {
     const int64_t c = std::max<int64_t>((int64_t)needed + needed / 2 + 8, 2 * (int64_t)current);
@@ -756,6 +767,7 @@ void Engine::abandon_step()
 {
     cur_ = 1 - cur_;
     stepped_ = false;   // the lists and the grid are unfinished too
+    unfinished_ = true;
     CK(cudaMemsetAsync(hist_.p, 0, hist_.n * sizeof(uint32_t), stream_));
     launch_slots_of_ids(pos_[cur_].p, slot_of_id_.p, n_, stream_);
     CK(cudaGetLastError());
@@ -872,6 +884,7 @@ void Engine::run_step(float dt, lsp_step_stats* st)
         if (!retry_step(attempt)) break;
     }
     stepped_ = true;
+    unfinished_ = false;
     if (device_loop) {
         float me;
         std::memcpy(&me, &hstatus_->max_err_bits, 4);
@@ -939,6 +952,7 @@ void Engine::read_field(int field, float* out, int64_t n)
 {
     if (!out || n != n_) throw Error(LSP_ERR_INVALID, "read_field: n must equal the particle count");
     if (n == 0) return;
+    if (unfinished_ && step_result_field(field)) throw Error(LSP_ERR_STATE, "read_field: the last step gave up");
     activate();
     const void* src = nullptr;
     int comps = 1, mode = 0;

@@ -55,6 +55,8 @@ DevParams physics_params(const lsp_params& p, const HostKernels& hk, float dt);
 int initial_neighbor_capacity(const lsp_params& p);
 // Neighbour-list capacity after an overflow of `needed` entries with `current` allocated.
 int grown_neighbor_capacity(int needed, int current);
+// Whether a field is computed by the step (the others are the particles' state).
+bool step_result_field(int field);
 // LSP_WARM_AUTO switch point: warm_auto_iterations, or max(12, pci_max_iterations / 2) for 0.
 int warm_auto_switch(const lsp_params& p);
 
@@ -217,6 +219,7 @@ private:
     int64_t prof_n_[LSP_PROF_COUNT] = {};
     int64_t launches_ = 0;
     DevArray<int32_t> bounds_;
+    bool unfinished_ = false;   // the last step gave up half-way: its results are neither the old nor new ones
     bool stepped_ = false;   // a step has run on the current particle set (lists, grid, features valid)
 
     // Learned warm start state.

@@ -99,6 +99,36 @@ def test_scene_of_a_batch(solver, edge, barriers, graph, before):
         twin.close()
 
 
+RESULTS = [abi.FIELD_DENSITY, abi.FIELD_PRESSURE, abi.FIELD_PRED_DENSITY, abi.FIELD_DENSITY_ERROR,
+           abi.FIELD_PRED_POSITION, abi.FIELD_PRED_HALF_VELOCITY, abi.FIELD_PRED_PRESSURE_FORCE,
+           abi.FIELD_NEIGHBOR_COUNT]
+
+
+@pytest.mark.parametrize("barrier", [2, 6, 9])
+def test_results_of_a_step_that_gave_up(barrier):
+    """They are neither the last step's (other slots, partly overwritten) nor a step's at all."""
+    import ctypes
+    sc = scene(abi.LSP_SOLVER_PCISPH)
+    s, twin = from_scene(sc), from_scene(sc)
+    b = batch_from_scenes([sc, sc])
+    for x in (s, twin, b):
+        x.update(sc.dt)
+    refused(abi.LSP_ERR_TIMEOUT, s._call, "lsp_stalled_step", ctypes.c_float(sc.dt), barrier)
+    refused(abi.LSP_ERR_TIMEOUT, b._call, "lsp_batch_stalled_step", ctypes.c_float(sc.dt), 1, barrier)
+    for f in RESULTS:
+        refused(abi.LSP_ERR_STATE, s.read, f)
+        for k in range(2):
+            refused(abi.LSP_ERR_STATE, b.read, k, f)
+    assert np.array_equal(bits(s.read(abi.FIELD_SPEED_SQUARED)), bits(twin.read(abi.FIELD_SPEED_SQUARED)))
+    for x in (s, twin, b):
+        x.update(sc.dt)
+    for f in RESULTS:
+        for got in (s.read(f), b.read(0, f), b.read(1, f)):
+            assert np.array_equal(bits(got), bits(twin.read(f))), f
+    for x in (s, twin, b):
+        x.close()
+
+
 def test_what_is_refused():
     import ctypes
     sc = scene(abi.LSP_SOLVER_PCISPH)
